@@ -436,10 +436,14 @@ typedef struct
      * kernel that also runs the DMMA pairs). */
     int b_staging;
     /* Early split of heavy C tile rows.  A tile row that needs several
-     * windows of C tiles walks all its products once per window; when that
+     * windows of C tiles runs one scalar row per warp where C is written as
+     * CSR alone and B's rows strictly increase: rows of more than about
+     * split_target products are cut into tasks of about that many (0 = by
+     * nnz(C), between 2^14 and 2^17).  Otherwise it
+     * walks all its products once per window; when that
      * walk exceeds split_target products the row is cut into tasks of
      * consecutive windows of about split_target products each, which
-     * persistent CTAs take from a device queue.  0 = the default (2^20);
+     * persistent CTAs take from a device queue (0 = 2^20);
      * negative = never split (each tile row's CTA runs its windows in
      * sequence).  Every setting gives bitwise the same C. */
     int split_target;
@@ -523,8 +527,8 @@ typedef struct
     double symbolic_ms;
     double numeric_kernel_ms;
     /* Window tasks of the last numeric step: C tile rows that need several
-     * windows of C tiles are cut into windows that persistent CTAs take from
-     * a device queue (the early split of src/dmma_tile_early_split.h). */
+     * windows of C tiles are cut into tasks (rows, pieces of rows, or windows
+     * of C tiles) that persistent CTAs take from a device queue (the early split of src/dmma_tile_early_split.h). */
     long long split_windows;
     /* 1 when the last numeric phase ran as a launch of a captured CUDA graph
      * (cuda_graphs), else 0. */

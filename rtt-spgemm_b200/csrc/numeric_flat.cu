@@ -1483,7 +1483,13 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
     const bool glob = split && cfg.global_rows > 0 && acsr && !cfg.conflict_safe &&
                       cfg.csr_col != nullptr && !cfg.write_tiles &&
                       (cfg.global_rows == 2 || S.tilen <= (1 << 20));
-    if (split)
+    // heavy tile rows one scalar row per warp (numeric_rowwin.cu): CSR output
+    // alone, A from its CSR rows, strictly increasing B rows
+    const bool rowwin = split && !glob && acsr && !cfg.conflict_safe && cfg.csr_col != nullptr &&
+                        !cfg.write_tiles;
+    if (rowwin)
+        RTT_CHECK(numeric_rowwin_device(ws, A, B, S, cfg));
+    else if (split)
     {
         RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(WinQueue), s));
         auto plan = !glob                  ? k_win_plan<ACC_SMALL, 0>
@@ -1549,12 +1555,14 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
         ws.launches++;
         RTT_CUDA(cudaEventRecord(ws.join_ev, ws.side));
     }
-    else if (split)
+    else if (split && !rowwin)
     {
         // The workers go first, on the side stream, so that the split rows'
         // tasks start while the tile-row CTAs run (the reference's heavy grid
         // enqueued before its light grid, src/dmma_tile_early_split.h:13-27).
         // One wave of resident CTAs; with an empty queue they exit at once.
+        // (strictly increasing B rows with the fused CSR output alone never
+        // come here: numeric_rowwin_device takes them)
         auto wk = acsr ? (cfg.conflict_safe ? k_numeric_flat<true, ACC_SMALL, CTAS_SMALL, true, true, true>
                                             : k_numeric_flat<false, ACC_SMALL, CTAS_SMALL, true, true, true>)
                        : (cfg.conflict_safe ? k_numeric_flat<true, ACC_SMALL, CTAS_SMALL, true, true, false>

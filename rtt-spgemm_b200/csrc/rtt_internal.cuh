@@ -323,6 +323,10 @@ struct SymbolicOut
     DevBuf w_task, w_heavy, w_queue, w_flag;
     DevBuf w_cursor; // per worker CTA: window cursors of its task's A entries
     DevBuf g_slot, g_rel; // per global-row worker CTA: tile column table, row offsets
+    // row windows of heavy tile rows: tasks (pieces of long rows, groups of
+    // rows), the C tile masks row by row, each warp's places in B's rows, the
+    // tile columns of the cuts and B's rows' places there
+    DevBuf r_big, r_normal, r_mask, r_cursor, r_cut, r_part;
     // symbolic step 2: heavy tile rows (flag per tile row, list) and the
     // list of tile rows for the wide-window CTAs
     DevBuf s2_heavy, s2_list, s2_wlist;
@@ -348,7 +352,8 @@ struct SymbolicOut
                                &c_tr_nnz,   &count_tmp,  &tile_cnt,   &w_task,     &w_heavy,
                                &w_queue,    &w_flag,     &s2_heavy,   &s2_list,
                                &s2_wlist,   &s1_list,    &w_cursor,   &g_slot,
-                               &g_rel};
+                               &g_rel,      &r_big,      &r_normal,   &r_mask,
+                               &r_cursor,   &r_cut,      &r_part};
         for (const DevBuf *b : all)
             f(*b);
     }
@@ -397,6 +402,12 @@ int numeric_rows_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
 // numeric step without a copy pipeline: warp-private Gustavson per row pair
 int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
                         const NumericConfig &cfg);
+// heavy tile rows of a multi-window product, one scalar row per warp: plans
+// the tasks, marks the tile rows in S.w_heavy and runs them on ws.side (the
+// caller waits for ws.join_ev); S.w_heavy and S.w_queue are allocated, the
+// CSR row pointer is written, B's rows strictly increase
+int numeric_rowwin_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
+                          const NumericConfig &cfg);
 struct HybridDev;
 // numeric step on the FP64 tensor cores from hybrid leaves of A's and B's CSR
 // (A.csr_*, B.csr_*; the leaves are built into LA / LB): C's 16x16 tiles

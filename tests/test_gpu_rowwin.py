@@ -1,0 +1,100 @@
+"""Heavy C tile rows, one scalar row per warp (csrc/numeric_rowwin.cu), where
+its windows, pieces and cursors can go wrong: rows of exactly one window's
+entries or tiles and one more or less, tile columns further apart than one
+column index spans, rows with more A entries than the kept places, rows cut
+into pieces.  Bitwise equal to the tile-row kernel's windows
+(split_target = -1), and within the bound of the oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import rtt_spgemm as R
+from conftest import assert_csr_close
+from rtt_spgemm import generators as G
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+DEV = torch.device("cuda:0")
+
+
+def _rows(lists, n, seed):
+    """CSR whose row i has the columns lists[i]."""
+    rng = np.random.default_rng(seed)
+    cnt = [len(c) for c in lists]
+    rp = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+    col = np.concatenate([np.sort(np.asarray(c)) for c in lists]).astype(np.int32)
+    return G.CSR(len(lists), n, rp, col, rng.uniform(-1, 1, col.size))
+
+
+def _pick(m, per, k, seed):
+    rng = np.random.default_rng(seed)
+    return _rows([rng.choice(k, min(per, k), replace=False) for _ in range(m)], k, seed)
+
+
+def _entries():
+    # C rows of 511 .. 1025 entries (windows of 512 or 1024), two B rows each
+    sizes = [511, 512, 513, 1023, 1024, 1025, 600, 1] * 4
+    b = _rows([np.arange(7 * i, 7 * i + s) for i, s in enumerate(sizes)] +
+              [np.arange(7 * i, 7 * i + s, 3) for i, s in enumerate(sizes)], 1300, 1)
+    return _rows([[i, i + 32] for i in range(32)], 64, 2), b
+
+
+def _tiles():
+    # C rows of 255 .. 513 tiles with one entry each (windows of 256 or 512)
+    sizes = [255, 256, 257, 511, 512, 513, 8, 7] * 4
+    b = _rows([16 * np.arange(i, i + s) + i % 16 for i, s in enumerate(sizes)], 16 * 700, 3)
+    return _rows([[i] for i in range(32)], 32, 4), b
+
+
+def _spans():
+    # a cluster of tiles, then tiles further apart than 512 * 32 tile columns
+    # span 8 of them; and single entries around the end of one span
+    n = 16 * 300000
+    far = [np.concatenate([np.arange(0, 1600, 16), 16 * np.arange(1000 + i, 290000, 8700)])
+           for i in range(30)]
+    edge = 16 * 32 * 512
+    far += [[0, edge - 1, edge, edge + 1, 2 * edge], list(range(edge - 800, edge + 800))]
+    return _pick(40, 6, 32, 5), _rows(far, n, 6)
+
+
+def _long():
+    # 3,000 A entries per row (places kept for 2,048), C rows of many windows
+    rng = np.random.default_rng(7)
+    b = _rows([rng.choice(9000, 40, replace=False) for _ in range(6000)], 9000, 8)
+    return _pick(20, 3000, 6000, 9), b
+
+
+def _hub():
+    # power-law rows: pieces cut by weight
+    a = G.rmat(12, 16, seed=3)
+    return a, a
+
+
+CASES = {"entries": _entries, "tiles": _tiles, "spans": _spans, "long": _long, "hub": _hub}
+
+
+def _run(a, b, cfg):
+    ctx = R.Context(0, cfg)
+    t = [(x.m, x.n, *(torch.from_numpy(v).to(DEV) for v in (x.rowptr, x.col, x.val)))
+         for x in (a, b)]
+    nnz, _ = ctx.symbolic(t[0], t[1])
+    out = (torch.full((a.m + 1,), -1, dtype=torch.int32, device=DEV),
+           torch.full((nnz,), -1, dtype=torch.int32, device=DEV),
+           torch.full((nnz,), float("nan"), dtype=torch.float64, device=DEV))
+    ctx.numeric(*out)
+    st = ctx.stats()
+    ctx.close()
+    return [x.cpu().numpy() for x in out], st
+
+
+@pytest.mark.parametrize("case", list(CASES))
+def test_row_windows(case, orc):
+    a, b = CASES[case]()
+    want, st0 = _run(a, b, dict(split_target=-1))
+    for target in (0, 1, 1 << 16):
+        got, st = _run(a, b, dict(split_target=target))
+        assert st["split_windows"] > 0 and st["nnz_cub"] == st0["nnz_cub"]
+        for g, w in zip(got, want):
+            assert np.array_equal(g.view(np.int32), w.view(np.int32)), (case, target)
+    assert_csr_close(*want, *orc.spgemm_csr(a, b), case)
