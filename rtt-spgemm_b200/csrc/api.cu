@@ -1755,7 +1755,7 @@ int rtt_tile_heatmap(rtt_context c, int which, int bins, unsigned long long *his
     Workspace &ws = c->ws;
     const TileBufs &TB = c->b_alias ? c->A : c->B;
     int tilem = 0, tilen = 0;
-    const int *tp = nullptr, *tc = nullptr;
+    const int *tp = nullptr, *te = nullptr, *tc = nullptr;
     if (which == 2)
     {
         tilem = c->S.tilem;
@@ -1769,11 +1769,12 @@ int rtt_tile_heatmap(rtt_context c, int which, int bins, unsigned long long *his
         tilem = T.tilem;
         tilen = T.tilen;
         tp = T.tile_ptr.as<int>();
+        te = T.payload ? nullptr : T.tile_end.as<int>();
         tc = T.tile_col.as<int>();
     }
     const size_t cells = (size_t)bins * bins;
     RTT_CHECK(c->diag_hist.ensure(sizeof(unsigned long long) * cells, ws.stream));
-    RTT_CHECK(tile_heatmap_device(ws, tilem, tilen, tp, tc, bins,
+    RTT_CHECK(tile_heatmap_device(ws, tilem, tilen, tp, te, tc, bins,
                                   c->diag_hist.as<unsigned long long>()));
     RTT_CUDA(cudaMemcpyAsync(hist, c->diag_hist.p, sizeof(unsigned long long) * cells,
                              cudaMemcpyDeviceToHost, ws.stream));

@@ -20,6 +20,7 @@
 #include "rtt_internal.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
+#include <algorithm>
 #include <climits>
 
 namespace rtt
@@ -28,98 +29,381 @@ namespace
 {
 
 // ------------------------------------------------------------ validation
+// The checks and the row segments go over the entries, not the rows: a warp
+// takes a chunk of consecutive entries, 256 at a time, whatever rows they
+// belong to, so hub rows and empty rows cost what their entries cost.  (A warp
+// per 32 rows left the 32 hub rows of an R-MAT matrix to one warp: 460 us for
+// the checks of R-MAT 2^16's 1M entries and 1 ms for its segments; now 14 and
+// 19 us.  96^3 stencil, 23.4M entries: 45 us and 110 us before, 44 and 124 us.)  The row starts among the 256 entries are marked in a shared bitmap.
+constexpr int CS_WARPS = 8, CS_THREADS = CS_WARPS * 32;
+constexpr int CS_BLOCK = 256, CS_WORDS = CS_BLOCK / 32;
+constexpr int CS_CTAS_MAX = 4096; // CTAs of entries, at most
+
+// First index in [0, n) with a[i] >= key, by one warp 32 probes at a time (a
+// need not be sorted: then some index).
+__device__ __forceinline__ int warp_lower_bound(const int *__restrict__ a, int n, long long key)
+{
+    int lo = 0, hi = n; // the answer lies in [lo, hi]
+    while (hi - lo > 0)
+    {
+        const int step = (hi - lo + 31) / 32;
+        const long long i = lo + (long long)lane_id() * step;
+        const unsigned less = __ballot_sync(FULL, i < hi && __ldg(a + min(i, (long long)n - 1)) < key);
+        const int k = __popc(less); // probes below key, the first k of a sorted list
+        if (k == 0)
+            return lo;
+        const long long nlo = lo + (long long)(k - 1) * step + 1;
+        hi = (int)min((long long)hi, lo + (long long)k * step);
+        lo = (int)min(nlo, (long long)hi);
+    }
+    return lo;
+}
+
+// Marks the rows that start in [s0, end), from row `cursor` on (the first that
+// starts at or past s0), in the warp's cleared bitmap; returns the first row
+// that starts at or past end.
+__device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__ rowptr, int rows,
+                                         int cursor, long long s0, long long end)
+{
+    const int lane = lane_id();
+    if (lane < CS_WORDS)
+        bits[lane] = 0u;
+    __syncwarp();
+    for (;;)
+    {
+        const int r = cursor + lane;
+        const long long x = r < rows ? (long long)__ldg(rowptr + r) : LLONG_MAX;
+        const bool in = x < end;
+        if (in && x >= s0)
+            atomicOr(&bits[(x - s0) >> 5], 1u << ((x - s0) & 31));
+        const int n = __popc(__ballot_sync(FULL, in));
+        cursor += n;
+        if (n < 32)
+            break;
+    }
+    __syncwarp();
+    return cursor;
+}
+
+// Row pointer and column checks, the flags, and how many row segments start in
+// each warp's chunk (warp_cnt) and each CTA's (cta_cnt), when not null.
 // flags[0]: some row's tile column decreases (needs the generic path)
 // flags[1]: some row's column decreases (entries not sorted inside rows)
 // flags[2]: some row repeats a column
-// One warp per 32 consecutive rows.  Rows of at most 256 entries: each lane
-// walks its own row.  A warp with a longer row walks the rows' entries, one
-// contiguous range, 32 at a time instead (a hub row costs len / 32 steps, not
-// len): a lane compares its entry with the one before unless the entry starts
-// a row; the row starts inside a step are one OR-reduced bit mask.
-__global__ void k_validate_csr(int m, int n, int nnz, const int *__restrict__ rowptr,
-                               const int *__restrict__ col, int *err, int *flags)
+__global__ void __launch_bounds__(CS_THREADS)
+    k_csr_scan(int m, int n, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
+               int ctas, int blocks, int *__restrict__ cta_cnt, int *__restrict__ warp_cnt,
+               int *err, int *flags)
 {
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (gw == 0 && lane == 0 && (rowptr[0] != 0 || rowptr[m] != nnz))
-        set_error(err, DERR_CSR_ROWPTR);
-    if (gw * 32 >= m)
-        return; // whole warp
-    const int r = (int)(gw * 32) + lane;
-    int b = 0, e = 0;
+    __shared__ uint32_t s_bits[CS_WARPS][CS_WORDS];
+    __shared__ int s_total;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     bool bad = false;
-    if (r < m)
+    for (long long r = blockIdx.x * (long long)CS_THREADS + tid; r < m;
+         r += (long long)gridDim.x * CS_THREADS)
     {
-        b = rowptr[r];
-        e = rowptr[r + 1];
-        bad = b < 0 || e < b || e > nnz;
+        const int b = rowptr[r], e = rowptr[r + 1];
+        bad |= b < 0 || e < b || e > nnz || (r == 0 && b != 0) || (r == m - 1 && e != nnz);
     }
-    if (__any_sync(FULL, bad))
+    if (tid == 0)
+        s_total = 0;
+    if (__syncthreads_or(bad))
     {
-        if (lane == 0)
+        if (tid == 0)
             set_error(err, DERR_CSR_ROWPTR);
         return;
     }
-    const int rows = min(32, m - (int)(gw * 32));
-    const int lo = __shfl_sync(FULL, b, 0), hi = __shfl_sync(FULL, e, rows - 1);
+    if ((int)blockIdx.x >= ctas)
+        return;
+    const long long span = (long long)blocks * CS_BLOCK;
+    const long long c0 = (blockIdx.x * (long long)CS_WARPS + warp) * span;
+    const long long c1 = min((long long)nnz, c0 + span);
+    int segs = 0;
     bool col_bad = false, tile_dec = false, col_dec = false, col_dup = false;
-    if (__reduce_max_sync(FULL, (unsigned)(e - b)) <= 256)
+    if (c0 < c1)
     {
-        // short rows: each lane walks its own row (the warp's rows share
-        // their cache lines)
-        int prev = -1;
-        for (int j = b; j < e; ++j)
+        uint32_t *bits = s_bits[warp];
+        const bool vec = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
+        int cursor = warp_lower_bound(rowptr, m, c0);
+        for (long long s0 = c0; s0 < c1; s0 += CS_BLOCK)
         {
-            const int c = __ldg(col + j);
-            if (c < 0 || c >= n)
+            // a lane's 4 neighbouring entries, twice
+            int4 v[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
             {
-                col_bad = true;
-                break;
+                const long long j = s0 + h * 128 + lane * 4;
+                if (vec && j + 4 <= c1)
+                    v[h] = __ldg(reinterpret_cast<const int4 *>(col + j));
+                else
+                    v[h] = make_int4(j < c1 ? __ldg(col + j) : 0, j + 1 < c1 ? __ldg(col + j + 1) : 0,
+                                     j + 2 < c1 ? __ldg(col + j + 2) : 0,
+                                     j + 3 < c1 ? __ldg(col + j + 3) : 0);
             }
-            if (prev >= 0)
+            int last = s0 > 0 ? __ldg(col + s0 - 1) : 0;
+            cursor = mark_rows(bits, rowptr, m, cursor, s0, min(c1, s0 + CS_BLOCK));
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
             {
-                tile_dec |= (c >> 4) < (prev >> 4);
-                col_dec |= c < prev;
-                col_dup |= c == prev;
-            }
-            prev = c;
-        }
-    }
-    else
-    {
-        // a long row: the warp walks its rows' entry range 32 at a time
-        for (long long c0 = lo; c0 < hi; c0 += 32)
-        {
-            const bool here = r < m && b >= c0 && b < c0 + 32;
-            const unsigned starts = __reduce_or_sync(FULL, here ? 1u << (int)(b - c0) : 0u);
-            const int j = (int)c0 + lane;
-            if (j < hi)
-            {
-                const int c = __ldg(col + j);
-                if (c < 0 || c >= n)
-                    col_bad = true;
-                else if (((starts >> lane) & 1u) == 0)
+                const long long j = s0 + h * 128 + lane * 4;
+                unsigned st = bits[h * 4 + (lane >> 3)] >> ((lane & 7) * 4);
+                if (j == 0)
+                    st |= 1u;
+                int p = __shfl_up_sync(FULL, v[h].w, 1);
+                if (lane == 0)
+                    p = last;
+                last = __shfl_sync(FULL, v[h].w, 31);
+                const int c[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+                const int k = (int)max(0ll, min(4ll, c1 - j)); // entries of the chunk
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
                 {
-                    const int p = __ldg(col + j - 1); // same row, j - 1 >= lo
-                    tile_dec |= (c >> 4) < (p >> 4);
-                    col_dec |= c < p;
-                    col_dup |= c == p;
+                    const bool in = i < k, start = (st >> i) & 1u;
+                    col_bad |= in && (unsigned)c[i] >= (unsigned)n;
+                    if (in && !start && c[i] <= p)
+                    {
+                        tile_dec |= (c[i] >> 4) < (p >> 4);
+                        col_dec |= c[i] < p;
+                        col_dup |= c[i] == p;
+                    }
+                    segs += in && (start || (unsigned)(c[i] ^ p) >= 16u);
+                    p = c[i];
                 }
             }
+            __syncwarp(); // before the bitmap is cleared
         }
     }
-    if (__any_sync(FULL, col_bad) && lane == 0)
-        set_error(err, DERR_CSR_COL);
-    const bool td = __any_sync(FULL, tile_dec), cd = __any_sync(FULL, col_dec),
-               dp = __any_sync(FULL, col_dup);
+    const unsigned fl = __reduce_or_sync(FULL, (tile_dec ? 1u : 0u) | (col_dec ? 2u : 0u) |
+                                                   (col_dup ? 4u : 0u) | (col_bad ? 8u : 0u));
+    if (lane == 0 && fl != 0u)
+    {
+        if (fl & 8u)
+            set_error(err, DERR_CSR_COL);
+        for (int f = 0; f < 3; ++f)
+            if ((fl >> f) & 1u)
+                atomicOr(&flags[f], 1);
+    }
+    if (cta_cnt == nullptr)
+        return;
+    segs = warp_sum(segs);
     if (lane == 0)
     {
-        if (td)
-            atomicOr(&flags[0], 1);
-        if (cd)
-            atomicOr(&flags[1], 1);
-        if (dp)
-            atomicOr(&flags[2], 1);
+        warp_cnt[blockIdx.x * CS_WARPS + warp] = segs;
+        atomicAdd(&s_total, segs);
+    }
+    __syncthreads();
+    if (tid == 0)
+        cta_cnt[blockIdx.x] = s_total;
+}
+
+// Row segments of a CSR whose rows have non-decreasing tile columns: every
+// maximal run of a row's entries inside one tile column J becomes the segment
+// (J << 16) | mask, mask bit (15 - c) for each column c of the run - the row's
+// 16-bit row mask in tile J, as csr2tile writes it into mask[].  A run's mask
+// is OR-ed over the lanes of its 32 entries by shuffles; what it has in the
+// next 32 is carried along, and past the warp's chunk it is followed entry by
+// entry.  seg_ptr[r] is the number of segments before row r's first entry.
+// Nothing is written for a CSR with errors.
+__global__ void __launch_bounds__(CS_THREADS)
+    k_csr_segments(int m, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
+                   int blocks, const int *__restrict__ cta_cnt, const int *__restrict__ warp_cnt,
+                   int *__restrict__ seg_ptr, unsigned long long *__restrict__ seg,
+                   const int *err)
+{
+    __shared__ uint32_t s_bits[CS_WARPS][CS_WORDS], s_starts[CS_WARPS][CS_WORDS];
+    __shared__ int s_pre[CS_WARPS][CS_WORDS], s_base;
+    if (*(volatile const int *)err != 0)
+        return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // segments of the CTAs and warps before
+    if (tid == 0)
+        s_base = 0;
+    __syncthreads();
+    int before = 0;
+    for (int i = tid; i < (int)blockIdx.x; i += CS_THREADS)
+        before += __ldg(cta_cnt + i);
+    before = warp_sum(before);
+    if (lane == 0 && before)
+        atomicAdd(&s_base, before);
+    const int wc = lane < warp ? __ldg(warp_cnt + blockIdx.x * CS_WARPS + lane) : 0;
+    __syncthreads();
+    int base = s_base + warp_sum(wc);
+    const long long span = (long long)blocks * CS_BLOCK;
+    const long long c0 = (blockIdx.x * (long long)CS_WARPS + warp) * span;
+    const long long c1 = min((long long)nnz, c0 + span);
+    if (c0 >= c1)
+        return;
+    uint32_t *bits = s_bits[warp], *starts = s_starts[warp];
+    int *pre = s_pre[warp];
+    int cursor = warp_lower_bound(rowptr, m, c0);
+    // the run that is open at the end of the last 32 entries
+    int open_at = -1, open_T = 0;
+    unsigned open_mk = 0;
+    for (long long s0 = c0; s0 < c1; s0 += CS_BLOCK)
+    {
+        int c[CS_WORDS];
+#pragma unroll
+        for (int i = 0; i < CS_WORDS; ++i)
+            c[i] = s0 + i * 32 + lane < c1 ? __ldg(col + s0 + i * 32 + lane) : 0;
+        int last = s0 > 0 ? __ldg(col + s0 - 1) : 0;
+        const int first = cursor;
+        cursor = mark_rows(bits, rowptr, m, cursor, s0, min(c1, s0 + CS_BLOCK));
+        int n = 0; // segments of the block so far
+#pragma unroll
+        for (int i = 0; i < CS_WORDS; ++i)
+        {
+            const long long j = s0 + i * 32 + lane;
+            int p = __shfl_up_sync(FULL, c[i], 1);
+            if (lane == 0)
+                p = last;
+            last = __shfl_sync(FULL, c[i], 31);
+            const bool in = j < c1;
+            const bool start = in && (j == 0 || ((bits[i] >> lane) & 1u) || (c[i] >> 4) != (p >> 4));
+            const unsigned st = __ballot_sync(FULL, start);
+            if (lane == 0)
+            {
+                starts[i] = st;
+                pre[i] = n;
+            }
+            unsigned mk = in ? 0x8000u >> (c[i] & 15) : 0u;
+            // entries before the first start belong to the open run
+            const int fs = st ? __ffs(st) - 1 : 32;
+            open_mk |= __reduce_or_sync(FULL, lane < fs ? mk : 0u);
+            if (st != 0u)
+            {
+                // OR over the lanes up to the next start
+                const unsigned later = lane == 31 ? 0u : st >> (lane + 1);
+                const int next = later ? lane + __ffs(later) : 32;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1)
+                {
+                    const unsigned v = __shfl_down_sync(FULL, mk, o);
+                    if (lane + o < next)
+                        mk |= v;
+                }
+                const int lst = 31 - __clz(st), at = base + n + __popc(st & ((1u << lane) - 1u));
+                if (start && lane != lst)
+                    seg[at] = ((unsigned long long)(c[i] >> 4) << 16) | mk;
+                if (lane == 0 && open_at >= 0)
+                    seg[open_at] = ((unsigned long long)open_T << 16) | open_mk;
+                open_at = base + n + __popc(st) - 1;
+                open_T = __shfl_sync(FULL, c[i] >> 4, lst);
+                open_mk = __shfl_sync(FULL, mk, lst);
+                n += __popc(st);
+            }
+        }
+        __syncwarp();
+        for (int r = first + lane; r < cursor; r += 32)
+        {
+            const int d = (int)(__ldg(rowptr + r) - s0);
+            seg_ptr[r] = base + pre[d >> 5] + __popc(starts[d >> 5] & ((1u << (d & 31)) - 1u));
+        }
+        base += n;
+        __syncwarp(); // before the bitmaps are written again
+    }
+    if (open_at >= 0)
+    {
+        // the last run's entries past the chunk: up to the next row's start
+        // (row `cursor`) or another tile column
+        const long long stop = min((long long)nnz, cursor <= m ? (long long)__ldg(rowptr + cursor)
+                                                               : (long long)nnz);
+        for (long long t0 = c1;; t0 += 32)
+        {
+            const long long t = t0 + lane;
+            const int ct = t < stop ? __ldg(col + t) : -1;
+            const unsigned out = __ballot_sync(FULL, ct < 0 || (ct >> 4) != open_T);
+            const int k = out ? __ffs(out) - 1 : 32;
+            open_mk |= __reduce_or_sync(FULL, lane < k ? 0x8000u >> (ct & 15) : 0u);
+            if (out)
+                break;
+        }
+        if (lane == 0)
+            seg[open_at] = ((unsigned long long)open_T << 16) | open_mk;
+    }
+    // after the last entry: empty rows, and the total
+    if (c1 == nnz)
+        for (int r = cursor + lane; r <= m; r += 32)
+            seg_ptr[r] = base;
+}
+
+// Tile index of every tile row from its rows' segments: the tile columns of
+// its segments as a bitmap, a warp per tile row, windows of ST_BITS tile
+// columns.  Tile row I's list starts at its first segment, so its place needs
+// no count of the tiles before it: tile_ptr[I] = seg_ptr[16 I], tile_end[I] one
+// past its last tile.  out[0] += tiles, out[1] = the most segments of a row.
+constexpr int ST_WARPS = 4, ST_WORDS = 256, ST_BITS = ST_WORDS * 32;
+__global__ void __launch_bounds__(ST_WARPS * 32)
+    k_seg_tiles(int m, int tilem, const int *__restrict__ seg_ptr,
+                const unsigned long long *__restrict__ seg, int *__restrict__ tile_ptr,
+                int *__restrict__ tile_end, int *__restrict__ tile_col, int *out, const int *err)
+{
+    __shared__ uint32_t s_bits[ST_WARPS][ST_WORDS];
+    __shared__ int s_count, s_max;
+    if (*(volatile const int *)err != 0)
+        return;
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const int I = blockIdx.x * ST_WARPS + warp;
+    uint32_t *bits = s_bits[warp];
+    if (threadIdx.x == 0)
+        s_count = s_max = 0;
+    __syncthreads();
+    if (I < tilem)
+    {
+        // lane r < 16: row r's segments
+        const int r = min(I * TD + lane, m), r1 = min(r + 1, m);
+        const int p = lane < TD ? __ldg(seg_ptr + r) : 0;
+        const int e = lane < TD ? __ldg(seg_ptr + r1) : 0;
+        const int s0 = __shfl_sync(FULL, p, 0), s1 = __shfl_sync(FULL, e, TD - 1);
+        int lo = INT_MAX, hi = -1;
+        if (p < e)
+        {
+            lo = (int)(__ldg(seg + p) >> 16);
+            hi = (int)(__ldg(seg + e - 1) >> 16);
+        }
+        lo = warp_min(lo);
+        hi = warp_max(hi);
+        const int most = (int)__reduce_max_sync(FULL, (unsigned)(e - p));
+        int n = 0;
+        for (long long w = lo; w <= hi; w += ST_BITS)
+        {
+            const int nwords = (int)((min((long long)hi + 1, w + ST_BITS) - w + 31) >> 5);
+            for (int i = lane; i < nwords; i += 32)
+                bits[i] = 0u;
+            __syncwarp();
+#pragma unroll 4
+            for (int q = s0 + lane; q < s1; q += 32)
+            {
+                const long long d = (long long)(__ldg(seg + q) >> 16) - w;
+                if (d >= 0 && d < 32ll * nwords)
+                    atomicOr(&bits[d >> 5], 1u << (d & 31));
+            }
+            __syncwarp();
+            for (int q0 = 0; q0 < nwords; q0 += 32)
+            {
+                uint32_t word = q0 + lane < nwords ? bits[q0 + lane] : 0u;
+                const int v = __popc(word), incl = warp_incl_scan(v);
+                int at = s0 + n + incl - v;
+                for (; word != 0u; word &= word - 1u)
+                    tile_col[at++] = (int)w + (q0 + lane) * 32 + __ffs(word) - 1;
+                n += __shfl_sync(FULL, incl, 31);
+            }
+            __syncwarp();
+        }
+        if (lane == 0)
+        {
+            tile_ptr[I] = s0;
+            tile_end[I] = s0 + n;
+            atomicAdd(&s_count, n);
+            atomicMax(&s_max, most);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        if (s_count > 0)
+            atomicAdd(&out[0], s_count);
+        if (s_max > *(volatile int *)&out[1])
+            atomicMax(&out[1], s_max);
     }
 }
 
@@ -237,178 +521,6 @@ __global__ void __launch_bounds__(256) k_c2t_fill(int m, int tilem, const int *_
 }
 
 // ------------------------------------------------------------ row segments
-// Row segments of a CSR whose rows have non-decreasing tile columns: every
-// maximal run of a row's entries inside one tile column J becomes the segment
-// (J << 16) | mask, mask bit (15 - c) for each column c of the run - the row's
-// 16-bit row mask in tile J, as csr2tile writes it into mask[].  One warp per
-// 32 consecutive rows (as k_validate_csr): each lane walks its own row when
-// the warp's rows are short; a warp holding a long row walks its rows one
-// after another, 32 entries at a time, and a segment is counted (and written)
-// by the lane that holds its first entry.
-__device__ __forceinline__ unsigned long long seg_pack(int T, unsigned mk)
-{
-    return ((unsigned long long)T << 16) | (mk & 0xFFFFu);
-}
-
-template <bool FILL>
-__global__ void __launch_bounds__(256)
-    k_row_segments(int m, const int *__restrict__ rowptr, const int *__restrict__ col,
-                   int *__restrict__ seg_cnt, const int *__restrict__ seg_ptr,
-                   unsigned long long *__restrict__ seg)
-{
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (gw * 32 >= m)
-        return; // whole warp
-    const int r0 = (int)(gw * 32), r = r0 + lane;
-    int b = 0, e = 0;
-    if (r < m)
-    {
-        b = rowptr[r];
-        e = rowptr[r + 1];
-    }
-    if (__reduce_max_sync(FULL, (unsigned)(e - b)) <= 256)
-    {
-        const int out = FILL && r < m ? seg_ptr[r] : 0;
-        int n = 0, T = -1;
-        unsigned mk = 0;
-        for (int j = b; j < e; ++j)
-        {
-            const int c = __ldg(col + j);
-            if ((c >> 4) != T)
-            {
-                if (T >= 0)
-                {
-                    if (FILL)
-                        seg[out + n] = seg_pack(T, mk);
-                    ++n;
-                }
-                T = c >> 4;
-                mk = 0;
-            }
-            mk |= 0x8000u >> (c & 15);
-        }
-        if (T >= 0)
-        {
-            if (FILL)
-                seg[out + n] = seg_pack(T, mk);
-            ++n;
-        }
-        if (!FILL)
-        {
-            if (r < m)
-                seg_cnt[r] = n;
-            // seg_cnt[m]: the most segments of a row
-            const unsigned wmax = __reduce_max_sync(FULL, r < m ? (unsigned)n : 0u);
-            if (lane == 0 && wmax > 0)
-                atomicMax(seg_cnt + m, (int)wmax);
-        }
-        return;
-    }
-    const int rows = min(32, m - r0);
-    for (int q = 0; q < rows; ++q)
-    {
-        const int qb = __shfl_sync(FULL, b, q), qe = __shfl_sync(FULL, e, q);
-        const int out = FILL ? seg_ptr[r0 + q] : 0;
-        int n = 0;
-        for (int c0 = qb; c0 < qe; c0 += 32)
-        {
-            const int j = c0 + lane;
-            bool start = false;
-            int T = 0;
-            if (j < qe)
-            {
-                T = __ldg(col + j) >> 4;
-                start = j == qb || (__ldg(col + j - 1) >> 4) != T;
-            }
-            const unsigned st = __ballot_sync(FULL, start);
-            if (FILL && start)
-            {
-                unsigned mk = 0;
-                for (int t = j; t < qe; ++t)
-                {
-                    const int c = __ldg(col + t);
-                    if ((c >> 4) != T)
-                        break;
-                    mk |= 0x8000u >> (c & 15);
-                }
-                seg[out + n + __popc(st & ((1u << lane) - 1u))] = seg_pack(T, mk);
-            }
-            n += __popc(st);
-        }
-        if (!FILL && lane == 0)
-        {
-            seg_cnt[r0 + q] = n;
-            atomicMax(seg_cnt + m, n);
-        }
-    }
-}
-
-// Tile structure (no per-entry payload) of a tile row from its rows'
-// segments: the tile columns are the union of the 16 rows' segment columns,
-// taken in ascending order by a half-warp (a lane per row walks its segment
-// list; the half-warp takes the minimum pending column, and the lanes holding
-// it step to their next segment).  FILL = false counts the tiles of each
-// tile row, FILL = true writes tile_col and tile_row from tile_ptr[I].  Tile
-// rows marked heavy are left to k_c2t_heavy_count / k_c2t_heavy_struct.
-template <bool FILL>
-__global__ void __launch_bounds__(256)
-    k_c2t_seg_tiles(int m, int tilem, const int *__restrict__ seg_ptr,
-                    const unsigned long long *__restrict__ seg, const int *__restrict__ tile_ptr,
-                    int *__restrict__ cnt, int *__restrict__ o_tcol, int *__restrict__ o_trow,
-                    int *err, const uint8_t *__restrict__ heavy)
-{
-    const int lane = threadIdx.x & 31, hl = lane & 15;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int I = gw * 2 + (lane >> 4);
-    const bool mine = I < tilem && !(heavy != nullptr && heavy[I]);
-    int p = 0, e = 0, t = 0, tend = 0;
-    if (mine)
-    {
-        if (I * TD + hl < m)
-        {
-            p = seg_ptr[I * TD + hl];
-            e = seg_ptr[I * TD + hl + 1];
-        }
-        if (FILL)
-        {
-            t = tile_ptr[I];
-            tend = tile_ptr[I + 1];
-        }
-    }
-    int cur = p < e ? (int)(__ldg(seg + p) >> 16) : INT_MAX;
-    int count = 0;
-    for (;;)
-    {
-        const int T = half_min(cur);
-        const bool has = T != INT_MAX;
-        if (!__any_sync(FULL, has))
-            break;
-        if (has)
-        {
-            if (FILL && hl == 0)
-            {
-                if (t < tend)
-                {
-                    o_tcol[t] = T;
-                    o_trow[t] = I;
-                }
-                else
-                    set_error(err, DERR_C2T_OVERFLOW);
-            }
-            ++t;
-            ++count;
-            if (cur == T)
-            {
-                ++p;
-                cur = p < e ? (int)(__ldg(seg + p) >> 16) : INT_MAX;
-            }
-        }
-    }
-    if (!FILL && mine && hl == 0)
-        cnt[I] = count;
-}
-
 // ------------------------------------------------ fast path, heavy tile rows
 // A tile row holding a row with thousands of entries (an R-MAT hub) spans
 // thousands of tile columns; the half-warp above takes them one per step and
@@ -563,37 +675,6 @@ __global__ void __launch_bounds__(HV_THREADS)
         if (threadIdx.x == 0)
             cnt[I] = S.count;
         __syncthreads();
-    }
-}
-
-// Structure only (no per-entry payload) of the heavy tile rows: tile
-// columns are the bitmap's set bits in order.
-__global__ void __launch_bounds__(HV_THREADS)
-    k_c2t_heavy_struct(int m, const int *__restrict__ list, const int *__restrict__ count,
-                       const int *__restrict__ rowptr, const int *__restrict__ col,
-                       const int *__restrict__ tile_ptr, int *__restrict__ o_tcol,
-                       int *__restrict__ o_trow, int *err)
-{
-    extern __shared__ __align__(16) unsigned char hv_dyn[];
-    HeavySmem &S = *reinterpret_cast<HeavySmem *>(hv_dyn);
-    const int n = *count;
-    for (int li = blockIdx.x; li < n; li += gridDim.x)
-    {
-        const int I = list[li];
-        heavy_bitmap(S, I, m, rowptr, col);
-        const int ntiles = S.count, t0 = tile_ptr[I];
-        if (t0 + ntiles != tile_ptr[I + 1])
-        {
-            if (threadIdx.x == 0)
-                set_error(err, DERR_C2T_OVERFLOW);
-        }
-        else
-            for (int k = threadIdx.x; k < ntiles; k += HV_THREADS)
-            {
-                o_tcol[t0 + k] = heavy_select(S, k);
-                o_trow[t0 + k] = I;
-            }
-        __syncthreads(); // the bitmap is rebuilt for the next tile row
     }
 }
 
@@ -988,13 +1069,15 @@ __global__ void k_copy_tiles_colmajor(int n, const int *__restrict__ order,
 }
 
 // ----------------------------------------------------------- CSR transpose
+// A warp per row (a thread per row left an R-MAT hub row to one thread: 64 us
+// at 2^16, now 12).
 __global__ void k_row_ids(int m, const int *__restrict__ rowptr, int *__restrict__ rows)
 {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     if (r >= m)
         return;
-    for (int j = rowptr[r]; j < rowptr[r + 1]; ++j)
-        rows[j] = r;
+    for (int j = rowptr[r] + lane_id(), e = rowptr[r + 1]; j < e; j += 32)
+        rows[j] = (int)r;
 }
 
 __global__ void k_gather_transpose(int nnz, const int *__restrict__ order,
@@ -1035,6 +1118,28 @@ int sort_pairs(Workspace &ws, const int *keys_in, int *keys_out, const int *vals
 
 inline int grid_for(long long threads, int block) { return (int)((threads + block - 1) / block); }
 
+// The warps' chunks of k_csr_scan and k_csr_segments: `blocks` times 256
+// entries each.  One block for small matrices, so that they spread over the
+// SMs; up to 8, where a chunk's own set-up (its first row, the segments before
+// it) is spread over more entries, while every SM keeps 8 CTAs (64^3 stencil:
+// the scan 18 us against 24 with one block); more only to stay within
+// CS_CTAS_MAX.
+struct CsChunks
+{
+    int blocks, ctas;
+    explicit CsChunks(int nnz)
+    {
+        const int all = ceil_div(ceil_div(nnz, CS_BLOCK), CS_WARPS); // CTAs of one block a warp
+        blocks = std::max(std::max(1, std::min(8, all / 1200)), ceil_div(all, CS_CTAS_MAX));
+        ctas = ceil_div(all, blocks);
+    }
+    // CTAs of the scan: those of the entries, and enough for the row pointer
+    int grid(int m) const
+    {
+        return std::max(1, std::max(ctas, std::min(1024, ceil_div(m, 4 * CS_THREADS))));
+    }
+};
+
 } // namespace
 
 int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, const int *col,
@@ -1055,9 +1160,11 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
 
     RTT_CHECK(out.tile_ptr.ensure(sizeof(int) * (tilem + 1), s));
     RTT_CHECK(out.tmp0.ensure(sizeof(int) * (tilem + 1), s));
-    RTT_CHECK(out.tmp1.ensure(sizeof(int) * 4, s));
+    // [0..2] flags of the rows, [3] heavy tile rows listed, [4] tiles, [5] the
+    // most segments of a row
+    RTT_CHECK(out.tmp1.ensure(sizeof(int) * 8, s));
     int *flags = out.tmp1.as<int>();
-    RTT_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * 3, s));
+    RTT_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * 6, s));
     if (m == 0)
     {
         RTT_CUDA(cudaMemsetAsync(out.tile_ptr.p, 0, sizeof(int), s));
@@ -1073,38 +1180,68 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
         RTT_CHECK(out.val.ensure(tiny, s));
         return RTT_OK;
     }
-    k_validate_csr<<<grid_for((long long)ceil_div(m, 32) * 32, 256), 256, 0, s>>>(
-        m, n, nnz, rowptr, col, ws.err.as<int>(), flags);
+    const CsChunks ch(nnz);
+    const bool want_segs = segments || !payload;
+    if (want_segs)
+    {
+        RTT_CHECK(out.seg_cnt.ensure(sizeof(int) * ((size_t)ch.ctas * (CS_WARPS + 1) + 1), s));
+        RTT_CHECK(out.seg_ptr.ensure(sizeof(int) * ((size_t)m + 1), s));
+        // at most one segment per entry: sized by nnz, no host read
+        RTT_CHECK(out.seg.ensure(sizeof(unsigned long long) * ((size_t)nnz + 1), s));
+    }
+    if (!payload)
+    {
+        RTT_CHECK(out.tile_end.ensure(sizeof(int) * (size_t)tilem + 16, s));
+        // a tile per segment at most: sized by nnz, no host read
+        RTT_CHECK(out.tile_col.ensure(sizeof(int) * (size_t)nnz + 16, s));
+    }
+    // segments starting in each CTA's and each warp's entries
+    int *cta_cnt = want_segs ? out.seg_cnt.as<int>() : nullptr;
+    int *warp_cnt = want_segs ? cta_cnt + ch.ctas : nullptr;
+    k_csr_scan<<<ch.grid(m), CS_THREADS, 0, s>>>(m, n, nnz, rowptr, col, ch.ctas, ch.blocks,
+                                                 cta_cnt, warp_cnt, ws.err.as<int>(), flags);
     ws.launches++;
-    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 4, flags, sizeof(int) * 3, cudaMemcpyDeviceToHost, s));
+    // the segments and the tile index are made before the host sees the flags
+    // (every run of entries in one tile column is a segment, sorted or not),
+    // so that one synchronisation brings flags, errors and sizes
+    if (want_segs)
+    {
+        if (nnz > 0)
+        {
+            k_csr_segments<<<ch.ctas, CS_THREADS, 0, s>>>(
+                m, nnz, rowptr, col, ch.blocks, cta_cnt, warp_cnt, out.seg_ptr.as<int>(),
+                out.seg.as<unsigned long long>(), ws.err.as<int>());
+            ws.launches++;
+        }
+        else
+            RTT_CUDA(cudaMemsetAsync(out.seg_ptr.p, 0, sizeof(int) * ((size_t)m + 1), s));
+    }
+    if (!payload)
+    {
+        k_seg_tiles<<<ceil_div(tilem, ST_WARPS), ST_WARPS * 32, 0, s>>>(
+            m, tilem, out.seg_ptr.as<int>(), out.seg.as<unsigned long long>(),
+            out.tile_ptr.as<int>(), out.tile_end.as<int>(), out.tile_col.as<int>(), flags + 4,
+            ws.err.as<int>());
+        ws.launches++;
+    }
+    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 2, flags, sizeof(int) * 6, cudaMemcpyDeviceToHost, s));
     RTT_CHECK(check_device_error(ws, "csr2tile validate"));
-    const bool generic = ws.h_scalars[4] != 0;
-    const bool unsorted = ws.h_scalars[5] != 0;
+    const bool generic = ws.h_scalars[2] != 0;
+    const bool unsorted = ws.h_scalars[3] != 0;
     // rows that are unsorted may hide repeated columns too
-    out.dup_cols = ws.h_scalars[6] != 0 || unsorted;
+    out.dup_cols = ws.h_scalars[4] != 0 || unsorted;
     out.generic = generic;
-    out.has_segments = false;
     // the structure alone comes from the row segments, which need rows whose
     // tile columns never decrease; otherwise the whole tile payload is built
-    const bool structure_only = !payload && !generic;
-    if ((segments || structure_only) && !generic)
+    out.has_segments = want_segs && !generic;
+    if (!payload && !generic)
     {
-        // row segments: count per row, scan, fill
-        RTT_CHECK(out.seg_cnt.ensure(sizeof(int) * ((size_t)m + 1), s));
-        RTT_CHECK(out.seg_ptr.ensure(sizeof(int) * ((size_t)m + 1), s));
-        RTT_CUDA(cudaMemsetAsync(out.seg_cnt.as<int>() + m, 0, sizeof(int), s));
-        const int grid = grid_for((long long)ceil_div(m, 32) * 32, 256);
-        k_row_segments<false><<<grid, 256, 0, s>>>(m, rowptr, col, out.seg_cnt.as<int>(), nullptr,
-                                                   nullptr);
-        ws.launches++;
-        RTT_CHECK(scan_exclusive_int(ws, out.seg_cnt.as<int>(), out.seg_ptr.as<int>(), m));
-        // at most one segment per entry: size by nnz, no host read
-        RTT_CHECK(out.seg.ensure(sizeof(unsigned long long) * ((size_t)nnz + 1), s));
-        k_row_segments<true><<<grid, 256, 0, s>>>(m, rowptr, col, nullptr, out.seg_ptr.as<int>(),
-                                                  out.seg.as<unsigned long long>());
-        ws.launches++;
-        out.has_segments = true;
+        out.numtile = ws.h_scalars[6];
+        out.max_row_segs = ws.h_scalars[7];
+        out.payload = false;
+        return RTT_OK;
     }
+    out.max_row_segs = 0;
 
     int *cnt = out.tmp0.as<int>();
     // heavy tile rows (a CTA each) are listed on the device; their kernels
@@ -1133,39 +1270,6 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
         k_c2t_heavy_count<<<hv_grid, HV_THREADS, hv_smem, s>>>(m, hv_list, hv_count, rowptr, col,
                                                                cnt);
         ws.launches++;
-    }
-    if (structure_only)
-    {
-        // tile_ptr, tile_col and tile_row only (from the row segments)
-        const int grid = grid_for((long long)ceil_div(tilem, 2) * 32, 256);
-        k_c2t_seg_tiles<false><<<grid, 256, 0, s>>>(m, tilem, out.seg_ptr.as<int>(),
-                                                     out.seg.as<unsigned long long>(), nullptr,
-                                                     cnt, nullptr, nullptr, ws.err.as<int>(),
-                                                     heavy);
-        ws.launches++;
-        RTT_CHECK(scan_exclusive_int(ws, cnt, out.tile_ptr.as<int>(), tilem));
-        int numtile = 0;
-        // the most segments of a row comes back with the tile count (one sync)
-        RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 2, out.seg_cnt.as<int>() + m, sizeof(int),
-                                 cudaMemcpyDeviceToHost, s));
-        RTT_CHECK(read_int(ws, out.tile_ptr.as<int>() + tilem, &numtile));
-        out.max_row_segs = ws.h_scalars[2];
-        out.numtile = numtile;
-        RTT_CHECK(out.tile_col.ensure(sizeof(int) * (size_t)numtile + 16, s));
-        RTT_CHECK(out.tile_row.ensure(sizeof(int) * (size_t)numtile + 16, s));
-        k_c2t_seg_tiles<true><<<grid, 256, 0, s>>>(m, tilem, out.seg_ptr.as<int>(),
-                                                    out.seg.as<unsigned long long>(),
-                                                    out.tile_ptr.as<int>(), nullptr,
-                                                    out.tile_col.as<int>(), out.tile_row.as<int>(),
-                                                    ws.err.as<int>(), heavy);
-        RTT_CUDA(cudaFuncSetAttribute(k_c2t_heavy_struct,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hv_smem));
-        k_c2t_heavy_struct<<<hv_grid, HV_THREADS, hv_smem, s>>>(
-            m, hv_list, hv_count, rowptr, col, out.tile_ptr.as<int>(), out.tile_col.as<int>(),
-            out.tile_row.as<int>(), ws.err.as<int>());
-        ws.launches += 2;
-        out.payload = false;
-        return RTT_OK;
     }
     if (!generic)
         k_c2t_count<<<grid_for((long long)ceil_div(tilem, 2) * 32, 256), 256, 0, s>>>(m, tilem, rowptr,
@@ -1232,7 +1336,7 @@ int csr2tile_refill_device(Workspace &ws, const int *rowptr, const int *col, con
     // the structure arrays with the same bytes and the values in tile order
     if (!t.generic)
     {
-        RTT_CHECK(t.tmp1.ensure(sizeof(int) * 4, s));
+        RTT_CHECK(t.tmp1.ensure(sizeof(int) * 8, s));
         RTT_CHECK(t.tmp2.ensure((size_t)tilem + 16, s));
         RTT_CHECK(t.tmp3.ensure(sizeof(int) * (size_t)tilem + 16, s));
         uint8_t *heavy = t.tmp2.as<uint8_t>();
@@ -1273,8 +1377,9 @@ int validate_csr_device(Workspace &ws, int m, int n, int nnz, const int *rowptr,
     RTT_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * 3, ws.stream));
     if (m > 0)
     {
-        k_validate_csr<<<grid_for((long long)ceil_div(m, 32) * 32, 256), 256, 0, ws.stream>>>(
-            m, n, nnz, rowptr, col, ws.err.as<int>(), flags);
+        const CsChunks ch(nnz);
+        k_csr_scan<<<ch.grid(m), CS_THREADS, 0, ws.stream>>>(
+            m, n, nnz, rowptr, col, ch.ctas, ch.blocks, nullptr, nullptr, ws.err.as<int>(), flags);
         ws.launches++;
     }
     RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 4, flags, sizeof(int) * 3, cudaMemcpyDeviceToHost,
@@ -1359,7 +1464,7 @@ int csr_transpose_device(Workspace &ws, int m, int n, int nnz, const int *rowptr
     int *keys = ws.tmp[2].as<int>(), *order = ws.tmp[3].as<int>();
     if (m > 0)
     {
-        k_row_ids<<<grid_for(m, 256), 256, 0, s>>>(m, rowptr, rows);
+        k_row_ids<<<grid_for((long long)m * 32, 256), 256, 0, s>>>(m, rowptr, rows);
         ws.launches++;
     }
     if (nnz > 0)

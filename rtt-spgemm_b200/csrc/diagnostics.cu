@@ -24,6 +24,7 @@ namespace
 // one thread per tile row: every tile (I, J) adds one to bin (I * bins /
 // tilem, J * bins / tilen)
 __global__ void k_tile_heatmap(int tilem, int tilen, int bins, const int *__restrict__ tile_ptr,
+                               const int *__restrict__ tile_end,
                                const int *__restrict__ tile_col,
                                unsigned long long *__restrict__ hist, int *err)
 {
@@ -31,7 +32,8 @@ __global__ void k_tile_heatmap(int tilem, int tilen, int bins, const int *__rest
     if (I >= tilem)
         return;
     const long long bi = (long long)I * bins / tilem;
-    for (int t = tile_ptr[I]; t < tile_ptr[I + 1]; ++t)
+    const int end = tile_end != nullptr ? tile_end[I] : tile_ptr[I + 1];
+    for (int t = tile_ptr[I]; t < end; ++t)
     {
         const int J = tile_col[t];
         if (J < 0 || J >= tilen)
@@ -47,14 +49,14 @@ __global__ void k_tile_heatmap(int tilem, int tilen, int bins, const int *__rest
 } // namespace
 
 int tile_heatmap_device(Workspace &ws, int tilem, int tilen, const int *tile_ptr,
-                        const int *tile_col, int bins, unsigned long long *d_hist)
+                        const int *tile_end, const int *tile_col, int bins, unsigned long long *d_hist)
 {
     RTT_CUDA(cudaMemsetAsync(d_hist, 0, sizeof(unsigned long long) * (size_t)bins * bins,
                              ws.stream));
     if (tilem > 0 && tilen > 0)
     {
         k_tile_heatmap<<<(tilem + 255) / 256, 256, 0, ws.stream>>>(tilem, tilen, bins, tile_ptr,
-                                                                    tile_col, d_hist,
+                                                                    tile_end, tile_col, d_hist,
                                                                     ws.err.as<int>());
         ws.launches++;
     }

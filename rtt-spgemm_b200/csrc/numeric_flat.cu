@@ -545,7 +545,8 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32)
     if (I >= tilem)
         return;
     const int cs0 = __ldg(c_tile_ptr + I), cs1 = __ldg(c_tile_ptr + I + 1);
-    const int a0 = __ldg(A.tile_ptr + I), a1 = __ldg(A.tile_ptr + I + 1);
+    int a0, a1;
+    tile_range(A, I, a0, a1);
     bool multi = false;
     if (cs1 > cs0 && a0 < a1)
     {
@@ -801,7 +802,8 @@ __global__ void __launch_bounds__(F_THREADS, MIN_CTAS)
             if (I >= tilem || (heavy != nullptr && heavy[I]))
                 break;
         }
-        const int a0 = __ldg(A.tile_ptr + I), a1 = __ldg(A.tile_ptr + I + 1);
+        int a0, a1;
+        tile_range(A, I, a0, a1);
         const int cs0 = __ldg(c_tile_ptr + I), cs1 = __ldg(c_tile_ptr + I + 1);
         if (cs0 == cs1 || a0 == a1)
         {

@@ -44,6 +44,7 @@ struct DevTiles
 {
     int m, n, tilem, tilen, numtile, nnz;
     const int *tile_ptr;    // tilem + 1 (row-major structure)
+    const int *tile_end;    // tilem: one past each tile row's last tile (nullptr: tile_ptr[I + 1])
     const int *tile_col;    // numtile
     const int *tile_nnz;    // numtile + 1, offsets into col/val (data order)
     const uint8_t *ptr;     // numtile * 16, exclusive row offsets (data order)
@@ -68,6 +69,13 @@ struct DevTiles
     const unsigned long long *seg;    // seg_ptr[m]
     int max_row_segs;                 // most segments of one row (when seg_ptr is set)
 };
+
+// Tiles [b, e) of tile row I.
+__device__ __forceinline__ void tile_range(const DevTiles &T, int I, int &b, int &e)
+{
+    b = __ldg(T.tile_ptr + I);
+    e = T.tile_end != nullptr ? __ldg(T.tile_end + I) : __ldg(T.tile_ptr + I + 1);
+}
 
 // C tile structure produced by the symbolic phase.
 struct DevCTiles
@@ -241,6 +249,7 @@ void freeze_growth(bool on);
 struct TileBufs
 {
     DevBuf tile_ptr, tile_col, tile_row, tile_nnz, ptr, col, val, mask;
+    DevBuf tile_end; // structure-only builds: tile row I is [tile_ptr[I], tile_end[I])
     DevBuf csc_ptr, csc_row, csc_data, row_data;
     DevBuf tmp0, tmp1, tmp2, tmp3;
     DevBuf seg_ptr, seg, seg_cnt; // row segments (csr2tile_device with segments = true)
@@ -259,7 +268,7 @@ struct TileBufs
         const DevBuf *all[] = {&tile_ptr, &tile_col, &tile_row, &tile_nnz, &ptr,  &col,
                                &val,      &mask,     &csc_ptr,  &csc_row,  &csc_data,
                                &row_data, &tmp0,     &tmp1,     &tmp2,     &tmp3,
-                               &seg_ptr,  &seg,      &seg_cnt};
+                               &seg_ptr,  &seg,      &seg_cnt,  &tile_end};
         for (const DevBuf *b : all)
             f(*b);
     }
@@ -267,7 +276,7 @@ struct TileBufs
 
 // segments: also list the row segments of the CSR (seg_ptr, seg; only when
 // every row's tile columns are non-decreasing, else has_segments stays false).
-// payload = false: only the tile index (tile_ptr, tile_col, tile_row) and the
+// payload = false: only the tile index (tile_ptr, tile_end, tile_col) and the
 // row segments, when the rows allow it (out.payload tells what was built)
 int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, const int *col,
                     const double *val, TileBufs &out, bool packed_col, bool sort_within_rows,
@@ -276,7 +285,7 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
 // from a CSR of the same structure get the values val (no host round trip)
 int csr2tile_refill_device(Workspace &ws, const int *rowptr, const int *col, const double *val,
                            TileBufs &t, bool packed_col);
-// k_validate_csr on the device, then the host reads the error word (syncs):
+// the CSR checks on the device, then the host reads the error word (syncs):
 // RTT_ERR_DEVICE_CHECK code 101/102 for a malformed CSR; flags: 3 device ints
 // (tile column / column decreases in a row, repeated column), copied to
 // ws.h_scalars[4..6]
@@ -364,7 +373,7 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
                          int *cnt);
 // tile counts of a tile grid on a bins x bins histogram (device, cleared first)
 int tile_heatmap_device(Workspace &ws, int tilem, int tilen, const int *tile_ptr,
-                        const int *tile_col, int bins, unsigned long long *d_hist);
+                        const int *tile_end, const int *tile_col, int bins, unsigned long long *d_hist);
 // tile rows [I0, I1) of a device tile matrix with its CSR rows (the 64-bit
 // products run A in such slices; B stays whole)
 DevTiles tile_row_slice(const DevTiles &A, int I0, int I1);

@@ -294,6 +294,7 @@ DevTiles TileBufs::view() const
     t.numtile = numtile;
     t.nnz = nnz;
     t.tile_ptr = tile_ptr.as<int>();
+    t.tile_end = payload ? nullptr : tile_end.as<int>();
     t.tile_col = tile_col.as<int>();
     // the per-entry arrays only when built (null views otherwise)
     t.tile_nnz = payload ? tile_nnz.as<int>() : nullptr;
@@ -318,6 +319,8 @@ DevTiles tile_row_slice(const DevTiles &A, int I0, int I1)
 {
     DevTiles t = A;
     t.tile_ptr = A.tile_ptr + I0;
+    if (A.tile_end != nullptr)
+        t.tile_end = A.tile_end + I0;
     t.tilem = I1 - I0;
     t.m = std::min(A.m, I1 * TD) - I0 * TD;
     if (A.csr_rowptr != nullptr)

@@ -128,7 +128,8 @@ __device__ __forceinline__ void row_window(const DevTiles &A, const DevTiles &B,
     for (int a = a0 + lane; a < a1; a += 32)
     {
         const int K = __ldg(A.tile_col + a);
-        const int b0 = __ldg(B.tile_ptr + K), b1 = __ldg(B.tile_ptr + K + 1);
+        int b0, b1;
+        tile_range(B, K, b0, b1);
         if (b0 < b1)
         {
             lo = min(lo, __ldg(B.tile_col + b0));
@@ -155,7 +156,8 @@ __device__ __forceinline__ void fill_bitmap(const DevTiles &A, const DevTiles &B
         if (a < a1)
         {
             const int K = __ldg(A.tile_col + a);
-            const int b0 = __ldg(B.tile_ptr + K), b1 = __ldg(B.tile_ptr + K + 1);
+            int b0, b1;
+            tile_range(B, K, b0, b1);
             s = clip ? lower_bound(B.tile_col, b0, b1, w) : b0;
             const int e = clip ? lower_bound(B.tile_col, s, b1, wend) : b1;
             len = e - s;
@@ -229,7 +231,8 @@ __global__ void __launch_bounds__(SYM_WARPS * 32)
     if (I >= A.tilem)
         return;
     WarpSmem1 &S = sm[wi];
-    const int a0 = __ldg(A.tile_ptr + I), a1 = __ldg(A.tile_ptr + I + 1);
+    int a0, a1;
+    tile_range(A, I, a0, a1);
     int lo, hi;
     long long pairs;
     row_window(A, B, a0, a1, lo, hi, pairs);
@@ -277,7 +280,8 @@ __global__ void __launch_bounds__(S1_WIDE_WARPS * 32)
     for (int li = blockIdx.x; li < n; li += gridDim.x)
     {
         const int I = wide[li];
-        const int a0 = __ldg(A.tile_ptr + I), a1 = __ldg(A.tile_ptr + I + 1);
+        int a0, a1;
+        tile_range(A, I, a0, a1);
         if (tid == 0)
         {
             s_lo = INT_MAX;
@@ -360,7 +364,8 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
     const int I = list != nullptr ? list[blockIdx.x] : (int)blockIdx.x;
     if (I >= A.tilem || (list == nullptr && heavy != nullptr && heavy[I]))
         return;
-    const int a0 = __ldg(A.tile_ptr + I), a1 = __ldg(A.tile_ptr + I + 1);
+    int a0, a1;
+    tile_range(A, I, a0, a1);
     const int cbeg = __ldg(c_tile_ptr + I), cend = __ldg(c_tile_ptr + I + 1);
     const int nrows = min(TD, A.m - I * TD);
     const int r0 = warp * 2, r1 = r0 + 1; // warp-private walk (NW == S2_WARPS) and counts
@@ -380,7 +385,8 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
         for (int a = a0 + tid; a < a1; a += NT)
         {
             const int K = __ldg(A.tile_col + a);
-            const int b0 = __ldg(B.tile_ptr + K), b1 = __ldg(B.tile_ptr + K + 1);
+            int b0, b1;
+            tile_range(B, K, b0, b1);
             if (b0 < b1)
             {
                 lo = min(lo, __ldg(B.tile_col + b0));
@@ -427,7 +433,8 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
         for (int a = a0 + warp; a < a1; a += NW)
         {
             const int K = __ldg(A.tile_col + a);
-            int b0 = __ldg(B.tile_ptr + K), b1 = __ldg(B.tile_ptr + K + 1);
+            int b0, b1;
+            tile_range(B, K, b0, b1);
             if (clip)
             {
                 b0 = lower_bound(B.tile_col, b0, b1, w);

@@ -1,0 +1,83 @@
+"""The entry-wise CSR passes of the device path (checks, row segments, tile
+index: csrc/csr2tile.cu) at the ends of their 256-entry blocks, 8-block CTAs
+and warps' chunks: entry counts around them, runs of one tile column and rows
+that cross them, long rows, thousands of empty rows, an unaligned column array,
+and errors in the last entry.  C = A * B against the oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import rtt_spgemm as R
+from conftest import assert_csr_close
+from rtt_spgemm import generators as G
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+DEV = torch.device("cuda:0")
+
+
+def _csr(counts, n, seed, runs=False):
+    """Rows of the given lengths: random columns, or runs of neighbours."""
+    rng = np.random.default_rng(seed)
+    cols = []
+    for k in counts:
+        if runs:
+            cols.append(np.arange(k) + int(rng.integers(0, n - k + 1)))
+        else:
+            cols.append(np.sort(rng.choice(n, k, replace=False)))
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    col = np.concatenate(cols).astype(np.int32) if cols else np.zeros(0, np.int32)
+    return G.CSR(len(counts), n, rp, col, rng.uniform(-1, 1, col.size))
+
+
+def _dev(a, shift=0):
+    col = torch.zeros(a.nnz + shift, dtype=torch.int32, device=DEV)
+    col[shift:] = torch.from_numpy(a.col)
+    return (a.m, a.n, torch.from_numpy(a.rowptr).to(DEV), col[shift:],
+            torch.from_numpy(a.val).to(DEV))
+
+
+def _tiles(a):
+    rows = np.repeat(np.arange(a.m), np.diff(a.rowptr))
+    return np.unique((rows // 16).astype(np.int64) * (a.n // 16 + 1) + a.col // 16).size
+
+
+CASES = {
+    # entry counts around a block, a CTA of blocks and twice it
+    **{f"nnz{k}": (lambda k=k: _csr([7] * (k // 7) + [k % 7], 300, k))
+       for k in (1, 255, 256, 257, 2047, 2048, 2049, 4097)},
+    "runs": lambda: _csr([37] * 200, 400, 3, runs=True),       # runs across every block end
+    "one_row": lambda: _csr([5000], 9000, 4),                   # one row over many warps
+    "long_run": lambda: _csr([0, 900, 0, 1100, 3], 1200, 5, runs=True),
+    "empty": lambda: _csr([3] + [0] * 4000 + [5] * 60 + [0] * 3000, 500, 6),
+    "many": lambda: _csr([24] * 120000, 5000, 7, runs=True),    # several blocks to a warp
+}
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("case", list(CASES))
+def test_scan(case, shift, orc):
+    a = CASES[case]()
+    b = _csr([2] * a.n, 200, 8)
+    ctx = R.Context(0)
+    da, db = _dev(a, shift), _dev(b)
+    nnz, _ = ctx.symbolic(da, db)
+    out = (torch.empty(a.m + 1, dtype=torch.int32, device=DEV),
+           torch.empty(nnz, dtype=torch.int32, device=DEV),
+           torch.empty(nnz, dtype=torch.float64, device=DEV))
+    ctx.numeric(*out)
+    st = ctx.stats()
+    assert st["tiles_a"] == _tiles(a) and st["tiles_b"] == _tiles(b)
+    assert_csr_close(*(x.cpu().numpy() for x in out), *orc.spgemm_csr(a, b), case)
+    # the last entry's column, or the row pointer's end, out of range
+    for bad in ("col", "rowptr"):
+        a2 = G.CSR(a.m, a.n, a.rowptr.copy(), a.col.copy(), a.val)
+        if bad == "col":
+            a2.col[-1] = a.n
+        else:
+            a2.rowptr[-1] += 1
+        with pytest.raises(R.RttError) as e:
+            ctx.symbolic(_dev(a2, shift), db)
+        assert e.value.status == 2
+    ctx.close()
