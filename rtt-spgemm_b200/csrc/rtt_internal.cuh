@@ -339,14 +339,17 @@ struct SymbolicOut
     // symbolic step 2: heavy tile rows (flag per tile row, list) and the
     // list of tile rows for the wide-window CTAs
     DevBuf s2_heavy, s2_list, s2_wlist;
-    // symbolic step 1: tile rows with many tile pairs (list for a wide CTA)
-    DevBuf s1_list;
+    // symbolic step 1: tile rows with many tile pairs (list for a wide CTA);
+    // B's tile rows and the listed rows' C tiles as bitmaps of tile columns,
+    // C tiles per window of a tile row, and the tile rows whose masks step 2 keeps densely
+    DevBuf s1_list, s1_bits, s1_union, s1_wcnt, s2_dlist;
     // some C tile row needs more than one window of the flat numeric kernel
     // (set by the symbolic step; true when unknown)
     bool multi_window = true;
     // C tiles per window of the wide-window step-2 CTAs (0: the default,
     // -1: tile rows with many C tiles stay in the 254-slot CTAs)
     int sym_window_slots = 0;
+    int dense_windows = 0; // windows of a tile row with dense masks (step 1)
     int numtile = 0;
     long long nnz = 0;
     int tilem = 0, tilen = 0, m = 0, n = 0;
@@ -362,7 +365,8 @@ struct SymbolicOut
                                &w_queue,    &w_flag,     &s2_heavy,   &s2_list,
                                &s2_wlist,   &s1_list,    &w_cursor,   &g_slot,
                                &g_rel,      &r_big,      &r_normal,   &r_mask,
-                               &r_cursor,   &r_cut,      &r_part};
+                               &r_cursor,   &r_cut,      &r_part,     &s1_bits,
+                               &s1_wcnt,    &s2_dlist,   &s1_union};
         for (const DevBuf *b : all)
             f(*b);
     }

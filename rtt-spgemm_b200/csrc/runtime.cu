@@ -111,11 +111,12 @@ int Workspace::init(int dev)
     if (dev < 0 || dev >= count)
         return fail(RTT_ERR_INVALID_ARGUMENT, "device index out of range");
     RTT_CUDA(cudaSetDevice(dev));
-    cudaDeviceProp prop;
-    RTT_CUDA(cudaGetDeviceProperties(&prop, dev));
-    if (prop.major < 10)
+    int major = 0, minor = 0;
+    RTT_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    RTT_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
+    if (major < 10)
         return fail(RTT_ERR_NO_DEVICE, "this library is built for sm_100a (B200); found sm_" +
-                                           std::to_string(prop.major * 10 + prop.minor));
+                                           std::to_string(major * 10 + minor));
     {
         // the default pool keeps up to 8 GiB of freed memory for reuse (a
         // regrow then costs no driver allocation); above that it returns

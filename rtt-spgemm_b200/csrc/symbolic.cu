@@ -20,6 +20,7 @@
 // counts and the tile row total come out of the masks with popc.
 #include "rtt_internal.cuh"
 
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 
@@ -186,25 +187,38 @@ __device__ __forceinline__ void fill_bitmap(const DevTiles &A, const DevTiles &B
     }
 }
 
-// Step 1 of a tile row with more pairs than this goes to k_sym_count_wide:
-// one warp would walk them alone while the rest of the grid has finished.
+// B's bitmaps are built up to this size.
+constexpr size_t BIT_BYTES_MAX = size_t(1) << 30;
+
+// Step 1 of a tile row with more pairs than this goes to k_sym_count_wide (or
+// k_sym_count_bits): one warp would walk them alone while the rest of the grid
+// has finished.
 constexpr long long S1_WIDE_PAIRS = 1 << 16;
+constexpr long long S1_BITS_PAIRS = 512;
 constexpr int S1_WIDE_WARPS = 16;
 
+// Rows listed as wide whose C tiles fill at least 1 / DENSE_SPAN of the tile
+// columns they span keep their masks densely in step 2 (k_sym_dense), window
+// by window of DENSE_TILES tile columns.
+constexpr int DENSE_TILES = 1024, DENSE_WORDS = DENSE_TILES / 32, DENSE_SPAN = 8;
+
 // Step-1 outcome of tile row I: C tiles, the step-2 window flag and the
-// step-2 lists: heavy rows (heavy[I] = 1) and rows with more C tiles than
-// one 254-slot window (heavy[I] = 2, for the wide-window CTAs).
+// step-2 lists: rows with dense masks (heavy[I] = 3), heavy rows (1) and rows
+// with more C tiles than one 254-slot window (2, for the wide-window CTAs).
 __device__ __forceinline__ void step1_out(const DevTiles &A, int I, int count, int lo, int hi,
                                           int lane, int *cnt, int *multi, uint8_t *heavy,
                                           int *list, int *list_count, int *wlist,
-                                          int *wlist_count)
+                                          int *wlist_count, int *dlist = nullptr,
+                                          int *dlist_count = nullptr)
 {
     // step 2 will need more than one window for this tile row; with an
     // unbalanced row pair it becomes a heavy row (a wide CTA of its own)
     const bool multi_win = count > S2_SLOTS || (hi >= 0 && (long long)hi - lo + 1 > WBITS);
-    const bool hv = multi_win && heavy != nullptr &&
+    const bool dense = dlist != nullptr && count > S2_SLOTS &&
+                       (long long)DENSE_SPAN * count >= (long long)hi - lo + 1;
+    const bool hv = multi_win && heavy != nullptr && !dense &&
                     skewed_pairs(A, I, min(TD, A.m - I * TD), lane, HEAVY_PAIR);
-    const bool wide = !hv && count > S2_SLOTS && wlist != nullptr;
+    const bool wide = !hv && !dense && count > S2_SLOTS && wlist != nullptr;
     if (lane == 0)
     {
         cnt[I] = count;
@@ -212,8 +226,10 @@ __device__ __forceinline__ void step1_out(const DevTiles &A, int I, int count, i
             atomicOr(multi, 1);
         if (heavy != nullptr)
         {
-            heavy[I] = hv ? 1 : wide ? 2 : 0;
-            if (hv)
+            heavy[I] = dense ? 3 : hv ? 1 : wide ? 2 : 0;
+            if (dense)
+                dlist[atomicAdd(dlist_count, 1)] = I;
+            else if (hv)
                 list[atomicAdd(list_count, 1)] = I;
             else if (wide)
                 wlist[atomicAdd(wlist_count, 1)] = I;
@@ -223,7 +239,8 @@ __device__ __forceinline__ void step1_out(const DevTiles &A, int I, int count, i
 
 __global__ void __launch_bounds__(SYM_WARPS * 32)
     k_sym_count(DevTiles A, DevTiles B, int *cnt, int *multi, uint8_t *heavy, int *list,
-                int *list_count, int *wide, int *wide_count, int *wlist, int *wlist_count)
+                int *list_count, int *wide, int *wide_count, int *wlist, int *wlist_count,
+                int bit_words)
 {
     __shared__ WarpSmem1 sm[SYM_WARPS];
     const int lane = lane_id(), wi = threadIdx.x >> 5;
@@ -236,7 +253,9 @@ __global__ void __launch_bounds__(SYM_WARPS * 32)
     int lo, hi;
     long long pairs;
     row_window(A, B, a0, a1, lo, hi, pairs);
-    if (pairs > S1_WIDE_PAIRS)
+    // with B's bitmaps at hand: where their words are fewer than half the pairs
+    if (pairs > S1_WIDE_PAIRS ||
+        (bit_words > 0 && pairs > S1_BITS_PAIRS && 2 * pairs > (long long)(a1 - a0) * bit_words))
     {
         if (lane == 0)
             wide[atomicAdd(wide_count, 1)] = I;
@@ -329,6 +348,303 @@ __global__ void __launch_bounds__(S1_WIDE_WARPS * 32)
             step1_out(A, I, s_count, lo, hi, lane, cnt, multi, heavy, list, list_count, wlist,
                       wlist_count);
         __syncthreads(); // s_* are reset for the next tile row
+    }
+}
+
+// B's tile rows as bitmaps of tile columns, bit_words (a multiple of
+// DENSE_WORDS) words each, when step 1 listed wide rows: a warp per tile row.
+constexpr int BITS_WARPS = 4;
+__global__ void __launch_bounds__(BITS_WARPS * 32)
+    k_tile_bitmaps(DevTiles B, int bit_words, const int *wide_count, uint32_t *__restrict__ bits)
+{
+    __shared__ uint32_t s_bits[BITS_WARPS][WWORDS];
+    if (*(volatile const int *)wide_count == 0)
+        return;
+    const int lane = lane_id();
+    const int K = blockIdx.x * BITS_WARPS + (threadIdx.x >> 5);
+    if (K >= B.tilem)
+        return;
+    uint32_t *sb = s_bits[threadIdx.x >> 5];
+    uint32_t *out = bits + (size_t)K * bit_words;
+    int b0, b1;
+    tile_range(B, K, b0, b1);
+    for (int w0 = 0; w0 < bit_words; w0 += WWORDS)
+    {
+        const int nw = min(WWORDS, bit_words - w0);
+        for (int i = lane; i < nw; i += 32)
+            sb[i] = 0u;
+        __syncwarp();
+        // the list's part in these words (tile columns increase)
+        const int lo = lower_bound(B.tile_col, b0, b1, w0 * 32);
+        for (int b = lo + lane; b < b1; b += 32)
+        {
+            const int d = __ldg(B.tile_col + b) - w0 * 32;
+            if (d >= nw * 32)
+                break;
+            atomicOr(&sb[d >> 5], 1u << (d & 31));
+        }
+        __syncwarp();
+        for (int i = lane; i < nw; i += 32)
+            out[w0 + i] = sb[i];
+        __syncwarp();
+    }
+}
+
+// Step 1 of the listed tile rows from B's bitmaps: the union is an OR of the
+// bitmaps of its A tiles, in registers (a lane owns a word of each of 4
+// windows), so a pair costs a bit and not a list entry's search and shared
+// atomic.  R-MAT 2^16 A*A^T: step 1 took 3.3 ms from the lists (of up to
+// thousands of tiles per B tile row), 0.12 ms like this.  uni: the union, for
+// step 2; wcnt: C tiles per (tile row, window of DENSE_TILES).
+constexpr int SB_WARPS = 8, SB_Q = 4;
+__global__ void __launch_bounds__(SB_WARPS * 32)
+    k_sym_count_bits(DevTiles A, int bit_words, const uint32_t *__restrict__ bits, int *cnt,
+                     int *wcnt, uint32_t *__restrict__ uni, int *multi, uint8_t *heavy, int *list,
+                     int *list_count,
+                     const int *wide, const int *wide_count, int *wlist, int *wlist_count,
+                     int *dlist, int *dlist_count)
+{
+    __shared__ uint32_t s_or[SB_Q * 32];
+    __shared__ int s_count, s_lo, s_hi;
+    const int tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const int n = *wide_count, nwin = bit_words / DENSE_WORDS;
+    for (int li = blockIdx.x; li < n; li += gridDim.x)
+    {
+        const int I = wide[li];
+        int a0, a1;
+        tile_range(A, I, a0, a1);
+        if (tid == 0)
+        {
+            s_count = 0;
+            s_lo = INT_MAX;
+            s_hi = -1;
+        }
+        for (int w0 = 0; w0 < bit_words; w0 += SB_Q * 32)
+        {
+            if (tid < SB_Q * 32)
+                s_or[tid] = 0u;
+            __syncthreads();
+            uint32_t acc[SB_Q] = {};
+#pragma unroll 2
+            for (int a = a0 + warp; a < a1; a += SB_WARPS)
+            {
+                const uint32_t *row = bits + (size_t)__ldg(A.tile_col + a) * bit_words + w0;
+#pragma unroll
+                for (int q = 0; q < SB_Q; ++q)
+                    if (w0 + q * 32 < bit_words)
+                        acc[q] |= __ldg(row + q * 32 + lane);
+            }
+#pragma unroll
+            for (int q = 0; q < SB_Q; ++q)
+                if (acc[q] != 0u)
+                    atomicOr(&s_or[q * 32 + lane], acc[q]);
+            __syncthreads();
+            if (warp < SB_Q && w0 + warp * 32 < bit_words)
+            {
+                const uint32_t v = s_or[warp * 32 + lane];
+                uni[(size_t)I * bit_words + w0 + warp * 32 + lane] = v;
+                const int c = warp_sum(__popc(v));
+                const unsigned any = __ballot_sync(FULL, v != 0u);
+                if (any != 0u)
+                {
+                    const int f = __ffs(any) - 1, l = 31 - __clz(any);
+                    const int first = f * 32 + __ffs(__shfl_sync(FULL, v, f)) - 1;
+                    const int last = l * 32 + 31 - __clz(__shfl_sync(FULL, v, l));
+                    if (lane == 0)
+                    {
+                        atomicAdd(&s_count, c);
+                        atomicMin(&s_lo, (w0 + warp * 32) * 32 + first);
+                        atomicMax(&s_hi, (w0 + warp * 32) * 32 + last);
+                    }
+                }
+                if (lane == 0)
+                    wcnt[(size_t)I * nwin + w0 / 32 + warp] = c;
+            }
+            __syncthreads();
+        }
+        if (warp == 0)
+            step1_out(A, I, s_count, s_lo, s_hi, lane, cnt, multi, heavy, list, list_count, wlist,
+                      wlist_count, dlist, dlist_count);
+        __syncthreads(); // s_* are reset for the next tile row
+    }
+}
+
+// Step 2 of the tile rows with dense masks, one (tile row, window) at a time:
+// the window's 16 x DENSE_TILES row masks directly addressed in shared memory,
+// so an A entry's segments are OR-ed without a slot table or a second walk of
+// the row for its next window (the wide-window CTAs took 5.6 ms for R-MAT 2^16
+// A*A^T at 16 warps per SM; this takes 2.0 ms at 64).  32 entries' segments are
+// spread over the lanes one by one, whatever their rows' lengths.  Bound by the
+// search of a lane's entry and the shared atomics.
+constexpr int SD_WARPS = 16, SD_THREADS = SD_WARPS * 32;
+struct DenseSmem
+{
+    uint32_t mw[S2_PAIRS][DENSE_TILES]; // row 2p in the low half, 2p + 1 in the high
+    int start[SD_WARPS][32], pre[SD_WARPS][32]; // 32 entries: first segment, segments before
+    int row[SD_WARPS][32];
+    int rp[TD + 1], rowcnt[TD], base;
+};
+__global__ void __launch_bounds__(SD_THREADS, 4)
+    k_sym_dense(DevTiles A, DevTiles B, int nwin, const int *__restrict__ dlist, int ndense,
+                const int *__restrict__ wcnt, const uint32_t *__restrict__ uni,
+                const int *__restrict__ c_tile_ptr, int *__restrict__ c_tile_col, int *__restrict__ c_tile_row,
+                uint16_t *__restrict__ c_mask, int *__restrict__ c_tile_cnt,
+                int *__restrict__ c_row_cnt, int *__restrict__ c_tr_nnz, int *multi)
+{
+    extern __shared__ __align__(16) unsigned char sd_raw[];
+    DenseSmem &S = *reinterpret_cast<DenseSmem *>(sd_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long items = (long long)ndense * nwin;
+    for (long long it = blockIdx.x; it < items; it += gridDim.x)
+    {
+        // the tile rows' first windows first: they hold the most of a
+        // power-law matrix's columns
+        const int I = __ldg(dlist + it % ndense), wi = (int)(it / ndense);
+        const int *wc = wcnt + (size_t)I * nwin;
+        const int here = __ldg(wc + wi);
+        if (here == 0)
+            continue; // uniform
+        const int nrows = min(TD, A.m - I * TD);
+        __syncthreads(); // the previous item is done with shared memory
+        for (int i = tid; i < S2_PAIRS * DENSE_TILES / 4; i += SD_THREADS)
+            reinterpret_cast<uint4 *>(S.mw)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (tid <= nrows)
+            S.rp[tid] = __ldg(A.csr_rowptr + I * TD + tid);
+        if (tid < TD)
+            S.rowcnt[tid] = 0;
+        if (warp == 0)
+        {
+            // C tiles of the windows before
+            int before = 0;
+            for (int w = lane; w < wi; w += 32)
+                before += __ldg(wc + w);
+            before = warp_sum(before);
+            if (lane == 0)
+                S.base = __ldg(c_tile_ptr + I) + before;
+        }
+        __syncthreads();
+        const int w0 = wi * DENSE_TILES;
+        const int eb = S.rp[0], ee = S.rp[nrows];
+        for (int c0 = eb + warp * 32; c0 < ee; c0 += SD_THREADS)
+        {
+            const int e = c0 + lane;
+            int s0 = 0, ns = 0, r = 0;
+            if (e < ee)
+            {
+#pragma unroll
+                for (int h = 8; h > 0; h >>= 1)
+                    if (r + h < nrows && S.rp[r + h] <= e)
+                        r += h;
+                const int k = __ldg(A.csr_col + e);
+                if ((unsigned)k < (unsigned)B.m)
+                {
+                    s0 = __ldg(B.seg_ptr + k);
+                    int s1 = __ldg(B.seg_ptr + k + 1);
+                    if (nwin > 1 && s1 - s0 > 8) // shorter lists are filtered below
+                    {
+                        s0 = wi > 0 ? seg_lower_bound(B.seg, s0, s1, w0) : s0;
+                        s1 = wi + 1 < nwin ? seg_lower_bound(B.seg, s0, s1, w0 + DENSE_TILES) : s1;
+                    }
+                    ns = s1 - s0;
+                }
+            }
+            const int incl = warp_incl_scan(ns);
+            const int total = __shfl_sync(FULL, incl, 31);
+            S.start[warp][lane] = s0 - (incl - ns);
+            S.pre[warp][lane] = incl - ns;
+            S.row[warp][lane] = r;
+            __syncwarp();
+            constexpr int U = 2;
+            for (int p0 = lane; p0 < total; p0 += 32 * U)
+            {
+                unsigned long long sg[U];
+                int o[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    // the entry of segment p: the last one with pre <= p
+                    const int p = p0 + 32 * u;
+                    int lo = 0;
+#pragma unroll
+                    for (int h = 16; h > 0; h >>= 1)
+                        if (S.pre[warp][lo + h] <= p)
+                            lo += h;
+                    o[u] = S.row[warp][lo];
+                    sg[u] = p < total ? __ldg(B.seg + S.start[warp][lo] + p) : 0ull;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    const int d = (int)(sg[u] >> 16) - w0;
+                    if ((unsigned)d < (unsigned)DENSE_TILES)
+                        atomicOr(&S.mw[o[u] >> 1][d],
+                                 ((unsigned)sg[u] & 0xFFFFu) << ((o[u] & 1) * 16));
+                }
+            }
+            __syncwarp(); // before the next batch overwrites the lists
+        }
+        __syncthreads();
+        // the window's tiles in order (the union of step 1: a tile may hold
+        // no entry): a warp takes DENSE_TILES / SD_WARPS of them, 32 at a time
+        constexpr int PER = DENSE_TILES / SD_WARPS / 32;
+        const uint32_t word = __ldg(uni + ((size_t)I * nwin + wi) * DENSE_WORDS + lane);
+        const int upto = warp_incl_scan(__popc(word));
+        int at = S.base + __shfl_sync(FULL, upto - __popc(word), warp * PER);
+        unsigned bal[PER];
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            bal[q] = __shfl_sync(FULL, word, warp * PER + q);
+        int rows[S2_PAIRS] = {}; // entries of rows 2p (low half) and 2p + 1
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+        {
+            if ((bal[q] >> lane) & 1u)
+            {
+                const int t = (warp * PER + q) * 32 + lane;
+                const int c = at + __popc(bal[q] & ((1u << lane) - 1u));
+                uint32_t v[S2_PAIRS];
+                int n = 0;
+#pragma unroll
+                for (int p = 0; p < S2_PAIRS; ++p)
+                {
+                    v[p] = S.mw[p][t];
+                    const int lo = __popc(v[p] & 0xFFFFu), hi = __popc(v[p] >> 16);
+                    rows[p] += lo | (hi << 16);
+                    n += lo + hi;
+                }
+                c_tile_col[c] = w0 + t;
+                c_tile_row[c] = I;
+                c_tile_cnt[c] = n;
+                uint4 *m = reinterpret_cast<uint4 *>(c_mask + (size_t)c * TD);
+                m[0] = make_uint4(v[0], v[1], v[2], v[3]);
+                m[1] = make_uint4(v[4], v[5], v[6], v[7]);
+            }
+            at += __popc(bal[q]);
+        }
+#pragma unroll
+        for (int p = 0; p < S2_PAIRS; ++p)
+        {
+            const int v = warp_sum(rows[p]);
+            if (lane == 0 && v != 0)
+            {
+                atomicAdd(&S.rowcnt[2 * p], v & 0xFFFF);
+                atomicAdd(&S.rowcnt[2 * p + 1], v >> 16);
+            }
+        }
+        __syncthreads();
+        if (warp == 0)
+        {
+            const int v = lane < nrows ? S.rowcnt[lane] : 0;
+            if (v != 0)
+                atomicAdd(c_row_cnt + I * TD + lane, v);
+            const int tot = warp_sum(v);
+            if (lane == 0)
+            {
+                atomicAdd(c_tr_nnz + I, tot);
+                if (*(volatile int *)multi == 0)
+                    atomicOr(multi, 1); // more C tiles than a numeric window holds
+            }
+        }
     }
 }
 
@@ -875,7 +1191,7 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
     // flags: [0] some tile row needs several step-2 windows, [1] several
     // numeric windows, [2] heavy tile rows listed for the wide step-2 CTA,
     // [3] tile rows listed for the wide step-1 CTA, [4] tile rows listed for
-    // the wide-window step-2 CTAs
+    // the wide-window step-2 CTAs, [5] tile rows with dense masks
     RTT_CHECK(S.w_flag.ensure(sizeof(int) * 8, s));
     RTT_CUDA(cudaMemsetAsync(S.w_flag.p, 0, sizeof(int) * 8, s));
     RTT_CHECK(S.s2_heavy.ensure((size_t)tilem + 16, s));
@@ -888,16 +1204,47 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
     {
         int *flag = S.w_flag.as<int>();
         int *wlist = wide ? S.s2_wlist.as<int>() : nullptr;
-        k_sym_count<<<ceil_div(tilem, SYM_WARPS), SYM_WARPS * 32, 0, s>>>(
-            A, B, cnt, flag, S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2,
-            S.s1_list.as<int>(), flag + 3, wlist, flag + 4);
         int sms = 0;
         RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
-        // persistent CTAs over the wide list (empty: they exit at once)
-        k_sym_count_wide<<<std::min(tilem, 2 * sms), S1_WIDE_WARPS * 32, 0, s>>>(
+        // B's tile rows as bitmaps, where they are not much larger than B's
+        // tile lists (R-MAT 2^16: 2 MB, 2^20: 512 MB; the 96^3 stencil's 380 MB
+        // against 1.3 million tiles are not built)
+        const int bit_words = ceil_div(std::max(B.tilen, 1), DENSE_TILES) * DENSE_WORDS;
+        const size_t bit_bytes = sizeof(uint32_t) * (size_t)bit_words * (size_t)B.tilem;
+        const size_t uni_bytes = sizeof(uint32_t) * (size_t)bit_words * (size_t)tilem;
+        const bool bits = wide && B.seg_ptr != nullptr && A.csr_rowptr != nullptr &&
+                          A.csr_col != nullptr && std::max(bit_bytes, uni_bytes) <= BIT_BYTES_MAX &&
+                          bit_bytes <= 64 * (size_t)B.numtile;
+        S.dense_windows = 0;
+        if (bits)
+        {
+            S.dense_windows = bit_words / DENSE_WORDS;
+            RTT_CHECK(S.s1_bits.ensure(bit_bytes, s));
+            RTT_CHECK(S.s1_union.ensure(uni_bytes, s));
+            RTT_CHECK(S.s1_wcnt.ensure(sizeof(int) * (size_t)tilem * S.dense_windows, s));
+            RTT_CHECK(S.s2_dlist.ensure(sizeof(int) * (size_t)tilem + 16, s));
+        }
+        k_sym_count<<<ceil_div(tilem, SYM_WARPS), SYM_WARPS * 32, 0, s>>>(
             A, B, cnt, flag, S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2,
-            S.s1_list.as<int>(), flag + 3, wlist, flag + 4);
-        ws.launches += 2;
+            S.s1_list.as<int>(), flag + 3, wlist, flag + 4, bits ? bit_words : 0);
+        ws.launches++;
+        if (bits)
+        {
+            k_tile_bitmaps<<<ceil_div(B.tilem, BITS_WARPS), BITS_WARPS * 32, 0, s>>>(
+                B, bit_words, flag + 3, S.s1_bits.as<uint32_t>());
+            k_sym_count_bits<<<std::min(tilem, 8 * sms), SB_WARPS * 32, 0, s>>>(
+                A, bit_words, S.s1_bits.as<uint32_t>(), cnt, S.s1_wcnt.as<int>(),
+                S.s1_union.as<uint32_t>(), flag,
+                S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2, S.s1_list.as<int>(),
+                flag + 3, wlist, flag + 4, S.s2_dlist.as<int>(), flag + 5);
+            ws.launches++;
+        }
+        else
+            // persistent CTAs over the wide list (empty: they exit at once)
+            k_sym_count_wide<<<std::min(tilem, 2 * sms), S1_WIDE_WARPS * 32, 0, s>>>(
+                A, B, cnt, flag, S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2,
+                S.s1_list.as<int>(), flag + 3, wlist, flag + 4);
+        ws.launches++;
     }
     return RTT_OK;
 }
@@ -918,13 +1265,14 @@ int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Symboli
     int *cnt = S.count_tmp.as<int>();
     RTT_CHECK(symbolic_tile_counts(ws, A, B, S, cnt));
     RTT_CHECK(scan_exclusive_int(ws, cnt, S.c_tile_ptr.as<int>(), tilem));
-    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 16, S.w_flag.p, sizeof(int) * 5,
+    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 16, S.w_flag.p, sizeof(int) * 6,
                              cudaMemcpyDeviceToHost, s));
     int numtile = 0;
     RTT_CHECK(read_int_checked(ws, S.c_tile_ptr.as<int>() + tilem, &numtile, "symbolic step 1"));
     const bool sym_multi = ws.h_scalars[16] != 0;
     const int n_heavy = ws.h_scalars[18];
     const int n_wide = S.sym_window_slots >= 0 ? ws.h_scalars[20] : 0;
+    const int n_dense = ws.h_scalars[21];
     const int wslots = S.sym_window_slots > 0 ? S.sym_window_slots : S2_WIDE_DEFAULT;
     const int wstride = (wslots + 2) | 1;
     S.numtile = numtile;
@@ -956,6 +1304,25 @@ int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Symboli
             ws.launches++;
             return RTT_OK;
         };
+        if (n_dense > 0)
+        {
+            // rows with dense masks: their windows add up the counts
+            RTT_CUDA(cudaMemsetAsync(S.c_row_cnt.p, 0, sizeof(int) * (size_t)(S.m + 1), s));
+            RTT_CUDA(cudaMemsetAsync(S.c_tr_nnz.p, 0, sizeof(int) * (size_t)(tilem + 1), s));
+            int sms = 0;
+            RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+            RTT_CUDA(cudaFuncSetAttribute(k_sym_dense, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(DenseSmem)));
+            const long long items = (long long)n_dense * S.dense_windows;
+            k_sym_dense<<<(int)std::min<long long>(items, 4 * sms), SD_THREADS, sizeof(DenseSmem),
+                          s>>>(
+                A, B, S.dense_windows, S.s2_dlist.as<int>(), n_dense, S.s1_wcnt.as<int>(),
+                S.s1_union.as<uint32_t>(),
+                S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(), S.c_tile_row.as<int>(),
+                S.c_mask.as<uint16_t>(), S.tile_cnt.as<int>(), S.c_row_cnt.as<int>(),
+                S.c_tr_nnz.as<int>(), S.w_flag.as<int>() + 1);
+            ws.launches++;
+        }
         if (n_heavy > 0 || n_wide > 0)
         {
             // heavy rows (one 32-warp CTA each) and rows with many C tiles
@@ -994,7 +1361,7 @@ int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Symboli
         // 4-warp CTAs when every tile row fits one window; a tile row with
         // several windows walks its entries once per window, so it keeps 8
         const bool small = segs && !sym_multi;
-        const uint8_t *skip = n_heavy > 0 || n_wide > 0 ? S.s2_heavy.as<uint8_t>() : nullptr;
+        const uint8_t *skip = n_heavy > 0 || n_wide > 0 || n_dense > 0 ? S.s2_heavy.as<uint8_t>() : nullptr;
         if (small)
             RTT_CHECK(go(k_sym_rows<false, S2_SEG_WARPS, true>, tilem, S2_SEG_WARPS * 32,
                          smem2_bytes<S2_SEG_WARPS, false>(S2_STRIDE), s, skip, nullptr, 0));
