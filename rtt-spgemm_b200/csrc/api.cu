@@ -742,7 +742,7 @@ int run_phase(rtt_context c, int slot, const std::vector<long long> &head, bool 
 }
 
 // Device work of the numeric step into C's CSR (c_row_ptr, c_col_idx,
-// c_values), counters copied to ws.h_scalars64[2..5]; no host reads unless
+// c_values), counters and error word published; no host reads unless
 // fused_csr_output == 0 (tile2csr sizes its output on the host).
 int numeric_enqueue(rtt_context c, int *c_row_ptr, int *c_col_idx, double *c_values, int cutoff)
 {
@@ -799,16 +799,17 @@ int numeric_enqueue(rtt_context c, int *c_row_ptr, int *c_col_idx, double *c_val
                                        S.tilem, TD, nullptr, -1, c_row_ptr, c_col_idx, c_values,
                                        false));
     }
-    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars64 + 2, c->counters.p, sizeof(long long) * 4,
-                             cudaMemcpyDeviceToHost, ws.stream));
-    return RTT_OK;
+    Publish pub;
+    pub.add(c->counters.p, reinterpret_cast<int *>(ws.h_scalars64 + 2), 8);
+    publish_error(ws, pub);
+    return publish(ws, pub);
 }
 
 // After numeric_enqueue (eager or graph): device checks, then the statistics.
 int numeric_finish(rtt_context c)
 {
     Workspace &ws = c->ws;
-    RTT_CHECK(check_device_error(ws, "numeric"));
+    RTT_CHECK(wait_published(ws, "numeric"));
     if (c->cfg.stage_timing && c->S.numtile > 0)
     {
         float tn = 0.f;
@@ -841,18 +842,23 @@ int numeric_args_ok(rtt_context c, const int *c_row_ptr, const int *c_col_idx,
 // CSR rows, and the device views the symbolic and numeric steps take.  The
 // shape checks of the entry points come first.  Shared by the 32-bit product
 // and the 64-bit (chunked) one.
+// defer: the tile indexes are enqueued without a host read (csr2tile_settle).
 int prepare_operands(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B, int op,
-                     DevTiles &dA, DevTiles &dB)
+                     DevTiles &dA, DevTiles &dB, bool defer = false)
 {
     Workspace &ws = c->ws;
     // The flat numeric step reads A and B from their CSR rows, so only the
     // tile index and B's row segments are built; the per-entry tile arrays
     // are built for the kernels that read them (DMMA pairs, TMA staging).
     const bool payload = c->cfg.dmma_pair_cutoff > 0 || c->cfg.b_staging != 0;
+    // (shapes that are refused below: A's own errors are reported first)
+    defer = defer && (op == RTT_OP_AAT || (B == nullptr ? A->rows == A->cols
+                                                        : B->rows == A->cols && B->nnz >= 0 &&
+                                                              B->nnz <= INT_MAX));
     // B's row segments drive symbolic step 2: A's own when B is A
     RTT_CHECK(map_device_error(csr2tile_device(ws, A->rows, A->cols, (int)A->nnz, A->row_ptr,
                                                A->col_idx, A->values, c->A, true, false,
-                                               op == RTT_OP_AB && B == nullptr, payload)));
+                                               op == RTT_OP_AB && B == nullptr, payload, defer)));
     c->a_rp = A->row_ptr;
     c->a_ci = A->col_idx;
     c->a_va = A->values;
@@ -882,7 +888,7 @@ int prepare_operands(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B
             RTT_CHECK(map_device_error(csr2tile_device(ws, A->cols, A->rows, (int)A->nnz,
                                                        c->bt_rowptr.as<int>(), c->bt_col.as<int>(),
                                                        c->bt_val.as<double>(), c->B, true, false,
-                                                       true, payload)));
+                                                       true, payload, defer)));
             c->b_rp = c->bt_rowptr.as<int>();
             c->b_ci = c->bt_col.as<int>();
             c->b_va = c->bt_val.as<double>();
@@ -896,7 +902,7 @@ int prepare_operands(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B
                 return rtt::fail(RTT_ERR_INVALID_ARGUMENT, "bad B shape");
             RTT_CHECK(map_device_error(csr2tile_device(ws, B->rows, B->cols, (int)B->nnz,
                                                        B->row_ptr, B->col_idx, B->values, c->B,
-                                                       true, false, true, payload)));
+                                                       true, false, true, payload, defer)));
             c->b_rp = B->row_ptr;
             c->b_ci = B->col_idx;
             c->b_va = B->values;
@@ -914,6 +920,42 @@ int prepare_operands(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B
     // A's CSR rows: step 2 walks the tile row's entries straight from them
     dA.csr_rowptr = A->row_ptr;
     dA.csr_col = A->col_idx;
+    return RTT_OK;
+}
+
+// The operands' tile indexes and step 1 up to one synchronisation, which brings
+// the operands' flags and sizes beside C's tiles; operands whose rows need the
+// tile payload (unsorted ones) are then built again, host read by host read.
+int operands_and_step1(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B, int op,
+                       DevTiles &dA, DevTiles &dB)
+{
+    Workspace &ws = c->ws;
+    RTT_CHECK(prepare_operands(c, A, B, op, dA, dB, true));
+    const TileBufs &TB = c->b_alias ? c->A : c->B;
+    if (c->cfg.stage_timing != 0)
+        RTT_CUDA(cudaEventRecord(ws.ev[1], ws.stream));
+    const bool wait_a = !c->A.payload, wait_b = !c->b_alias && !c->B.payload;
+    Publish words;
+    if (wait_a)
+        words.add(csr2tile_words(c->A), ws.h_scalars + 24, CSR_WORDS);
+    if (wait_b)
+        words.add(csr2tile_words(c->B), ws.h_scalars + 32, CSR_WORDS);
+    RTT_CHECK(map_device_error(symbolic_step1(ws, dA, dB, c->S, words)));
+    bool settled = true;
+    if (wait_a)
+        settled &= csr2tile_settle(c->A, ws.h_scalars + 24);
+    if (wait_b)
+        settled &= csr2tile_settle(c->B, ws.h_scalars + 32);
+    if (!settled)
+    {
+        RTT_CHECK(prepare_operands(c, A, B, op, dA, dB));
+        return map_device_error(symbolic_step1(ws, dA, dB, c->S));
+    }
+    dA.numtile = c->A.numtile;
+    dB.numtile = TB.numtile;
+    dA.max_row_segs = c->A.max_row_segs;
+    dB.max_row_segs = TB.max_row_segs;
+    c->b_dups = TB.dup_cols;
     return RTT_OK;
 }
 
@@ -1649,11 +1691,17 @@ int rtt_spgemm_symbolic(rtt_context c, const rtt_csr_view *A, const rtt_csr_view
     if (timing)
         RTT_CUDA(cudaEventRecord(ws.ev[0], ws.stream));
     DevTiles dA, dB;
-    RTT_CHECK(prepare_operands(c, A, B, op, dA, dB));
+    {
+        const int st = operands_and_step1(c, A, B, op, dA, dB);
+        if (st != RTT_OK)
+        {
+            // work enqueued before the failure may have left an error word
+            cudaMemsetAsync(ws.err.p, 0, sizeof(int), ws.stream);
+            return st;
+        }
+    }
     const TileBufs &TB = c->b_alias ? c->A : c->B;
-    if (timing)
-        RTT_CUDA(cudaEventRecord(ws.ev[1], ws.stream));
-    RTT_CHECK(map_device_error(symbolic_device(ws, dA, dB, c->S, !c->b_dups)));
+    RTT_CHECK(map_device_error(symbolic_step2(ws, dA, dB, c->S, !c->b_dups)));
     if (timing)
     {
         float t01 = 0.f, t12 = 0.f;

@@ -1069,15 +1069,32 @@ __global__ void k_copy_tiles_colmajor(int n, const int *__restrict__ order,
 }
 
 // ----------------------------------------------------------- CSR transpose
-// A warp per row (a thread per row left an R-MAT hub row to one thread: 64 us
-// at 2^16, now 12).
-__global__ void k_row_ids(int m, const int *__restrict__ rowptr, int *__restrict__ rows)
+// A warp per 32 rows: a lane its own row up to 16 entries, the longer rows by
+// the whole warp (a thread per row left an R-MAT hub row to one thread: 64 us
+// at 2^16, now 7).  Nothing is written after an error (a row pointer not yet
+// checked on the host).
+__global__ void k_row_ids(int m, const int *__restrict__ rowptr, int *__restrict__ rows,
+                          const int *err)
 {
-    const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    if (r >= m)
+    if (*(volatile const int *)err != 0)
         return;
-    for (int j = rowptr[r] + lane_id(), e = rowptr[r + 1]; j < e; j += 32)
-        rows[j] = (int)r;
+    const int lane = lane_id();
+    const long long r0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * 32;
+    if (r0 >= m)
+        return;
+    const int r = (int)min(r0 + lane, (long long)m - 1);
+    const int b = rowptr[r], e = r0 + lane < m ? rowptr[r + 1] : b;
+    const bool lng = e - b > 16;
+    if (!lng)
+        for (int j = b; j < e; ++j)
+            rows[j] = r;
+    for (unsigned ls = __ballot_sync(FULL, lng); ls != 0u; ls &= ls - 1u)
+    {
+        const int q = __ffs(ls) - 1;
+        const int qb = __shfl_sync(FULL, b, q), qe = __shfl_sync(FULL, e, q);
+        for (int j = qb + lane; j < qe; j += 32)
+            rows[j] = (int)r0 + q;
+    }
 }
 
 __global__ void k_gather_transpose(int nnz, const int *__restrict__ order,
@@ -1144,7 +1161,7 @@ struct CsChunks
 
 int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, const int *col,
                     const double *val, TileBufs &out, bool packed_col, bool sort_within_rows,
-                    bool segments, bool payload)
+                    bool segments, bool payload, bool defer)
 {
     if (m < 0 || n < 0 || nnz < 0)
         return fail(RTT_ERR_INVALID_ARGUMENT, "csr2tile: negative size");
@@ -1224,23 +1241,27 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
             ws.err.as<int>());
         ws.launches++;
     }
-    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 2, flags, sizeof(int) * 6, cudaMemcpyDeviceToHost, s));
-    RTT_CHECK(check_device_error(ws, "csr2tile validate"));
+    if (defer && !payload)
+    {
+        // until csr2tile_settle
+        const int none[CSR_WORDS] = {};
+        csr2tile_settle(out, none);
+        return RTT_OK;
+    }
+    Publish pub;
+    pub.add(flags, ws.h_scalars + 2, CSR_WORDS);
+    publish_error(ws, pub);
+    RTT_CHECK(publish(ws, pub));
+    RTT_CHECK(wait_published(ws, "csr2tile validate"));
+    if (!payload && csr2tile_settle(out, ws.h_scalars + 2))
+        return RTT_OK;
     const bool generic = ws.h_scalars[2] != 0;
     const bool unsorted = ws.h_scalars[3] != 0;
     // rows that are unsorted may hide repeated columns too
     out.dup_cols = ws.h_scalars[4] != 0 || unsorted;
     out.generic = generic;
-    // the structure alone comes from the row segments, which need rows whose
-    // tile columns never decrease; otherwise the whole tile payload is built
+    out.payload = true;
     out.has_segments = want_segs && !generic;
-    if (!payload && !generic)
-    {
-        out.numtile = ws.h_scalars[6];
-        out.max_row_segs = ws.h_scalars[7];
-        out.payload = false;
-        return RTT_OK;
-    }
     out.max_row_segs = 0;
 
     int *cnt = out.tmp0.as<int>();
@@ -1325,6 +1346,22 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     return RTT_OK;
 }
 
+const int *csr2tile_words(const TileBufs &t) { return t.tmp1.as<int>(); }
+
+bool csr2tile_settle(TileBufs &t, const int *words)
+{
+    t.generic = words[0] != 0;
+    // rows that are unsorted may hide repeated columns too
+    t.dup_cols = words[2] != 0 || words[1] != 0;
+    // the structure alone comes from the row segments, which need rows whose
+    // tile columns never decrease; otherwise the whole tile payload is built
+    t.has_segments = !t.generic;
+    t.payload = t.generic;
+    t.numtile = words[4];
+    t.max_row_segs = words[5];
+    return !t.generic;
+}
+
 int csr2tile_refill_device(Workspace &ws, const int *rowptr, const int *col, const double *val,
                            TileBufs &t, bool packed_col)
 {
@@ -1382,9 +1419,11 @@ int validate_csr_device(Workspace &ws, int m, int n, int nnz, const int *rowptr,
             m, n, nnz, rowptr, col, ch.ctas, ch.blocks, nullptr, nullptr, ws.err.as<int>(), flags);
         ws.launches++;
     }
-    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 4, flags, sizeof(int) * 3, cudaMemcpyDeviceToHost,
-                             ws.stream));
-    return check_device_error(ws, "csr validate");
+    Publish pub;
+    pub.add(flags, ws.h_scalars + 4, 3);
+    publish_error(ws, pub);
+    RTT_CHECK(publish(ws, pub));
+    return wait_published(ws, "csr validate");
 }
 
 int build_tile_csc(Workspace &ws, TileBufs &t)
@@ -1464,7 +1503,7 @@ int csr_transpose_device(Workspace &ws, int m, int n, int nnz, const int *rowptr
     int *keys = ws.tmp[2].as<int>(), *order = ws.tmp[3].as<int>();
     if (m > 0)
     {
-        k_row_ids<<<grid_for((long long)m * 32, 256), 256, 0, s>>>(m, rowptr, rows);
+        k_row_ids<<<grid_for(m, 256), 256, 0, s>>>(m, rowptr, rows, ws.err.as<int>());
         ws.launches++;
     }
     if (nnz > 0)

@@ -216,7 +216,7 @@ struct Workspace
     DevBuf err;        // int device error word
     DevBuf scan_tmp;   // CUB temp storage
     DevBuf tmp[4];     // grow-only scratch of the transpose and the batch tables
-    int *h_scalars = nullptr; // pinned, 32 ints
+    int *h_scalars = nullptr; // pinned, 64 ints
     long long *h_scalars64 = nullptr; // pinned, 8 long long
     int launches = 0;
     int syncs = 0;
@@ -229,17 +229,41 @@ struct Workspace
     void destroy();
 };
 
-// exclusive scan of n ints in place into out (n + 1 entries: out[n] = total)
-int scan_exclusive_int(Workspace &ws, const int *in, int *out, int n);
+// Device words that a kernel writes into the workspace's page-locked host words
+// (which the device reaches directly) ahead of a synchronisation: one launch,
+// or the tail of a scan, in place of a copy per value.
+struct Publish
+{
+    static constexpr int MAX = 6;
+    const int *src[MAX];
+    int *dst[MAX];
+    int words[MAX];
+    int count = 0;
+    void add(const void *from, int *to, int n)
+    {
+        src[count] = static_cast<const int *>(from);
+        dst[count] = to;
+        words[count++] = n;
+    }
+};
+// enqueue the publication
+int publish(Workspace &ws, const Publish &p);
+// exclusive scan of n ints in place into out (n + 1 entries: out[n] = total),
+// then the publication, if any
+int scan_exclusive_int(Workspace &ws, const int *in, int *out, int n, const Publish *pub = nullptr);
 // exclusive scan of n ints into int64 offsets (n + 1 entries)
-int scan_exclusive_i64(Workspace &ws, const int *in, long long *out, int n);
+int scan_exclusive_i64(Workspace &ws, const int *in, long long *out, int n,
+                       const Publish *pub = nullptr);
+// adds the device error word to p; wait_published then syncs and returns
+// RTT_ERR_DEVICE_CHECK on error
+void publish_error(Workspace &ws, Publish &p);
+int wait_published(Workspace &ws, const char *stage);
 // read the device error word (syncs the stream); returns RTT_ERR_DEVICE_CHECK on error
 int check_device_error(Workspace &ws, const char *stage);
 // copy one int / int64 from device to host (syncs)
 int read_int(Workspace &ws, const int *d, int *h);
 int read_i64(Workspace &ws, const long long *d, long long *h);
-// the same reads with the device error word checked in the same synchronisation
-int read_int_checked(Workspace &ws, const int *d, int *h, const char *stage);
+// the same read with the device error word checked in the same synchronisation
 int read_i64_checked(Workspace &ws, const long long *d, long long *h, const char *stage);
 // while on, DevBuf growth on this thread fails with RTT_ERR_STATE (graph capture)
 void freeze_growth(bool on);
@@ -280,7 +304,14 @@ struct TileBufs
 // row segments, when the rows allow it (out.payload tells what was built)
 int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, const int *col,
                     const double *val, TileBufs &out, bool packed_col, bool sort_within_rows,
-                    bool segments = false, bool payload = true);
+                    bool segments = false, bool payload = true, bool defer = false);
+// A deferred structure-only build (defer, payload = false) is enqueued without a
+// host read: its flags and sizes are CSR_WORDS words at csr2tile_words(t), to
+// be published and given to csr2tile_settle after a synchronisation (with the
+// error word checked).  false: the rows need the payload build.
+constexpr int CSR_WORDS = 6;
+const int *csr2tile_words(const TileBufs &t);
+bool csr2tile_settle(TileBufs &t, const int *words);
 // values-only update: tiles built by csr2tile_device (sort_within_rows false)
 // from a CSR of the same structure get the values val (no host round trip)
 int csr2tile_refill_device(Workspace &ws, const int *rowptr, const int *col, const double *val,
@@ -382,7 +413,12 @@ int tile_heatmap_device(Workspace &ws, int tilem, int tilen, const int *tile_ptr
 // products run A in such slices; B stays whole)
 DevTiles tile_row_slice(const DevTiles &A, int I0, int I1);
 // b_sorted: B's CSR rows have strictly increasing columns (lets the walk of a
-// wide tile row's windows cut long B rows to each window)
+// wide tile row's windows cut long B rows to each window).  Step 1 ends in a
+// synchronisation that also brings what extra publishes.
+int symbolic_step1(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
+                   Publish extra = Publish());
+int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
+                   bool b_sorted);
 int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
                     bool b_sorted = false);
 
@@ -415,6 +451,10 @@ int numeric_rows_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
 // numeric step without a copy pipeline: warp-private Gustavson per row pair
 int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
                         const NumericConfig &cfg);
+// every tile row of a product whose tile rows fit one window: A from its CSR
+// rows, B's rows strictly increase, C's CSR alone (its row pointer is written)
+int numeric_tilerow_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
+                           const NumericConfig &cfg);
 // heavy tile rows of a multi-window product, one scalar row per warp: plans
 // the tasks, marks the tile rows in S.w_heavy and runs them on ws.side (the
 // caller waits for ws.join_ev); S.w_heavy and S.w_queue are allocated, the

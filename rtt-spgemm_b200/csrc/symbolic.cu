@@ -240,9 +240,11 @@ __device__ __forceinline__ void step1_out(const DevTiles &A, int I, int count, i
 __global__ void __launch_bounds__(SYM_WARPS * 32)
     k_sym_count(DevTiles A, DevTiles B, int *cnt, int *multi, uint8_t *heavy, int *list,
                 int *list_count, int *wide, int *wide_count, int *wlist, int *wlist_count,
-                int bit_words)
+                int bit_words, const int *err)
 {
     __shared__ WarpSmem1 sm[SYM_WARPS];
+    if (*(volatile const int *)err != 0)
+        return; // the operands' tile index was not made
     const int lane = lane_id(), wi = threadIdx.x >> 5;
     const int I = blockIdx.x * SYM_WARPS + wi;
     if (I >= A.tilem)
@@ -1211,10 +1213,12 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
         // against 1.3 million tiles are not built)
         const int bit_words = ceil_div(std::max(B.tilen, 1), DENSE_TILES) * DENSE_WORDS;
         const size_t bit_bytes = sizeof(uint32_t) * (size_t)bit_words * (size_t)B.tilem;
+        // (a tile for 8 entries while the host does not know B's tiles yet)
+        const size_t b_tiles = (size_t)(B.numtile > 0 ? B.numtile : B.nnz / 8);
         const size_t uni_bytes = sizeof(uint32_t) * (size_t)bit_words * (size_t)tilem;
         const bool bits = wide && B.seg_ptr != nullptr && A.csr_rowptr != nullptr &&
                           A.csr_col != nullptr && std::max(bit_bytes, uni_bytes) <= BIT_BYTES_MAX &&
-                          bit_bytes <= 64 * (size_t)B.numtile;
+                          bit_bytes <= 64 * b_tiles;
         S.dense_windows = 0;
         if (bits)
         {
@@ -1226,7 +1230,8 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
         }
         k_sym_count<<<ceil_div(tilem, SYM_WARPS), SYM_WARPS * 32, 0, s>>>(
             A, B, cnt, flag, S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2,
-            S.s1_list.as<int>(), flag + 3, wlist, flag + 4, bits ? bit_words : 0);
+            S.s1_list.as<int>(), flag + 3, wlist, flag + 4, bits ? bit_words : 0,
+            ws.err.as<int>());
         ws.launches++;
         if (bits)
         {
@@ -1249,8 +1254,8 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
     return RTT_OK;
 }
 
-int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
-                    bool b_sorted)
+int symbolic_step1(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
+                   Publish extra)
 {
     cudaStream_t s = ws.stream;
     if (A.n != B.m)
@@ -1264,11 +1269,26 @@ int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Symboli
     RTT_CHECK(S.c_tile_ptr.ensure(sizeof(int) * (size_t)(tilem + 1), s));
     int *cnt = S.count_tmp.as<int>();
     RTT_CHECK(symbolic_tile_counts(ws, A, B, S, cnt));
-    RTT_CHECK(scan_exclusive_int(ws, cnt, S.c_tile_ptr.as<int>(), tilem));
-    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 16, S.w_flag.p, sizeof(int) * 6,
-                             cudaMemcpyDeviceToHost, s));
-    int numtile = 0;
-    RTT_CHECK(read_int_checked(ws, S.c_tile_ptr.as<int>() + tilem, &numtile, "symbolic step 1"));
+    extra.add(S.w_flag.p, ws.h_scalars + 16, 6);
+    extra.add(S.c_tile_ptr.as<int>() + tilem, ws.h_scalars, 1);
+    publish_error(ws, extra);
+    RTT_CHECK(scan_exclusive_int(ws, cnt, S.c_tile_ptr.as<int>(), tilem, &extra));
+    return wait_published(ws, "symbolic step 1");
+}
+
+int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
+                    bool b_sorted)
+{
+    RTT_CHECK(symbolic_step1(ws, A, B, S));
+    return symbolic_step2(ws, A, B, S, b_sorted);
+}
+
+int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
+                   bool b_sorted)
+{
+    cudaStream_t s = ws.stream;
+    const int tilem = A.tilem;
+    const int numtile = ws.h_scalars[0];
     const bool sym_multi = ws.h_scalars[16] != 0;
     const int n_heavy = ws.h_scalars[18];
     const int n_wide = S.sym_window_slots >= 0 ? ws.h_scalars[20] : 0;
@@ -1376,14 +1396,15 @@ int symbolic_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Symboli
         if (n_heavy > 0 || n_wide > 0)
             RTT_CUDA(cudaStreamWaitEvent(s, ws.join_ev, 0));
     }
-    // read with nnz(C) below (one synchronisation for both)
-    RTT_CUDA(cudaMemcpyAsync(ws.h_scalars + 12, S.w_flag.as<int>() + 1, sizeof(int),
-                             cudaMemcpyDeviceToHost, s));
     // exact sizes: nnz(C) as int64 over tile rows first (int32 overflow check)
     long long *tr64 = S.c_rowptr.as<long long>();
-    RTT_CHECK(scan_exclusive_i64(ws, S.c_tr_nnz.as<int>(), tr64, tilem));
-    long long nnz = 0;
-    RTT_CHECK(read_i64_checked(ws, tr64 + tilem, &nnz, "symbolic step 2"));
+    Publish pub;
+    pub.add(S.w_flag.as<int>() + 1, ws.h_scalars + 12, 1);
+    pub.add(tr64 + tilem, reinterpret_cast<int *>(ws.h_scalars64), 2);
+    publish_error(ws, pub);
+    RTT_CHECK(scan_exclusive_i64(ws, S.c_tr_nnz.as<int>(), tr64, tilem, &pub));
+    RTT_CHECK(wait_published(ws, "symbolic step 2"));
+    const long long nnz = ws.h_scalars64[0];
     S.nnz = nnz;
     S.multi_window = ws.h_scalars[12] != 0;
     if (nnz > (long long)INT_MAX)

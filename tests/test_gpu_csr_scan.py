@@ -77,7 +77,10 @@ def test_scan(case, shift, orc):
             a2.col[-1] = a.n
         else:
             a2.rowptr[-1] += 1
-        with pytest.raises(R.RttError) as e:
-            ctx.symbolic(_dev(a2, shift), db)
-        assert e.value.status == 2
+        for args in ((_dev(a2, shift), db), (_dev(a2, shift), None, R.RTT_OP_AAT)):
+            with pytest.raises(R.RttError) as e:
+                ctx.symbolic(*args)
+            assert e.value.status == 2
+    # the context is as good as before
+    assert ctx.symbolic(da, db)[0] == nnz
     ctx.close()
