@@ -59,30 +59,35 @@ constexpr int S2_STRIDE = 257;           // odd stride: the pairs' mask rows in 
 // step 1 lists as such run in CTAs whose slot table holds u16 slots, up to
 // S2_WIDE_MAX C tiles per window (rtt_config.sym_window_slots; the mask rows
 // after the fixed part of dynamic shared memory).
+// 16 warps when B's row segments drive the walk: with 8 the two CTAs that
+// shared memory leaves per SM were latency-bound (banded 200k, half-band 32:
+// step 2 1.76 -> 1.33 ms).  The window is no larger than the widest such row of
+// the product needs, which leaves room for more CTAs.
+constexpr int S2_WIDE_WARPS = 16;
 constexpr int S2_WIDE_DEFAULT = 2045;
 constexpr int S2_WIDE_MAX = 6000; // the 32-warp CTA's mask rows within 227 KB
 
 // Shared memory of a step-2 CTA; the mask rows (S2_PAIRS rows of `stride`
 // words: per slot, row 2p in the low 16 bits and 2p + 1 in the high 16)
 // follow it.
-template <int NW, bool WIDE>
+template <int NW, bool WIDE, bool SEGS>
 struct CtaSmem2
 {
     using Slot = typename std::conditional<WIDE, uint16_t, uint8_t>::type;
     static constexpr int NONE = WIDE ? 0xFFFF : 0xFF;
     uint32_t bitmap[WWORDS];
     int wordpre[WWORDS];
-    int4 ent[NW][32];                    // per warp: B row start, length, mask shift, mask row
+    int4 ent[SEGS ? 1 : NW][32];         // per warp: B row start, length, mask shift, mask row
     Slot slot[WBITS];                    // window column -> slot
     int lo, hi, nb, wend;
     int share;                           // the warps share the A entries (unbalanced rows)
     int rp[TD + 1];                      // the tile row's A row pointers (segment walk)
 };
 
-template <int NW, bool WIDE>
+template <int NW, bool WIDE, bool SEGS>
 constexpr size_t smem2_bytes(int stride)
 {
-    return (sizeof(CtaSmem2<NW, WIDE>) + 15) / 16 * 16 + sizeof(uint32_t) * S2_PAIRS * (size_t)stride;
+    return (sizeof(CtaSmem2<NW, WIDE, SEGS>) + 15) / 16 * 16 + sizeof(uint32_t) * S2_PAIRS * (size_t)stride;
 }
 
 // First segment in [lo, hi) whose tile column is >= J (a row's segments are
@@ -224,6 +229,8 @@ __device__ __forceinline__ void step1_out(const DevTiles &A, int I, int count, i
         cnt[I] = count;
         if (multi_win)
             atomicOr(multi, 1);
+        if ((hv || wide) && count > *(volatile int *)(multi + 6))
+            atomicMax(multi + 6, count);
         if (heavy != nullptr)
         {
             heavy[I] = dense ? 3 : hv ? 1 : wide ? 2 : 0;
@@ -658,18 +665,19 @@ __global__ void __launch_bounds__(SD_THREADS, 4)
 // the tile rows in order (a heavy one is skipped when heavy[] marks it), or
 // S2_HEAVY_WARPS for the heavy rows of list[] (all warps share the walk).
 template <bool NARROW, int NW, bool SEGS, bool WIDE = false>
-__global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW == S2_SEG_WARPS ? 10 : 1)
+__global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW == S2_SEG_WARPS ? 10 : NW == S2_WIDE_WARPS ? 2 : 1)
     k_sym_rows(DevTiles A, DevTiles B, const int *__restrict__ c_tile_ptr,
                int *__restrict__ c_tile_col, int *__restrict__ c_tile_row,
                uint16_t *__restrict__ c_mask, int *__restrict__ c_tile_cnt,
                int *__restrict__ c_row_cnt, int *__restrict__ c_tr_nnz, int *multi, int *err,
                const uint8_t *__restrict__ heavy, const int *__restrict__ list, int wide_slots)
 {
-    static_assert(NW == S2_WARPS || NW == S2_HEAVY_WARPS || (SEGS && NW == S2_SEG_WARPS),
+    static_assert(NW == S2_WARPS || NW == S2_HEAVY_WARPS || (SEGS && NW == S2_SEG_WARPS) ||
+                      (SEGS && WIDE && NW == S2_WIDE_WARPS),
                   "CTA shapes");
     constexpr int PPW = (S2_PAIRS + NW - 1) / NW; // row pairs each warp counts
     constexpr int NT = NW * 32;
-    using Smem = CtaSmem2<NW, WIDE>;
+    using Smem = CtaSmem2<NW, WIDE, SEGS>;
     using Slot = typename Smem::Slot;
     constexpr int NONE = Smem::NONE;
     // slots per window and the odd stride of the mask rows
@@ -688,7 +696,7 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
     const int nrows = min(TD, A.m - I * TD);
     const int r0 = warp * 2, r1 = r0 + 1; // warp-private walk (NW == S2_WARPS) and counts
     uint32_t *mw = MW + min(warp, S2_PAIRS - 1) * STRIDE;
-    int4 *ent = S.ent[warp];
+    int4 *ent = S.ent[SEGS ? 0 : warp];
     int run[PPW][2] = {}; // entries so far of rows 2p, 2p + 1, pair p = warp + q * NW
 
     // tile-column range reachable from the tile row
@@ -1193,7 +1201,8 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
     // flags: [0] some tile row needs several step-2 windows, [1] several
     // numeric windows, [2] heavy tile rows listed for the wide step-2 CTA,
     // [3] tile rows listed for the wide step-1 CTA, [4] tile rows listed for
-    // the wide-window step-2 CTAs, [5] tile rows with dense masks
+    // the wide-window step-2 CTAs, [5] tile rows with dense masks, [6] the most
+    // C tiles of the rows listed in [2] and [4]
     RTT_CHECK(S.w_flag.ensure(sizeof(int) * 8, s));
     RTT_CUDA(cudaMemsetAsync(S.w_flag.p, 0, sizeof(int) * 8, s));
     RTT_CHECK(S.s2_heavy.ensure((size_t)tilem + 16, s));
@@ -1269,7 +1278,7 @@ int symbolic_step1(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
     RTT_CHECK(S.c_tile_ptr.ensure(sizeof(int) * (size_t)(tilem + 1), s));
     int *cnt = S.count_tmp.as<int>();
     RTT_CHECK(symbolic_tile_counts(ws, A, B, S, cnt));
-    extra.add(S.w_flag.p, ws.h_scalars + 16, 6);
+    extra.add(S.w_flag.p, ws.h_scalars + 16, 7);
     extra.add(S.c_tile_ptr.as<int>() + tilem, ws.h_scalars, 1);
     publish_error(ws, extra);
     RTT_CHECK(scan_exclusive_int(ws, cnt, S.c_tile_ptr.as<int>(), tilem, &extra));
@@ -1293,7 +1302,9 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
     const int n_heavy = ws.h_scalars[18];
     const int n_wide = S.sym_window_slots >= 0 ? ws.h_scalars[20] : 0;
     const int n_dense = ws.h_scalars[21];
-    const int wslots = S.sym_window_slots > 0 ? S.sym_window_slots : S2_WIDE_DEFAULT;
+    const int wslots = S.sym_window_slots > 0
+                           ? S.sym_window_slots
+                           : std::min(S2_WIDE_DEFAULT, std::max(ws.h_scalars[22], S2_SLOTS) | 63);
     const int wstride = (wslots + 2) | 1;
     S.numtile = numtile;
     const size_t nt = (size_t)numtile;
@@ -1356,7 +1367,8 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
             auto hk = segs ? k_sym_rows<false, S2_HEAVY_WARPS, true, true>
                            : b_sorted ? k_sym_rows<true, S2_HEAVY_WARPS, false, true>
                                       : k_sym_rows<false, S2_HEAVY_WARPS, false, true>;
-            RTT_CHECK(go(hk, n_heavy, S2_HEAVY_WARPS * 32, smem2_bytes<S2_HEAVY_WARPS, true>(wstride),
+            RTT_CHECK(go(hk, n_heavy, S2_HEAVY_WARPS * 32, segs ? smem2_bytes<S2_HEAVY_WARPS, true, true>(wstride)
+                              : smem2_bytes<S2_HEAVY_WARPS, true, false>(wstride),
                          ws.side, nullptr, S.s2_list.as<int>(), wslots));
         }
         else if (n_heavy > 0)
@@ -1365,16 +1377,22 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
                            : b_sorted ? k_sym_rows<true, S2_HEAVY_WARPS, false>
                                       : k_sym_rows<false, S2_HEAVY_WARPS, false>;
             RTT_CHECK(go(hk, n_heavy, S2_HEAVY_WARPS * 32,
-                         smem2_bytes<S2_HEAVY_WARPS, false>(S2_STRIDE), ws.side, nullptr,
+                         segs ? smem2_bytes<S2_HEAVY_WARPS, false, true>(S2_STRIDE)
+                              : smem2_bytes<S2_HEAVY_WARPS, false, false>(S2_STRIDE),
+                         ws.side, nullptr,
                          S.s2_list.as<int>(), 0));
         }
         if (n_wide > 0)
         {
-            auto wk = segs ? k_sym_rows<false, S2_WARPS, true, true>
-                           : b_sorted ? k_sym_rows<true, S2_WARPS, false, true>
-                                      : k_sym_rows<false, S2_WARPS, false, true>;
-            RTT_CHECK(go(wk, n_wide, S2_THREADS, smem2_bytes<S2_WARPS, true>(wstride), ws.side,
-                         nullptr, S.s2_wlist.as<int>(), wslots));
+            if (segs)
+                RTT_CHECK(go(k_sym_rows<false, S2_WIDE_WARPS, true, true>, n_wide,
+                             S2_WIDE_WARPS * 32, smem2_bytes<S2_WIDE_WARPS, true, true>(wstride),
+                             ws.side, nullptr, S.s2_wlist.as<int>(), wslots));
+            else
+                RTT_CHECK(go(b_sorted ? k_sym_rows<true, S2_WARPS, false, true>
+                                      : k_sym_rows<false, S2_WARPS, false, true>,
+                             n_wide, S2_THREADS, smem2_bytes<S2_WARPS, true, false>(wstride),
+                             ws.side, nullptr, S.s2_wlist.as<int>(), wslots));
         }
         if (n_heavy > 0 || n_wide > 0)
             RTT_CUDA(cudaEventRecord(ws.join_ev, ws.side));
@@ -1384,14 +1402,16 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
         const uint8_t *skip = n_heavy > 0 || n_wide > 0 || n_dense > 0 ? S.s2_heavy.as<uint8_t>() : nullptr;
         if (small)
             RTT_CHECK(go(k_sym_rows<false, S2_SEG_WARPS, true>, tilem, S2_SEG_WARPS * 32,
-                         smem2_bytes<S2_SEG_WARPS, false>(S2_STRIDE), s, skip, nullptr, 0));
+                         smem2_bytes<S2_SEG_WARPS, false, true>(S2_STRIDE), s, skip, nullptr, 0));
         else
         {
             auto kern = segs ? k_sym_rows<false, S2_WARPS, true>
                              : b_sorted && sym_multi ? k_sym_rows<true, S2_WARPS, false>
                                                      : k_sym_rows<false, S2_WARPS, false>;
-            RTT_CHECK(go(kern, tilem, S2_THREADS, smem2_bytes<S2_WARPS, false>(S2_STRIDE), s, skip,
-                         nullptr, 0));
+            RTT_CHECK(go(kern, tilem, S2_THREADS,
+                         segs ? smem2_bytes<S2_WARPS, false, true>(S2_STRIDE)
+                              : smem2_bytes<S2_WARPS, false, false>(S2_STRIDE),
+                         s, skip, nullptr, 0));
         }
         if (n_heavy > 0 || n_wide > 0)
             RTT_CUDA(cudaStreamWaitEvent(s, ws.join_ev, 0));
