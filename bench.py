@@ -892,7 +892,8 @@ def run_ours(args) -> None:
                      "kernel": ("k_numeric_rows (TMA-staged numeric + fused tile2csr)" if args.staging
                                 else "k_numeric_leaf (FP64 DMMA from hybrid leaves; the leaf "
                                      "build and tile2csr outside the kernel time)" if args.leaf_dmma
-                                else "k_numeric_flat (numeric + fused tile2csr)"),
+                                else ("k_numeric_rowwin" if "rmat" in args.workload
+                                      else "k_numeric_tilerow") + " (numeric + fused tile2csr)"),
                      "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
                      "peak_source": peaks["source"], "kernel_ms": num_ms,

@@ -439,11 +439,10 @@ typedef struct
      * windows of C tiles runs one scalar row per warp where C is written as
      * CSR alone and B's rows strictly increase: rows of more than about
      * split_target products are cut into tasks of about that many (0 = by
-     * nnz(C), between 2^14 and 2^17).  Otherwise it
-     * walks all its products once per window; when that
-     * walk exceeds split_target products the row is cut into tasks of
-     * consecutive windows of about split_target products each, which
-     * persistent CTAs take from a device queue (0 = 2^20);
+     * nnz(C), between 2^14 and 2^17).  Otherwise it walks all its products
+     * once per window; when that walk exceeds split_target products the row
+     * is cut into tasks of consecutive windows of about split_target products
+     * each, which persistent CTAs take from a device queue (0 = 2^20);
      * negative = never split (each tile row's CTA runs its windows in
      * sequence).  Every setting gives bitwise the same C. */
     int split_target;
@@ -496,9 +495,9 @@ typedef struct
      * slower than the windows: a warp per row leaves the others waiting on
      * hub rows), 2 = atomic adds for rows of at least 4 windows, the task's
      * tables in shared memory and its entries shared by all warps (rows of
-     * fewer windows keep them; R-MAT 2^16 A*A^T numeric 21.0 -> 13.0 ms
-     * on B200; values within the FP64 bound, their last bits depending on
-     * the order of the adds).  Only with the fused CSR output and sorted B
+     * fewer windows keep them; R-MAT 2^16 A*A^T numeric 13.0 ms on B200,
+     * the row windows of setting 0 take 4.8 ms; values within the FP64
+     * bound, their last bits depending on the order of the adds).  Only with the fused CSR output and sorted B
      * rows without repeated columns (1: at most 2^20 tile columns);
      * otherwise the windows. */
     int global_rows;
