@@ -482,16 +482,18 @@ __global__ void __launch_bounds__(SB_WARPS * 32)
 // the window's 16 x DENSE_TILES row masks directly addressed in shared memory,
 // so an A entry's segments are OR-ed without a slot table or a second walk of
 // the row for its next window (the wide-window CTAs took 5.6 ms for R-MAT 2^16
-// A*A^T at 16 warps per SM; this takes 2.0 ms at 64).  32 entries' segments are
-// spread over the lanes one by one, whatever their rows' lengths.  Bound by the
-// search of a lane's entry and the shared atomics.
+// A*A^T at 16 warps per SM; this takes 1.7 ms at 64).  A batch's segments are
+// spread over the lanes one by one, whatever their rows' lengths; the warps take
+// batches from a counter (shares fixed ahead left them waiting at the window's
+// barrier: 2.0 ms).  Bound by the search of a lane's entry, the shared atomics
+// and what is left of that wait.
 constexpr int SD_WARPS = 16, SD_THREADS = SD_WARPS * 32;
 struct DenseSmem
 {
     uint32_t mw[S2_PAIRS][DENSE_TILES]; // row 2p in the low half, 2p + 1 in the high
     int start[SD_WARPS][32], pre[SD_WARPS][32]; // 32 entries: first segment, segments before
     int row[SD_WARPS][32];
-    int rp[TD + 1], rowcnt[TD], base;
+    int rp[TD + 1], rowcnt[TD], base, next;
 };
 __global__ void __launch_bounds__(SD_THREADS, 4)
     k_sym_dense(DevTiles A, DevTiles B, int nwin, const int *__restrict__ dlist, int ndense,
@@ -521,6 +523,8 @@ __global__ void __launch_bounds__(SD_THREADS, 4)
             S.rp[tid] = __ldg(A.csr_rowptr + I * TD + tid);
         if (tid < TD)
             S.rowcnt[tid] = 0;
+        if (tid == 0)
+            S.next = 0;
         if (warp == 0)
         {
             // C tiles of the windows before
@@ -534,11 +538,20 @@ __global__ void __launch_bounds__(SD_THREADS, 4)
         __syncthreads();
         const int w0 = wi * DENSE_TILES;
         const int eb = S.rp[0], ee = S.rp[nrows];
-        for (int c0 = eb + warp * 32; c0 < ee; c0 += SD_THREADS)
+        // the warps take the entries from a counter, up to 32 at a time and few
+        // enough for every warp to have some
+        const int per = min(32, (ee - eb + SD_WARPS - 1) / SD_WARPS);
+        for (;;)
         {
+            int c0 = 0;
+            if (lane == 0)
+                c0 = atomicAdd(&S.next, per);
+            c0 = eb + __shfl_sync(FULL, c0, 0);
+            if (c0 >= ee)
+                break;
             const int e = c0 + lane;
             int s0 = 0, ns = 0, r = 0;
-            if (e < ee)
+            if (lane < per && e < ee)
             {
 #pragma unroll
                 for (int h = 8; h > 0; h >>= 1)
