@@ -189,9 +189,10 @@ __device__ void publish_words(const Publish &p)
 __global__ void k_publish(Publish p) { publish_words(p); }
 
 // Scans of up to SCAN_ONE values in one CTA: one launch in place of the
-// library scan's two, its zero and the copies of its results (5-point 61x67
-// A^2: 174 -> 128 us per product with the publications).  8,192 values take
-// 3 us like this and 3 us in the library's scan.
+// library scan's two, its zero and the copies of its results.  With the
+// publication 256 values take 6 us, 4,096 (one round) 7.5 us, 12,500 12 to 17
+// us; the library's launches and a publication about 11 us.  (16 neighbouring
+// values per thread in one round took 16 us for the 12,500.)
 constexpr int SCAN_ONE = 16384, SCAN_THREADS = 1024, SCAN_PER = 4;
 template <typename T>
 __global__ void __launch_bounds__(SCAN_THREADS)
