@@ -838,6 +838,17 @@ int numeric_args_ok(rtt_context c, const int *c_row_ptr, const int *c_col_idx,
 
 } // namespace
 
+// Symbolic step 2 reads A's entries from its CSR rows where it walks B's row
+// segments, else from A's tiles: a B whose rows list no segments (tile columns
+// that decrease) needs them also where A's own rows do not.
+int payload_without_segments(rtt_context c)
+{
+    if (c->B.has_segments || c->A.payload)
+        return RTT_OK;
+    return map_device_error(csr2tile_device(c->ws, c->A.m, c->A.n, c->A.nnz, c->a_rp, c->a_ci,
+                                            c->a_va, c->A, true, false));
+}
+
 // csr2tile of A (and B: A's own tiles for A*A, A^T's for A*A^T), B's scalar
 // CSR rows, and the device views the symbolic and numeric steps take.  The
 // shape checks of the entry points come first.  Shared by the 32-bit product
@@ -909,6 +920,7 @@ int prepare_operands(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B
             c->b_nnz = B->nnz;
         }
         c->b_dups = c->B.dup_cols;
+        RTT_CHECK(payload_without_segments(c));
     }
     const TileBufs &TB = c->b_alias ? c->A : c->B;
     dB = TB.view();
@@ -1771,6 +1783,7 @@ int rtt_spgemm_update_b(rtt_context c, const rtt_csr_view *B, const int *row_new
     c->b_va = b.values;
     c->b_nnz = b.nnz;
     c->b_dups = c->B.dup_cols;
+    RTT_CHECK(payload_without_segments(c));
     DevTiles dB = c->B.view();
     dB.csr_rowptr = c->b_rp;
     dB.csr_col = c->b_ci;

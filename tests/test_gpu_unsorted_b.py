@@ -1,0 +1,94 @@
+"""C = A * B where A's rows are sorted and B's are not: B then lists no row
+segments, and symbolic step 2 walks A's tiles, which a sorted A keeps only for
+such a B.  One and several windows per tile row, hub rows, the 64-bit products
+in chunks, batches, another B for the same A, and new values."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import rtt_spgemm as R
+from conftest import assert_csr_close
+from rtt_spgemm import generators as G
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+DEV = torch.device("cuda:0")
+
+
+def _dev(a):
+    return (a.m, a.n, torch.from_numpy(a.rowptr).to(DEV), torch.from_numpy(a.col).to(DEV),
+            torch.from_numpy(a.val).to(DEV))
+
+
+def _shuffled(a, seed):
+    """The entries of every row in random order."""
+    rng = np.random.default_rng(seed)
+    rows = np.repeat(np.arange(a.m), np.diff(a.rowptr))
+    order = np.lexsort((rng.random(a.nnz), rows))
+    return G.CSR(a.m, a.n, a.rowptr, a.col[order].copy(), a.val[order].copy())
+
+
+def _out(m, nnz, wide=False):
+    return (torch.full((m + 1,), -1, dtype=torch.int64 if wide else torch.int32, device=DEV),
+            torch.full((nnz,), -1, dtype=torch.int32, device=DEV),
+            torch.full((nnz,), float("nan"), dtype=torch.float64, device=DEV))
+
+
+def _close(out, a, b, orc, tag):
+    assert_csr_close(*(x.cpu().numpy() for x in out), *orc.spgemm_csr(a, b), tag)
+
+
+CASES = {
+    "small": lambda: (G.random_csr(500, 300, 0.02, seed=51), G.random_csr(300, 700, 0.015, seed=52)),
+    "windows": lambda: (G.random_csr(300, 900, 0.03, seed=53), G.random_csr(900, 30000, 0.01, seed=54)),
+    "hubs": lambda: (G.rmat(12, 16, seed=3), G.rmat(12, 16, seed=4)),
+    "grid": lambda: (G.stencil_27(9, 1), G.stencil_27(9, 2)),
+}
+
+
+@pytest.mark.parametrize("case", list(CASES))
+def test_sorted_a_unsorted_b(case, orc):
+    a, b = CASES[case]()
+    bs = _shuffled(b, 7)
+    da, db, dbs = _dev(a), _dev(b), _dev(bs)
+    ctx = R.Context(0)
+    nnz, _ = ctx.symbolic(da, dbs)
+    out = _out(a.m, nnz)
+    ctx.numeric(*out)
+    _close(out, a, bs, orc, case)
+    # new values of both, the structure kept
+    va, vb = a.val[::-1].copy(), bs.val[::-1].copy()
+    ctx.numeric_values(torch.from_numpy(va).to(DEV), torch.from_numpy(vb).to(DEV), *out)
+    _close(out, G.CSR(a.m, a.n, a.rowptr, a.col, va), G.CSR(b.m, b.n, b.rowptr, bs.col, vb), orc, case)
+    # the same A with one B after the other
+    nnz, _ = ctx.symbolic(da, db)
+    for d, h in ((dbs, bs), (db, b), (dbs, bs)):
+        nnz, _ = ctx.update_b(d)
+        out = _out(a.m, nnz)
+        ctx.numeric(*out)
+        _close(out, a, h, orc, case + " update_b")
+    ctx.close()
+
+
+@pytest.mark.parametrize("case", ["windows", "hubs"])
+def test_in_chunks(case, orc):
+    a, b = CASES[case]()
+    bs = _shuffled(b, 8)
+    ctx = R.Context(0, dict(chunk_tiles=3000))
+    da, db = _dev(a), _dev(bs)
+    nnz = ctx.symbolic64(da, db)
+    out = _out(a.m, nnz, wide=True)
+    ctx.numeric64(*out)
+    _close(out, a, bs, orc, case)
+    ctx.close()
+
+
+def test_batched(orc):
+    pairs = [CASES[c]() for c in ("small", "grid", "small")]
+    hosts = [(a, _shuffled(b, 9 + i)) for i, (a, b) in enumerate(pairs)]
+    ctx = R.Context(0)
+    As, Bs = [_dev(a) for a, _ in hosts], [_dev(b) for _, b in hosts]
+    for (a, b), c in zip(hosts, R.spgemm_batched(ctx, As, Bs)):
+        _close(c, a, b, orc, "batched")
+    ctx.close()
