@@ -300,11 +300,11 @@ __global__ void __launch_bounds__(PREP_THREADS)
     const int I = blockIdx.x;
     if (I >= tilem)
     {
-        __shared__ int s_cut[CUTS + 1];
+        __shared__ int s_cut[CUTS + 1]; // first columns (16 tilen may pass INT_MAX)
         if (*(volatile const int *)&q->big == 0)
             return;
         for (int g = threadIdx.x; g <= CUTS; g += PREP_THREADS)
-            s_cut[g] = cut_tile[g];
+            s_cut[g] = (int)min((long long)cut_tile[g] * TD, (long long)INT_MAX);
         __syncthreads();
         constexpr int WARPS = PREP_THREADS / 32;
         const int warps = (int)(gridDim.x - tilem) * WARPS;
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(PREP_THREADS)
             const int fe = min(max(__ldg(B.csr_rowptr + k + 1), fs), B.nnz);
             for (int g = lane_id(); g <= CUTS; g += 32)
                 part[(size_t)k * (CUTS + 1) + g] =
-                    g == 0 ? fs : g == CUTS ? fe : lower_bound(B.csr_col, fs, fe, s_cut[g] * TD);
+                    g == 0 ? fs : g == CUTS ? fe : lower_bound(B.csr_col, fs, fe, s_cut[g]);
         }
         return;
     }

@@ -98,3 +98,17 @@ def test_row_windows(case, orc):
         for g, w in zip(got, want):
             assert np.array_equal(g.view(np.int32), w.view(np.int32)), (case, target)
     assert_csr_close(*want, *orc.spgemm_csr(a, b), case)
+
+
+def test_last_columns(orc):
+    """B's columns at the end of the int range: cuts past the last tile column."""
+    width, n = 40000, 2**31 - 1
+    b0 = _pick(400, 3000, width, 10)
+    b = G.CSR(b0.m, n, b0.rowptr, b0.col + (n - width), b0.val)
+    a = _pick(64, 200, 400, 11)
+    want, _ = _run(a, b0, dict(split_target=1))
+    got, st = _run(a, b, dict(split_target=1))
+    assert st["split_windows"] > a.m  # cut into pieces
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1] + (n - width))
+    assert np.array_equal(got[2].view(np.int64), want[2].view(np.int64))
+    assert_csr_close(*want, *orc.spgemm_csr(a, b0), "last columns")
