@@ -257,7 +257,7 @@ __device__ __forceinline__ long long warp_products(FlatSmem<ACC> &S, const Windo
                 // its columns inside the window's tile-column range
                 if (NARROW && CHECK && !SAFE && len > NARROW_MIN)
                 {
-                    const int lo = W.Jlo * TD, hi = (W.Jlo + W.Jspan + 1) * TD;
+                    const int lo = W.Jlo * TD, hi = first_column(W.Jlo + W.Jspan + 1);
                     const int fe = fs + len;
                     const int ci = place; // the entry's place in its tile row
                     const bool keep = cur != nullptr && (unsigned)ci < (unsigned)cursor_cap(A);
@@ -1185,7 +1185,7 @@ __global__ void __launch_bounds__(F_THREADS)
         const int r0 = warp * RPW, r1 = r0 + RPW - 1;
         if (r0 < nrows)
         {
-            const int lo = __ldg(c_tile_col + w0) * TD, hi = (__ldg(c_tile_col + w1 - 1) + 1) * TD;
+            const int lo = __ldg(c_tile_col + w0) * TD, hi = first_column(__ldg(c_tile_col + w1 - 1) + 1);
             const int e_a = s_ea[r0], e_m = s_ea[min(r0 + 1, nrows)], e_e = s_ea[min(r1 + 1, nrows)];
             for (int q0 = e_a; q0 < e_e; q0 += 32)
             {
@@ -1379,7 +1379,7 @@ __global__ void __launch_bounds__(F_THREADS)
         }
         __syncthreads();
         // products: the task's A entries, 32 per warp at a time
-        const int lo = jlo * TD, hi = (jlo + jspan) * TD;
+        const int lo = jlo * TD, hi = first_column(jlo + jspan);
         const int ea = s_ea[0], ee = s_ea[nrows];
         for (int q0 = ea + warp * 32; q0 < ee; q0 += F_THREADS)
         {

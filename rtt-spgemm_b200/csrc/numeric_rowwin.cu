@@ -300,11 +300,11 @@ __global__ void __launch_bounds__(PREP_THREADS)
     const int I = blockIdx.x;
     if (I >= tilem)
     {
-        __shared__ int s_cut[CUTS + 1]; // first columns (16 tilen may pass INT_MAX)
+        __shared__ int s_cut[CUTS + 1]; // first columns
         if (*(volatile const int *)&q->big == 0)
             return;
         for (int g = threadIdx.x; g <= CUTS; g += PREP_THREADS)
-            s_cut[g] = (int)min((long long)cut_tile[g] * TD, (long long)INT_MAX);
+            s_cut[g] = first_column(cut_tile[g]);
         __syncthreads();
         constexpr int WARPS = PREP_THREADS / 32;
         const int warps = (int)(gridDim.x - tilem) * WARPS;

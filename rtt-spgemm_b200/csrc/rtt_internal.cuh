@@ -174,6 +174,13 @@ __device__ __forceinline__ int lower_bound(const int *a, int lo, int hi, int key
     return lo;
 }
 
+// First column of tile column J, also for the one past the last tile column of a
+// matrix of nearly 2^31 columns (INT_MAX: past every column).
+__device__ __forceinline__ int first_column(int J)
+{
+    return (int)min((long long)J * TD, 0x7FFFFFFFll);
+}
+
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return a / b + (a % b != 0); }
 
 // --------------------------------------------------------------- host side

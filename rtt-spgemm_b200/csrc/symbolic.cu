@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
                             if (narrow && len > NARROW_MIN)
                             {
                                 const int sb = lower_bound(B.csr_col, fs, fs + len, w * TD);
-                                len = lower_bound(B.csr_col, sb, fs + len, wend * TD) - sb;
+                                len = lower_bound(B.csr_col, sb, fs + len, first_column(wend)) - sb;
                                 fs = sb;
                             }
                             sh = (r & 1) * 16;
@@ -1079,7 +1079,7 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
                         if (narrow && len > NARROW_MIN)
                         {
                             const int sb = lower_bound(B.csr_col, fs, fs + len, w * TD);
-                            len = lower_bound(B.csr_col, sb, fs + len, wend * TD) - sb;
+                            len = lower_bound(B.csr_col, sb, fs + len, first_column(wend)) - sb;
                             fs = sb;
                         }
                     }

@@ -101,14 +101,23 @@ def test_row_windows(case, orc):
 
 
 def test_last_columns(orc):
-    """B's columns at the end of the int range: cuts past the last tile column."""
+    """B's columns at the end of the int range: cuts and windows that end past
+    the last tile column."""
     width, n = 40000, 2**31 - 1
     b0 = _pick(400, 3000, width, 10)
     b = G.CSR(b0.m, n, b0.rowptr, b0.col + (n - width), b0.val)
     a = _pick(64, 200, 400, 11)
     want, _ = _run(a, b0, dict(split_target=1))
-    got, st = _run(a, b, dict(split_target=1))
-    assert st["split_windows"] > a.m  # cut into pieces
-    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1] + (n - width))
-    assert np.array_equal(got[2].view(np.int64), want[2].view(np.int64))
+    for cfg in (dict(split_target=1), dict(split_target=-1), dict(keep_tiles=1),
+                dict(sym_window_slots=-1), dict(global_rows=2)):
+        got, st = _run(a, b, cfg)
+        if cfg.get("split_target") == 1:
+            assert st["split_windows"] > a.m  # cut into pieces
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1] + (n - width)), cfg
+        if "global_rows" in cfg:
+            # atomic adds, in any order: two sums of at most 200 products of
+            # magnitude below 1, each within 200 * 200 * 2^-53 of the exact one
+            assert np.abs(got[2] - want[2]).max() <= 2 * 200 * 200 * 2.0**-53
+        else:
+            assert np.array_equal(got[2].view(np.int64), want[2].view(np.int64)), cfg
     assert_csr_close(*want, *orc.spgemm_csr(a, b0), "last columns")
