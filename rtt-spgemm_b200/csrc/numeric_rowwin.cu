@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32)
                const int *__restrict__ c_tile_nnz, const int *__restrict__ csr_rowptr,
                const int *__restrict__ cut_tile, uint8_t *__restrict__ heavy,
                RowTask *__restrict__ big, int big_cap, RowTask *__restrict__ normal, int group,
-               bool can_cut, long long target, RowQueue *q, long long *counters)
+               long long target, RowQueue *q, long long *counters)
 {
     const int lane = lane_id();
     const int I = blockIdx.x * PLAN_WARPS + (threadIdx.x >> 5);
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32)
     // work as finding its part of their B rows; `parts` cuts to a piece
     const long long size = max(target, 4ll * nA);
     int parts = 0;
-    if (live && can_cut && work > size + size / 2)
+    if (live && work > size + size / 2)
         for (parts = CUTS / 2; parts > 1 && work * parts > size * CUTS; parts /= 2)
             ;
     const int pieces = parts > 0 ? CUTS / parts : 0;
@@ -286,7 +286,8 @@ __host__ __device__ __forceinline__ size_t row_masks(int cs0, int I, int nt, int
 
 // Where B's rows pass the cuts: part[k * (CUTS + 1) + g] = first entry of row
 // k at or past part g's first column.  Long rows of C are cut at the same
-// columns, so their pieces find their part of every B row by one load.
+// columns, so their pieces find their part of every B row by one load.  (No
+// table for B's of more than PART_BYTES_MAX: their pieces search.)
 //
 // One launch for both: CTAs [0, tilem) copy a tile row's masks, the others list
 // B's parts when some row of C was cut.
@@ -365,14 +366,17 @@ constexpr size_t row_smem_bytes(int span)
     return (sizeof(RowSmem<EW, TW>) + sizeof(uint2) * (size_t)span + 15) / 16 * 16;
 }
 
-template <int EW, int TW>
+// TABLE: B's parts are listed (a kernel of its own: deciding at run time took 2 to 3 %
+// of R-MAT 2^14 A^2 and 2^16 A*A^T).
+template <int EW, int TW, bool TABLE>
 __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
     k_numeric_rowwin(DevTiles A, DevTiles B, long long nnzC, const int *__restrict__ c_tile_ptr,
                      const int *__restrict__ c_tile_col, const uint16_t *__restrict__ maskt,
                      const int *__restrict__ csr_rowptr, int *__restrict__ csr_col,
                      double *__restrict__ csr_val, const RowTask *__restrict__ big,
                      const RowTask *__restrict__ normal, RowQueue *q, int span,
-                     const int *__restrict__ part, int2 *cursors, int *err)
+                     const int *__restrict__ part, const int *__restrict__ cut_tile, int2 *cursors,
+                     int *err)
 {
     static_assert(EW <= 65535, "entry offsets are 16 bits");
     extern __shared__ __align__(16) unsigned char rw_raw[];
@@ -656,11 +660,19 @@ __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
                             if ((unsigned)k < (unsigned)B.m)
                             {
                                 // (parts lie in the row: k_row_prepare)
-                                const int *p = piece ? part + (size_t)k * (CUTS + 1) : B.csr_rowptr + k;
-                                fs = __ldg(p + (piece ? tk.y & 0xFFFF : 0));
-                                fe = __ldg(p + (piece ? tk.y >> 16 : 1));
+                                const bool listed = TABLE && piece;
+                                const int *p = listed ? part + (size_t)k * (CUTS + 1) : B.csr_rowptr + k;
+                                fs = __ldg(p + (listed ? tk.y & 0xFFFF : 0));
+                                fe = __ldg(p + (listed ? tk.y >> 16 : 1));
                                 fs = min(max(fs, 0), B.nnz);
                                 fe = min(max(fe, fs), B.nnz);
+                                if (!TABLE && piece)
+                                {
+                                    fs = lower_bound(B.csr_col, fs, fe,
+                                                     first_column(__ldg(cut_tile + (tk.y & 0xFFFF))));
+                                    fe = lower_bound(B.csr_col, fs, fe,
+                                                     first_column(__ldg(cut_tile + (tk.y >> 16))));
+                                }
                             }
                             if (!first)
                                 fs = lower_bound(B.csr_col, fs, fe, lo);
@@ -739,11 +751,11 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     RTT_CHECK(S.r_big.ensure(sizeof(RowTask) * (size_t)big_cap, s));
     RTT_CHECK(S.r_mask.ensure(sizeof(uint16_t) * row_masks(S.numtile, S.tilem, 0, 0), s));
     RTT_CHECK(S.r_cut.ensure(sizeof(int) * (CUTS + 1), s));
-    // (without the table of B's parts no row is cut)
     const size_t part_bytes = sizeof(int) * (size_t)B.m * (CUTS + 1) + 16;
-    const bool can_cut = part_bytes <= PART_BYTES_MAX;
-    if (can_cut)
+    const bool table = part_bytes <= PART_BYTES_MAX;
+    if (table)
         RTT_CHECK(S.r_part.ensure(part_bytes, s));
+    int *part = table ? S.r_part.as<int>() : nullptr;
     RTT_CHECK(S.w_queue.ensure(sizeof(RowQueue), s));
     RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(RowQueue), s));
     int sms = 0, per_sm = 0;
@@ -756,19 +768,19 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     k_row_plan<EW, TW><<<ceil_div(S.tilem, PLAN_WARPS), PLAN_WARPS * 32, 0, s>>>(
         S.tilem, S.m, A, B, S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(),
         S.c_tile_nnz.as<int>(), cfg.csr_rowptr, cut_tile, S.w_heavy.as<uint8_t>(),
-        S.r_big.as<RowTask>(), big_cap, S.r_normal.as<RowTask>(), group, can_cut,
+        S.r_big.as<RowTask>(), big_cap, S.r_normal.as<RowTask>(), group,
         cfg.split_target > 0 ? (long long)cfg.split_target : auto_target, S.w_queue.as<RowQueue>(),
         cfg.counters);
-    k_row_prepare<<<S.tilem + 8 * sms, PREP_THREADS, 0, s>>>(
+    k_row_prepare<<<S.tilem + (table ? 8 * sms : 0), PREP_THREADS, 0, s>>>(
         S.tilem, S.c_tile_ptr.as<int>(), S.c_mask.as<uint16_t>(), S.w_heavy.as<uint8_t>(),
-        S.r_mask.as<uint16_t>(), B, cut_tile, S.w_queue.as<RowQueue>(), S.r_part.as<int>());
+        S.r_mask.as<uint16_t>(), B, cut_tile, S.w_queue.as<RowQueue>(), part);
     ws.launches += 3;
     // 32-tile words of the column index: a power of two
     int span = 32;
     while (span < RW_SPAN_MAX && span * 32 < S.tilen)
         span *= 2;
     const size_t smem = RW_WARPS * row_smem_bytes<EW, TW>(span);
-    auto kern = k_numeric_rowwin<EW, TW>;
+    auto kern = table ? k_numeric_rowwin<EW, TW, true> : k_numeric_rowwin<EW, TW, false>;
     RTT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     RTT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RW_WARPS * 32, smem));
     // one wave of warps that take tasks from the queue, on the side stream
@@ -780,7 +792,7 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     kern<<<grid, RW_WARPS * 32, smem, ws.side>>>(
         A, B, S.nnz, S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(), S.r_mask.as<uint16_t>(),
         cfg.csr_rowptr, cfg.csr_col, cfg.csr_val, S.r_big.as<RowTask>(), S.r_normal.as<RowTask>(),
-        S.w_queue.as<RowQueue>(), span, S.r_part.as<int>(), S.r_cursor.as<int2>(), ws.err.as<int>());
+        S.w_queue.as<RowQueue>(), span, part, cut_tile, S.r_cursor.as<int2>(), ws.err.as<int>());
     ws.launches++;
     RTT_CUDA(cudaEventRecord(ws.join_ev, ws.side));
     return RTT_OK;

@@ -121,3 +121,28 @@ def test_last_columns(orc):
         else:
             assert np.array_equal(got[2].view(np.int64), want[2].view(np.int64)), cfg
     assert_csr_close(*want, *orc.spgemm_csr(a, b0), "last columns")
+
+
+def test_pieces_without_the_table(orc):
+    """B of more rows than the table of its parts holds: pieces find their part
+    of a B row by searching it."""
+    rows, width = 2_100_000, 6000
+    rng = np.random.default_rng(12)
+    long = set(rng.choice(rows, 3000, replace=False).tolist())
+    counts = np.ones(rows, np.int64)
+    counts[list(long)] = 900
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    col = rng.integers(0, width, rp[-1]).astype(np.int32)
+    for k in long:
+        col[rp[k]:rp[k + 1]] = np.sort(rng.choice(width, 900, replace=False))
+    b = G.CSR(rows, width, rp, col, rng.uniform(-1, 1, col.size))
+    picks = np.array(sorted(long))
+    a = _rows([np.union1d(rng.choice(picks, 1500, replace=False), rng.choice(rows, 15000))
+               for _ in range(24)], rows, 13)
+    want, _ = _run(a, b, dict(split_target=-1))
+    for target in (0, 1):
+        got, st = _run(a, b, dict(split_target=target))
+        assert st["split_windows"] > 8 * a.m  # cut into pieces
+        for g, w in zip(got, want):
+            assert np.array_equal(g.view(np.int32), w.view(np.int32)), target
+    assert_csr_close(*want, *orc.spgemm_csr(a, b), "no table")
