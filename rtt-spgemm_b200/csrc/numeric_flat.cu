@@ -1487,11 +1487,17 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
                       (cfg.global_rows == 2 || S.tilen <= (1 << 20));
     // heavy tile rows one scalar row per warp (numeric_rowwin.cu): CSR output
     // alone, A from its CSR rows, strictly increasing B rows
-    const bool rowwin = split && !glob && acsr && !cfg.conflict_safe && cfg.csr_col != nullptr &&
-                        !cfg.write_tiles;
+    bool rowwin = split && !glob && acsr && !cfg.conflict_safe && cfg.csr_col != nullptr &&
+                  !cfg.write_tiles;
     if (rowwin)
-        RTT_CHECK(numeric_rowwin_device(ws, A, B, S, cfg));
-    else if (split)
+    {
+        // window tasks, as below, when its scratch cannot be had
+        const int st = numeric_rowwin_device(ws, A, B, S, cfg);
+        rowwin = st != RTT_ERR_OUT_OF_MEMORY;
+        if (rowwin)
+            RTT_CHECK(st);
+    }
+    if (split && !rowwin)
     {
         RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(WinQueue), s));
         auto plan = !glob                  ? k_win_plan<ACC_SMALL, 0>
@@ -1573,8 +1579,8 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
         // tasks start while the tile-row CTAs run (the reference's heavy grid
         // enqueued before its light grid, src/dmma_tile_early_split.h:13-27).
         // One wave of resident CTAs; with an empty queue they exit at once.
-        // (strictly increasing B rows with the fused CSR output alone never
-        // come here: numeric_rowwin_device takes them)
+        // (strictly increasing B rows with the fused CSR output alone come
+        // here only without room for numeric_rowwin_device's scratch)
         auto wk = acsr ? (cfg.conflict_safe ? k_numeric_flat<true, ACC_SMALL, CTAS_SMALL, true, true, true>
                                             : k_numeric_flat<false, ACC_SMALL, CTAS_SMALL, true, true, true>)
                        : (cfg.conflict_safe ? k_numeric_flat<true, ACC_SMALL, CTAS_SMALL, true, true, false>

@@ -746,20 +746,40 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
                const NumericConfig &cfg)
 {
     cudaStream_t s = ws.stream;
+    // 32-tile words of the column index: a power of two
+    int span = 32;
+    while (span < RW_SPAN_MAX && span * 32 < S.tilen)
+        span *= 2;
+    const size_t smem = RW_WARPS * row_smem_bytes<EW, TW>(span);
+    // one wave of warps that take tasks from the queue
+    int sms = 0, per_sm = 0;
+    RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+    for (auto k : {k_numeric_rowwin<EW, TW, true>, k_numeric_rowwin<EW, TW, false>})
+        RTT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RTT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_numeric_rowwin<EW, TW, true>,
+                                                           RW_WARPS * 32, smem));
+    const int grid = std::max(1, per_sm * sms);
+    // scratch, before anything is enqueued: without it the caller runs the
+    // windows of the tile-row kernel
     const int big_cap = (int)std::min<long long>(S.nnz / 128 + (1 << 16), 1 << 24);
     RTT_CHECK(S.r_normal.ensure(sizeof(RowTask) * ((size_t)S.m + 16), s));
     RTT_CHECK(S.r_big.ensure(sizeof(RowTask) * (size_t)big_cap, s));
     RTT_CHECK(S.r_mask.ensure(sizeof(uint16_t) * row_masks(S.numtile, S.tilem, 0, 0), s));
     RTT_CHECK(S.r_cut.ensure(sizeof(int) * (CUTS + 1), s));
-    const size_t part_bytes = sizeof(int) * (size_t)B.m * (CUTS + 1) + 16;
-    const bool table = part_bytes <= PART_BYTES_MAX;
-    if (table)
-        RTT_CHECK(S.r_part.ensure(part_bytes, s));
-    int *part = table ? S.r_part.as<int>() : nullptr;
+    RTT_CHECK(S.r_cursor.ensure(sizeof(int2) * (size_t)grid * RW_WARPS * ROW_CURSORS, s));
     RTT_CHECK(S.w_queue.ensure(sizeof(RowQueue), s));
+    // the table of B's parts where it is small enough and can be had
+    const size_t part_bytes = sizeof(int) * (size_t)B.m * (CUTS + 1) + 16;
+    bool table = part_bytes <= PART_BYTES_MAX;
+    if (table)
+    {
+        const int st = S.r_part.ensure(part_bytes, s);
+        table = st == RTT_OK;
+        if (!table && st != RTT_ERR_OUT_OF_MEMORY)
+            return st;
+    }
+    int *part = table ? S.r_part.as<int>() : nullptr;
     RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(RowQueue), s));
-    int sms = 0, per_sm = 0;
-    RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
     int *cut_tile = S.r_cut.as<int>();
     k_cut_tiles<<<1, CUT_THREADS, 0, s>>>(B, S.tilen, cut_tile);
     // a task per row when the groups would leave warps without work
@@ -775,18 +795,8 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
         S.tilem, S.c_tile_ptr.as<int>(), S.c_mask.as<uint16_t>(), S.w_heavy.as<uint8_t>(),
         S.r_mask.as<uint16_t>(), B, cut_tile, S.w_queue.as<RowQueue>(), part);
     ws.launches += 3;
-    // 32-tile words of the column index: a power of two
-    int span = 32;
-    while (span < RW_SPAN_MAX && span * 32 < S.tilen)
-        span *= 2;
-    const size_t smem = RW_WARPS * row_smem_bytes<EW, TW>(span);
     auto kern = table ? k_numeric_rowwin<EW, TW, true> : k_numeric_rowwin<EW, TW, false>;
-    RTT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    RTT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RW_WARPS * 32, smem));
-    // one wave of warps that take tasks from the queue, on the side stream
-    // beside the tile-row CTAs of the other tile rows
-    const int grid = std::max(1, per_sm * sms);
-    RTT_CHECK(S.r_cursor.ensure(sizeof(int2) * (size_t)grid * RW_WARPS * ROW_CURSORS, s));
+    // on the side stream, beside the tile-row CTAs of the other tile rows
     RTT_CUDA(cudaEventRecord(ws.fork_ev, s));
     RTT_CUDA(cudaStreamWaitEvent(ws.side, ws.fork_ev, 0));
     kern<<<grid, RW_WARPS * 32, smem, ws.side>>>(
@@ -803,8 +813,12 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
 int numeric_rowwin_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
                           const NumericConfig &cfg)
 {
-    return S.nnz > EW_LONG * S.m ? rowwin_run<1024, 512>(ws, A, B, S, cfg)
-                                 : rowwin_run<512, 256>(ws, A, B, S, cfg);
+    const int st = S.nnz > EW_LONG * S.m ? rowwin_run<1024, 512>(ws, A, B, S, cfg)
+                                         : rowwin_run<512, 256>(ws, A, B, S, cfg);
+    if (st == RTT_ERR_OUT_OF_MEMORY) // leave the room to what runs instead
+        for (DevBuf *b : {&S.r_normal, &S.r_big, &S.r_mask, &S.r_cursor, &S.r_part})
+            b->release();
+    return st;
 }
 
 } // namespace rtt

@@ -465,7 +465,8 @@ int numeric_tilerow_device(Workspace &ws, const DevTiles &A, const DevTiles &B, 
 // heavy tile rows of a multi-window product, one scalar row per warp: plans
 // the tasks, marks the tile rows in S.w_heavy and runs them on ws.side (the
 // caller waits for ws.join_ev); S.w_heavy and S.w_queue are allocated, the
-// CSR row pointer is written, B's rows strictly increase
+// CSR row pointer is written, B's rows strictly increase.
+// RTT_ERR_OUT_OF_MEMORY: no room for its scratch, nothing was enqueued
 int numeric_rowwin_device(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut &S,
                           const NumericConfig &cfg);
 struct HybridDev;

@@ -193,7 +193,7 @@ __device__ __forceinline__ void fill_bitmap(const DevTiles &A, const DevTiles &B
 }
 
 // B's bitmaps are built up to this size.
-constexpr size_t BIT_BYTES_MAX = size_t(1) << 30;
+constexpr size_t BIT_BYTES_MAX = size_t(1) << 30; // (and C's, as large as that each)
 
 // Step 1 of a tile row with more pairs than this goes to k_sym_count_wide (or
 // k_sym_count_bits): one warp would walk them alone while the rest of the grid
@@ -1237,18 +1237,30 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
         const size_t bit_bytes = sizeof(uint32_t) * (size_t)bit_words * (size_t)B.tilem;
         // (a tile for 8 entries while the host does not know B's tiles yet)
         const size_t b_tiles = (size_t)(B.numtile > 0 ? B.numtile : B.nnz / 8);
+        // the union of every tile row of A likewise against A's tiles
+        const size_t a_tiles = (size_t)(A.numtile > 0 ? A.numtile : A.nnz / 8);
         const size_t uni_bytes = sizeof(uint32_t) * (size_t)bit_words * (size_t)tilem;
-        const bool bits = wide && B.seg_ptr != nullptr && A.csr_rowptr != nullptr &&
-                          A.csr_col != nullptr && std::max(bit_bytes, uni_bytes) <= BIT_BYTES_MAX &&
-                          bit_bytes <= 64 * b_tiles;
+        bool bits = wide && B.seg_ptr != nullptr && A.csr_rowptr != nullptr &&
+                    A.csr_col != nullptr && std::max(bit_bytes, uni_bytes) <= BIT_BYTES_MAX &&
+                    bit_bytes <= 64 * b_tiles && uni_bytes <= 64 * a_tiles;
         S.dense_windows = 0;
         if (bits)
         {
-            S.dense_windows = bit_words / DENSE_WORDS;
-            RTT_CHECK(S.s1_bits.ensure(bit_bytes, s));
-            RTT_CHECK(S.s1_union.ensure(uni_bytes, s));
-            RTT_CHECK(S.s1_wcnt.ensure(sizeof(int) * (size_t)tilem * S.dense_windows, s));
-            RTT_CHECK(S.s2_dlist.ensure(sizeof(int) * (size_t)tilem + 16, s));
+            const int nwin = bit_words / DENSE_WORDS;
+            int st = S.s2_dlist.ensure(sizeof(int) * (size_t)tilem + 16, s);
+            if (st == RTT_OK)
+                st = S.s1_wcnt.ensure(sizeof(int) * (size_t)tilem * nwin, s);
+            if (st == RTT_OK)
+                st = S.s1_union.ensure(uni_bytes, s);
+            if (st == RTT_OK)
+                st = S.s1_bits.ensure(bit_bytes, s);
+            bits = st != RTT_ERR_OUT_OF_MEMORY;
+            if (!bits) // the lists, as below, and the room to them
+                for (DevBuf *b : {&S.s2_dlist, &S.s1_wcnt, &S.s1_union, &S.s1_bits})
+                    b->release();
+            else
+                RTT_CHECK(st);
+            S.dense_windows = bits ? nwin : 0;
         }
         k_sym_count<<<ceil_div(tilem, SYM_WARPS), SYM_WARPS * 32, 0, s>>>(
             A, B, cnt, flag, S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2,

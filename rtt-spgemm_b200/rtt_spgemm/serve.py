@@ -25,11 +25,14 @@ runs, its operands plus the exact upper bound of the symbolic phase for C
 (nnzCub entries of 12 bytes: C cannot have more entries than products) plus
 its row pointer, against a fixed pool.  Operands that a request marks with a
 reuse key stay resident on the device (with A^T for A*A^T requests) and are
-not copied again.  Each context's own workspace (tile index, symbolic
-structure, the window cursors of the numeric step's persistent workers:
-4 bytes per A entry up to 32,768 per worker CTA) sits outside this
-accounting, so pool_bytes should leave room for it below the device's
-memory.
+not copied again.  Each context's own workspace sits outside this
+accounting (and outside structure_bytes, which counts the requests' bounds),
+so pool_bytes should leave room for it below the device's memory: 12 to 16
+bytes per entry of A and B (row segments, tile index), about 100 per C tile,
+and where tile rows of C need several windows 32 more per C tile, 48 MB of
+window cursors, 516 bytes per row of B (at most 1 GiB) and bitmaps of tile
+rows (at most 1 GiB each for B and C).  The last four are done without when
+they cannot be had.
 
 A request whose bound exceeds a quarter of the pool (exclusive_share) runs
 alone once nothing else is in flight, and a batch of one request runs
