@@ -435,16 +435,16 @@ typedef struct
      * streamed by TMA bulk copies through a shared-memory stage ring (the
      * kernel that also runs the DMMA pairs). */
     int b_staging;
-    /* Early split of heavy C tile rows.  A tile row that needs several
-     * windows of C tiles runs one scalar row per warp where C is written as
-     * CSR alone and B's rows strictly increase: rows of more than about
-     * split_target products are cut into tasks of about that many (0 = by
-     * nnz(C), between 2^14 and 2^17).  Otherwise it walks all its products
-     * once per window; when that walk exceeds split_target products the row
-     * is cut into tasks of consecutive windows of about split_target products
-     * each, which persistent CTAs take from a device queue (0 = 2^20);
-     * negative = never split (each tile row's CTA runs its windows in
-     * sequence).  Every setting gives bitwise the same C. */
+    /* Early split of heavy C tile rows: those that need several windows of C
+     * tiles are cut into tasks of about split_target products, which
+     * persistent CTAs take from a device queue.  Where C is written as CSR
+     * alone and B's rows strictly increase, a task is one of the tile row's 16
+     * scalar rows, or a piece of it, and gets a sixteenth of split_target, at
+     * most 2^17 (0 = by nnz(C), 2^14 to 2^17 per row).  Otherwise the tile
+     * row's products are walked once per window and a task is a run of
+     * consecutive windows (0 = 2^20).  Negative = never split (each tile row's
+     * CTA runs its windows in sequence).  Every setting gives bitwise the same
+     * C. */
     int split_target;
     /* Replay the numeric phase as a CUDA graph when nonzero (the default).
      * rtt_spgemm_numeric, rtt_spgemm_numeric_values and

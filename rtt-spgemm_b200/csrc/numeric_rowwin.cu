@@ -71,6 +71,9 @@ constexpr int PLAN_WARPS = 8;
 // window): rows with more are cut.  Between these by nnz(C) / 2048, so that
 // the row tasks of a product number some thousands: 2^14 against 2^16 took
 // R-MAT 2^14 A^2 from 4.36 to 3.80 ms, 2^16 A*A^T from 18.2 to 19.5 ms.
+// rtt_config.split_target counts a whole tile row's products, as for its
+// window tasks: a task of one of its 16 rows gets a sixteenth, and no more than
+// TARGET_MAX.
 constexpr long long TARGET_MIN = 1ll << 14, TARGET_MAX = 1ll << 17;
 
 struct RowTask
@@ -784,13 +787,14 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     k_cut_tiles<<<1, CUT_THREADS, 0, s>>>(B, S.tilen, cut_tile);
     // a task per row when the groups would leave warps without work
     const int group = S.m >= 64 * RW_GROUP * sms ? RW_GROUP : S.m >= 64 * sms ? 2 : 1;
-    const long long auto_target = std::max(TARGET_MIN, std::min(TARGET_MAX, S.nnz / 2048));
+    const long long target =
+        cfg.split_target > 0 ? std::max(1ll, std::min(TARGET_MAX, (long long)cfg.split_target / TD))
+                             : std::max(TARGET_MIN, std::min(TARGET_MAX, S.nnz / 2048));
     k_row_plan<EW, TW><<<ceil_div(S.tilem, PLAN_WARPS), PLAN_WARPS * 32, 0, s>>>(
         S.tilem, S.m, A, B, S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(),
         S.c_tile_nnz.as<int>(), cfg.csr_rowptr, cut_tile, S.w_heavy.as<uint8_t>(),
         S.r_big.as<RowTask>(), big_cap, S.r_normal.as<RowTask>(), group,
-        cfg.split_target > 0 ? (long long)cfg.split_target : auto_target, S.w_queue.as<RowQueue>(),
-        cfg.counters);
+        target, S.w_queue.as<RowQueue>(), cfg.counters);
     k_row_prepare<<<S.tilem + (table ? 8 * sms : 0), PREP_THREADS, 0, s>>>(
         S.tilem, S.c_tile_ptr.as<int>(), S.c_mask.as<uint16_t>(), S.w_heavy.as<uint8_t>(),
         S.r_mask.as<uint16_t>(), B, cut_tile, S.w_queue.as<RowQueue>(), part);

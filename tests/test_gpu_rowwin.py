@@ -146,3 +146,19 @@ def test_pieces_without_the_table(orc):
         for g, w in zip(got, want):
             assert np.array_equal(g.view(np.int32), w.view(np.int32)), target
     assert_csr_close(*want, *orc.spgemm_csr(a, b), "no table")
+
+
+def test_split_target_counts_tile_rows():
+    """A task of one scalar row gets a sixteenth of split_target, at most 2^17:
+    2^18 is this product's default."""
+    a = G.rmat(14, 16, seed=3)
+    want, st0 = _run(a, a, {})
+    _, whole = _run(a, a, dict(split_target=-1))
+    assert whole["split_windows"] == 0
+    tasks = {}
+    for target in (1 << 18, 1 << 22, 1 << 30):
+        got, st = _run(a, a, dict(split_target=target))
+        tasks[target] = st["split_windows"]
+        assert np.array_equal(got[2].view(np.int64), want[2].view(np.int64))
+    assert tasks[1 << 18] == st0["split_windows"]
+    assert tasks[1 << 22] == tasks[1 << 30]  # 2^18 and 2^26 a row: both 2^17
