@@ -8,9 +8,9 @@ The knobs (rtt_config fields):
 * ``b_staging`` - the accumulator / kernel switch: 0 is the flat kernel
   (warp-private Gustavson, direct B row loads), 1 the kernel with B's rows
   streamed through a TMA stage ring (the one that also runs DMMA pairs);
-* ``split_target`` - the tile-row bucket threshold of the early split: tile
-  rows whose windows walk more products than this are cut into window tasks
-  (0: the library default, negative: never);
+* ``split_target`` - the tile-row bucket threshold of the early split: the
+  products of one task of a heavy tile row, or of a run of its windows where
+  the tiles are written (0: the library default, negative: never);
 * ``sym_window_slots`` - the tile-row bucket threshold of symbolic step 2:
   tile rows with more C tiles than 254 run in wide-window CTAs of this many
   slots (0: 2045, -1: never);
@@ -26,7 +26,9 @@ the row count, the mean entries per row and the row-length skew (longest row
 once the operands are resident (after one untimed run each), keeps the
 fastest, and stores it with the candidates' times in a JSON file keyed by the
 GPU's name; later products of the class use the stored choice.  The file is
-``$RTT_TUNE_CACHE`` or ``~/.cache/rtt_spgemm/tune.json``.  All
+``$RTT_TUNE_CACHE`` or ``~/.cache/rtt_spgemm/tune.json``.  Choices timed on
+other kernels than these (another ``VERSION`` in the file) are not used: their
+classes are tuned again.  All
 configurations give results within the same FP64 bound (the DMMA path sums
 some products in another order).
 """
@@ -51,6 +53,10 @@ CANDIDATES = [
     {"dmma_pair_cutoff": 0, "b_staging": 0, "split_target": 0, "persistent_rows": 1},
     {"dmma_pair_cutoff": 0, "b_staging": 0, "split_target": 0, "global_rows": 2},
 ]
+
+# Raised when the kernels behind the knobs change what is fastest (2: heavy tile
+# rows one scalar row per warp, where ``global_rows`` and large splits won before).
+VERSION = 2
 
 OPS = {0: "AB", 1: "AAT"}
 
@@ -90,9 +96,12 @@ class Tuner:
     # -- persistence -------------------------------------------------------
     def _load(self) -> dict:
         try:
-            return json.loads(self.path.read_text())
+            table = json.loads(self.path.read_text())
+            if table.get("version") == VERSION:
+                return table
         except (OSError, ValueError):
-            return {"version": 1, "devices": {}}
+            pass
+        return {"version": VERSION, "devices": {}}
 
     def _save(self) -> None:
         self.path.parent.mkdir(parents=True, exist_ok=True)

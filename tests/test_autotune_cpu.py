@@ -55,3 +55,17 @@ def test_failing_candidate_is_skipped(tmp_path):
     assert t.choose("k", runner)["b_staging"] == 0
     e = json.loads((tmp_path / "t.json").read_text())["devices"]["d"]["k"]
     assert e["candidates"][0]["ms"] is None
+
+
+def test_choices_of_other_kernels_are_dropped(tmp_path):
+    path = tmp_path / "tune.json"
+    old = {"config": {"split_target": 0, "global_rows": 2}, "ms": 1.0}
+    path.write_text(json.dumps({"version": 1, "devices": {"d": {"k": old}}}))
+    cands = [{"split_target": 0}, {"split_target": 0, "global_rows": 2}]
+    t = T.Tuner(path, candidates=cands, device_name="d", repeats=1)
+    assert t.lookup("k") is None
+    assert t.choose("k", lambda cfg: 1.0 + cfg.get("global_rows", 0)) == cands[0]
+    stored = json.loads(path.read_text())
+    assert stored["version"] == T.VERSION and stored["devices"]["d"]["k"]["config"] == cands[0]
+    # and this version's are used
+    assert T.Tuner(path, candidates=cands, device_name="d").lookup("k") == cands[0]
