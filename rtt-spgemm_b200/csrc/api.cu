@@ -840,13 +840,27 @@ int numeric_args_ok(rtt_context c, const int *c_row_ptr, const int *c_col_idx,
 
 // Symbolic step 2 reads A's entries from its CSR rows where it walks B's row
 // segments, else from A's tiles: a B whose rows list no segments (tile columns
-// that decrease) needs them also where A's own rows do not.
+// that decrease) needs them also where A's own rows do not.  (A's and B's rows
+// have been checked.)
 int payload_without_segments(rtt_context c)
 {
-    if (c->B.has_segments || c->A.payload)
+    if (c->B.has_segments || c->B.m == 0 || c->A.payload)
         return RTT_OK;
-    return map_device_error(csr2tile_device(c->ws, c->A.m, c->A.n, c->A.nnz, c->a_rp, c->a_ci,
-                                            c->a_va, c->A, true, false));
+    return map_device_error(csr2tile_payload(c->ws, c->a_rp, c->a_ci, c->a_va, c->A, true));
+}
+
+// The device views that the symbolic and numeric steps take.
+void operand_views(rtt_context c, DevTiles &dA, DevTiles &dB)
+{
+    dB = (c->b_alias ? c->A : c->B).view();
+    dB.csr_rowptr = c->b_rp;
+    dB.csr_col = c->b_ci;
+    dB.csr_val = c->b_va;
+    dB.nnz = (int)c->b_nnz;
+    dA = c->A.view();
+    // A's CSR rows: step 2 walks the tile row's entries straight from them
+    dA.csr_rowptr = c->a_rp;
+    dA.csr_col = c->a_ci;
 }
 
 // csr2tile of A (and B: A's own tiles for A*A, A^T's for A*A^T), B's scalar
@@ -920,24 +934,17 @@ int prepare_operands(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B
             c->b_nnz = B->nnz;
         }
         c->b_dups = c->B.dup_cols;
-        RTT_CHECK(payload_without_segments(c));
+        if (!defer)
+            RTT_CHECK(payload_without_segments(c));
     }
-    const TileBufs &TB = c->b_alias ? c->A : c->B;
-    dB = TB.view();
-    dB.csr_rowptr = c->b_rp;
-    dB.csr_col = c->b_ci;
-    dB.csr_val = c->b_va;
-    dB.nnz = (int)c->b_nnz;
-    dA = c->A.view();
-    // A's CSR rows: step 2 walks the tile row's entries straight from them
-    dA.csr_rowptr = A->row_ptr;
-    dA.csr_col = A->col_idx;
+    operand_views(c, dA, dB);
     return RTT_OK;
 }
 
 // The operands' tile indexes and step 1 up to one synchronisation, which brings
 // the operands' flags and sizes beside C's tiles; operands whose rows need the
-// tile payload (unsorted ones) are then built again, host read by host read.
+// tile payload (unsorted ones, for which the index and step 1 came to nothing)
+// then get it, and step 1 runs again.
 int operands_and_step1(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B, int op,
                        DevTiles &dA, DevTiles &dB)
 {
@@ -958,16 +965,22 @@ int operands_and_step1(rtt_context c, const rtt_csr_view *A, const rtt_csr_view 
         settled &= csr2tile_settle(c->A, ws.h_scalars + 24);
     if (wait_b)
         settled &= csr2tile_settle(c->B, ws.h_scalars + 32);
+    c->b_dups = TB.dup_cols;
     if (!settled)
     {
-        RTT_CHECK(prepare_operands(c, A, B, op, dA, dB));
+        if (wait_a && c->A.generic)
+            RTT_CHECK(map_device_error(csr2tile_payload(ws, c->a_rp, c->a_ci, c->a_va, c->A, true)));
+        if (wait_b && c->B.generic)
+            RTT_CHECK(map_device_error(csr2tile_payload(ws, c->b_rp, c->b_ci, c->b_va, c->B, true)));
+        if (!c->b_alias)
+            RTT_CHECK(payload_without_segments(c));
+        operand_views(c, dA, dB);
         return map_device_error(symbolic_step1(ws, dA, dB, c->S));
     }
     dA.numtile = c->A.numtile;
     dB.numtile = TB.numtile;
     dA.max_row_segs = c->A.max_row_segs;
     dB.max_row_segs = TB.max_row_segs;
-    c->b_dups = TB.dup_cols;
     return RTT_OK;
 }
 
@@ -1784,14 +1797,8 @@ int rtt_spgemm_update_b(rtt_context c, const rtt_csr_view *B, const int *row_new
     c->b_nnz = b.nnz;
     c->b_dups = c->B.dup_cols;
     RTT_CHECK(payload_without_segments(c));
-    DevTiles dB = c->B.view();
-    dB.csr_rowptr = c->b_rp;
-    dB.csr_col = c->b_ci;
-    dB.csr_val = c->b_va;
-    dB.nnz = (int)c->b_nnz;
-    DevTiles dA = c->A.view();
-    dA.csr_rowptr = c->a_rp;
-    dA.csr_col = c->a_ci;
+    DevTiles dA, dB;
+    operand_views(c, dA, dB);
     RTT_CHECK(map_device_error(symbolic_device(ws, dA, dB, c->S, !c->b_dups)));
     c->stats.nnz_b = c->B.nnz;
     c->stats.nnz_c = c->S.nnz;

@@ -203,16 +203,17 @@ __global__ void __launch_bounds__(CS_THREADS)
 // is OR-ed over the lanes of its 32 entries by shuffles; what it has in the
 // next 32 is carried along, and past the warp's chunk it is followed entry by
 // entry.  seg_ptr[r] is the number of segments before row r's first entry.
-// Nothing is written for a CSR with errors.
+// Nothing is written for a CSR with errors, or one whose tile columns decrease
+// in some row (flags[0]): its segments have no use.
 __global__ void __launch_bounds__(CS_THREADS)
     k_csr_segments(int m, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
                    int blocks, const int *__restrict__ cta_cnt, const int *__restrict__ warp_cnt,
                    int *__restrict__ seg_ptr, unsigned long long *__restrict__ seg,
-                   const int *err)
+                   const int *err, const int *flags)
 {
     __shared__ uint32_t s_bits[CS_WARPS][CS_WORDS], s_starts[CS_WARPS][CS_WORDS];
     __shared__ int s_pre[CS_WARPS][CS_WORDS], s_base;
-    if (*(volatile const int *)err != 0)
+    if (*(volatile const int *)err != 0 || *(volatile const int *)flags != 0)
         return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // segments of the CTAs and warps before
@@ -335,12 +336,13 @@ constexpr int ST_WARPS = 4, ST_WORDS = 256, ST_BITS = ST_WORDS * 32;
 __global__ void __launch_bounds__(ST_WARPS * 32)
     k_seg_tiles(int m, int tilem, const int *__restrict__ seg_ptr,
                 const unsigned long long *__restrict__ seg, int *__restrict__ tile_ptr,
-                int *__restrict__ tile_end, int *__restrict__ tile_col, int *out, const int *err)
+                int *__restrict__ tile_end, int *__restrict__ tile_col, int *out, const int *err,
+                const int *flags)
 {
     __shared__ uint32_t s_bits[ST_WARPS][ST_WORDS];
     __shared__ int s_count, s_max;
-    if (*(volatile const int *)err != 0)
-        return;
+    if (*(volatile const int *)err != 0 || *(volatile const int *)flags != 0)
+        return; // (as k_csr_segments)
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     const int I = blockIdx.x * ST_WARPS + warp;
     uint32_t *bits = s_bits[warp];
@@ -1218,8 +1220,7 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     k_csr_scan<<<ch.grid(m), CS_THREADS, 0, s>>>(m, n, nnz, rowptr, col, ch.ctas, ch.blocks,
                                                  cta_cnt, warp_cnt, ws.err.as<int>(), flags);
     ws.launches++;
-    // the segments and the tile index are made before the host sees the flags
-    // (every run of entries in one tile column is a segment, sorted or not),
+    // the segments and the tile index are made before the host sees the flags,
     // so that one synchronisation brings flags, errors and sizes
     if (want_segs)
     {
@@ -1227,7 +1228,7 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
         {
             k_csr_segments<<<ch.ctas, CS_THREADS, 0, s>>>(
                 m, nnz, rowptr, col, ch.blocks, cta_cnt, warp_cnt, out.seg_ptr.as<int>(),
-                out.seg.as<unsigned long long>(), ws.err.as<int>());
+                out.seg.as<unsigned long long>(), ws.err.as<int>(), flags);
             ws.launches++;
         }
         else
@@ -1238,7 +1239,7 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
         k_seg_tiles<<<ceil_div(tilem, ST_WARPS), ST_WARPS * 32, 0, s>>>(
             m, tilem, out.seg_ptr.as<int>(), out.seg.as<unsigned long long>(),
             out.tile_ptr.as<int>(), out.tile_end.as<int>(), out.tile_col.as<int>(), flags + 4,
-            ws.err.as<int>());
+            ws.err.as<int>(), flags);
         ws.launches++;
     }
     if (defer && !payload)
@@ -1255,20 +1256,27 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     RTT_CHECK(wait_published(ws, "csr2tile validate"));
     if (!payload && csr2tile_settle(out, ws.h_scalars + 2))
         return RTT_OK;
-    const bool generic = ws.h_scalars[2] != 0;
     const bool unsorted = ws.h_scalars[3] != 0;
     // rows that are unsorted may hide repeated columns too
     out.dup_cols = ws.h_scalars[4] != 0 || unsorted;
-    out.generic = generic;
-    out.payload = true;
-    out.has_segments = want_segs && !generic;
+    out.generic = ws.h_scalars[2] != 0;
+    out.has_segments = want_segs && !out.generic;
     out.max_row_segs = 0;
+    return csr2tile_payload(ws, rowptr, col, val, out, packed_col, sort_within_rows && unsorted);
+}
 
+int csr2tile_payload(Workspace &ws, const int *rowptr, const int *col, const double *val,
+                     TileBufs &out, bool packed_col, bool sort_rows)
+{
+    cudaStream_t s = ws.stream;
+    const int m = out.m, nnz = out.nnz, tilem = out.tilem;
+    const bool generic = out.generic;
+    out.payload = true;
     int *cnt = out.tmp0.as<int>();
     // heavy tile rows (a CTA each) are listed on the device; their kernels
     // take the list length from device memory, so no host read is needed
     uint8_t *heavy = nullptr;
-    int *hv_list = nullptr, *hv_count = flags + 3;
+    int *hv_list = nullptr, *hv_count = out.tmp1.as<int>() + 3;
     int hv_grid = 0;
     const size_t hv_smem = sizeof(HeavySmem);
     if (!generic)
@@ -1336,7 +1344,7 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     }
     k_set_int<<<1, 1, 0, s>>>(out.tile_nnz.as<int>() + numtile, nnz);
     ws.launches++;
-    if (sort_within_rows && unsorted && numtile > 0)
+    if (sort_rows && numtile > 0)
     {
         k_sort_tile_rows<<<grid_for((long long)numtile * TD, 256), 256, 0, s>>>(
             numtile, out.tile_nnz.as<int>(), out.ptr.as<uint8_t>(), out.col.as<uint8_t>(),

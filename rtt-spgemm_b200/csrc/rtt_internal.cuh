@@ -68,6 +68,9 @@ struct DevTiles
     const int *seg_ptr;               // m + 1
     const unsigned long long *seg;    // seg_ptr[m]
     int max_row_segs;                 // most segments of one row (when seg_ptr is set)
+    // structure-only builds: a device word, not 0 when tile columns decrease in
+    // some row and the index was not made (nullptr: it was)
+    const int *unsorted;
 };
 
 // Tiles [b, e) of tile row I.
@@ -315,10 +318,13 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
 // A deferred structure-only build (defer, payload = false) is enqueued without a
 // host read: its flags and sizes are CSR_WORDS words at csr2tile_words(t), to
 // be published and given to csr2tile_settle after a synchronisation (with the
-// error word checked).  false: the rows need the payload build.
+// error word checked).  false: the rows need the payload build, which
+// csr2tile_payload adds (rows checked and settled, the flags known).
 constexpr int CSR_WORDS = 6;
 const int *csr2tile_words(const TileBufs &t);
 bool csr2tile_settle(TileBufs &t, const int *words);
+int csr2tile_payload(Workspace &ws, const int *rowptr, const int *col, const double *val,
+                     TileBufs &t, bool packed_col, bool sort_rows = false);
 // values-only update: tiles built by csr2tile_device (sort_within_rows false)
 // from a CSR of the same structure get the values val (no host round trip)
 int csr2tile_refill_device(Workspace &ws, const int *rowptr, const int *col, const double *val,

@@ -383,6 +383,7 @@ DevTiles TileBufs::view() const
     t.seg_ptr = has_segments ? seg_ptr.as<int>() : nullptr;
     t.seg = has_segments ? seg.as<unsigned long long>() : nullptr;
     t.max_row_segs = has_segments ? max_row_segs : 0;
+    t.unsorted = payload ? nullptr : csr2tile_words(*this);
     return t;
 }
 

@@ -250,7 +250,9 @@ __global__ void __launch_bounds__(SYM_WARPS * 32)
                 int bit_words, const int *err)
 {
     __shared__ WarpSmem1 sm[SYM_WARPS];
-    if (*(volatile const int *)err != 0)
+    if (*(volatile const int *)err != 0 ||
+        (A.unsorted != nullptr && *(volatile const int *)A.unsorted != 0) ||
+        (B.unsorted != nullptr && *(volatile const int *)B.unsorted != 0))
         return; // the operands' tile index was not made
     const int lane = lane_id(), wi = threadIdx.x >> 5;
     const int I = blockIdx.x * SYM_WARPS + wi;

@@ -84,6 +84,24 @@ def test_in_chunks(case, orc):
     ctx.close()
 
 
+@pytest.mark.parametrize("op", ["A2", "AB", "AAT"])
+def test_set_up_once(op, orc):
+    """Unsorted rows are checked and transposed once: one synchronisation for
+    the operands, one per tiled operand, two for steps 1 and 2."""
+    a, b = CASES["grid"]()
+    s = _shuffled(a, 11)
+    args = {"A2": (s, None, R.RTT_OP_AB), "AB": (s, _shuffled(b, 12), R.RTT_OP_AB),
+            "AAT": (s, None, R.RTT_OP_AAT)}[op]
+    ctx = R.Context(0)
+    dev = (_dev(args[0]), _dev(args[1]) if args[1] else None, args[2])  # borrowed until numeric
+    nnz, _ = ctx.symbolic(*dev)
+    out = _out(s.m, nnz)
+    ctx.numeric(*out)
+    assert ctx.stats()["host_syncs"] <= (6 if op == "AB" else 5)
+    _close(out, s, {"A2": s, "AB": args[1], "AAT": a.transpose()}[op], orc, op)
+    ctx.close()
+
+
 def test_batched(orc):
     pairs = [CASES[c]() for c in ("small", "grid", "small")]
     hosts = [(a, _shuffled(b, 9 + i)) for i, (a, b) in enumerate(pairs)]
