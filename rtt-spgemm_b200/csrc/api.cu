@@ -2213,6 +2213,10 @@ int rtt_spgemm_batched_symbolic(rtt_context c, int count, const rtt_csr_view *A,
     RTT_CUDA(cudaSetDevice(c->ws.device));
     Workspace &ws = c->ws;
     cudaStream_t s = ws.stream;
+    // (a batch's own operands are overwritten)
+    c->have_symbolic = false;
+    c->have_sym64 = false;
+    c->bat_active = false;
     // A's block diagonal (rows at row_off, columns shifted to col_off)
     RTT_CHECK(assemble(c, count, A, row_off, col_off, c->bat_a_rp, c->bat_a_col, c->bat_a_val,
                        c->bat_a_off, c->bat_a_max));
@@ -2380,10 +2384,12 @@ int rtt_reorder_plan_build_variant(rtt_context c, const rtt_csr_view *A, int var
     if (variant < RTT_REORDER_FULL || variant > RTT_REORDER_UNGUARDED)
         return rtt::fail(RTT_ERR_INVALID_ARGUMENT, "reorder_plan_build: unknown variant");
     RTT_CUDA(cudaSetDevice(c->ws.device));
+    // the context's A tiles become scratch: the last product's steps end here
+    c->have_symbolic = false;
+    c->have_sym64 = false;
     // the traversal trusts A's structure: validate it like csr2tile does
     RTT_CHECK(map_device_error(csr2tile_device(c->ws, A->rows, A->cols, (int)A->nnz, A->row_ptr,
                                                A->col_idx, A->values, c->A, true, false)));
-    c->have_symbolic = false; // the context's A tiles were reused as scratch
     return rtt::reorder_plan_device(c->ws, *A, variant, plan);
 }
 

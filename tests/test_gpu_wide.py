@@ -104,3 +104,34 @@ def test_wide_empty():
     A = G.CSR(0, 0, np.zeros(1, np.int32), np.zeros(0, np.int32), np.zeros(0))
     rp, ci, va, _ = _run64(A)
     assert rp.tolist() == [0] and ci.size == 0
+
+
+@pytest.mark.parametrize("other", ["reorder", "symbolic", "batched", "bad_batch", "trim"])
+def test_another_call_between_the_steps(other, orc):
+    """symbolic64, another call on the context that reuses its buffers, then
+    numeric64: refused, and the context is as good as before."""
+    A, B = G.stencil_27(8, 1), G.random_csr(3000, 3000, 0.004, seed=9)
+    ctx = R.Context(0)
+    da, db = _dev(A), _dev(B)
+    nnz = ctx.symbolic64(da)
+    out = [torch.empty(k, dtype=t, device="cuda:0") for k, t in
+           ((A.m + 1, torch.int64), (nnz, torch.int32), (nnz, torch.float64))]
+    if other == "reorder":
+        ctx.reorder_plan(db)
+    elif other == "symbolic":
+        ctx.symbolic(db)
+    elif other == "batched":
+        R.spgemm_batched(ctx, [db, da])
+    elif other == "bad_batch":
+        bad = (B.m, B.n, db[2], torch.full_like(db[3], B.n), db[4])
+        with pytest.raises(R.RttError):
+            R.spgemm_batched(ctx, [bad, da])
+    else:
+        ctx.trim()
+    with pytest.raises(R.RttError) as e:
+        ctx.numeric64(*out)
+    assert e.value.status == 11  # RTT_ERR_STATE
+    assert ctx.symbolic64(da) == nnz
+    ctx.numeric64(*out)
+    assert_csr_close(*(x.cpu().numpy() for x in out), *orc.spgemm_csr(A, A), other)
+    ctx.close()
