@@ -46,6 +46,7 @@ struct GraphSlot
 
 struct rtt_context_s
 {
+    rtt_context_s() { B.operand = 1; }
     rtt::Workspace ws;
     rtt_config cfg;
     rtt::TileBufs A, B;
@@ -968,6 +969,7 @@ int operands_and_step1(rtt_context c, const rtt_csr_view *A, const rtt_csr_view 
     c->b_dups = TB.dup_cols;
     if (!settled)
     {
+        RTT_CUDA(cudaMemsetAsync(ws.err.p, 0, sizeof(int) * 4, ws.stream));
         if (wait_a && c->A.generic)
             RTT_CHECK(map_device_error(csr2tile_payload(ws, c->a_rp, c->a_ci, c->a_va, c->A, true)));
         if (wait_b && c->B.generic)
@@ -1721,7 +1723,7 @@ int rtt_spgemm_symbolic(rtt_context c, const rtt_csr_view *A, const rtt_csr_view
         if (st != RTT_OK)
         {
             // work enqueued before the failure may have left an error word
-            cudaMemsetAsync(ws.err.p, 0, sizeof(int), ws.stream);
+            cudaMemsetAsync(ws.err.p, 0, sizeof(int) * 4, ws.stream);
             return st;
         }
     }

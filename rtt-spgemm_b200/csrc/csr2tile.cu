@@ -90,10 +90,13 @@ __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__
 // flags[0]: some row's tile column decreases (needs the generic path)
 // flags[1]: some row's column decreases (entries not sorted inside rows)
 // flags[2]: some row repeats a column
+// unmade: set for errors and flags[0]; what follows then makes no segments and no
+// index.  A word of its own beside the error word, which is hardly ever written:
+// flags[0], cleared for every matrix, took the small products' kernels 0.5 us each.
 __global__ void __launch_bounds__(CS_THREADS)
     k_csr_scan(int m, int n, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
                int ctas, int blocks, int *__restrict__ cta_cnt, int *__restrict__ warp_cnt,
-               int *err, int *flags)
+               int *err, int *flags, int *unmade)
 {
     __shared__ uint32_t s_bits[CS_WARPS][CS_WORDS];
     __shared__ int s_total;
@@ -110,7 +113,11 @@ __global__ void __launch_bounds__(CS_THREADS)
     if (__syncthreads_or(bad))
     {
         if (tid == 0)
+        {
             set_error(err, DERR_CSR_ROWPTR);
+            if (unmade != nullptr)
+                atomicOr(unmade, 1);
+        }
         return;
     }
     if ((int)blockIdx.x >= ctas)
@@ -179,6 +186,8 @@ __global__ void __launch_bounds__(CS_THREADS)
     {
         if (fl & 8u)
             set_error(err, DERR_CSR_COL);
+        if ((fl & 9u) && unmade != nullptr)
+            atomicOr(unmade, 1);
         for (int f = 0; f < 3; ++f)
             if ((fl >> f) & 1u)
                 atomicOr(&flags[f], 1);
@@ -203,18 +212,16 @@ __global__ void __launch_bounds__(CS_THREADS)
 // is OR-ed over the lanes of its 32 entries by shuffles; what it has in the
 // next 32 is carried along, and past the warp's chunk it is followed entry by
 // entry.  seg_ptr[r] is the number of segments before row r's first entry.
-// Nothing is written for a CSR with errors, or one whose tile columns decrease
-// in some row (flags[0]): its segments have no use.
+// Nothing is written where unmade is set.
 __global__ void __launch_bounds__(CS_THREADS)
     k_csr_segments(int m, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
                    int blocks, const int *__restrict__ cta_cnt, const int *__restrict__ warp_cnt,
                    int *__restrict__ seg_ptr, unsigned long long *__restrict__ seg,
-                   const int *err, const int *flags)
+                   const int *unmade)
 {
     __shared__ uint32_t s_bits[CS_WARPS][CS_WORDS], s_starts[CS_WARPS][CS_WORDS];
     __shared__ int s_pre[CS_WARPS][CS_WORDS], s_base;
-    if (*(volatile const int *)err != 0 || *(volatile const int *)flags != 0)
-        return;
+    const int stop = *(volatile const int *)unmade; // (looked at behind the first loads)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // segments of the CTAs and warps before
     if (tid == 0)
@@ -228,6 +235,8 @@ __global__ void __launch_bounds__(CS_THREADS)
         atomicAdd(&s_base, before);
     const int wc = lane < warp ? __ldg(warp_cnt + blockIdx.x * CS_WARPS + lane) : 0;
     __syncthreads();
+    if (stop != 0)
+        return;
     int base = s_base + warp_sum(wc);
     const long long span = (long long)blocks * CS_BLOCK;
     const long long c0 = (blockIdx.x * (long long)CS_WARPS + warp) * span;
@@ -329,32 +338,37 @@ __global__ void __launch_bounds__(CS_THREADS)
 
 // Tile index of every tile row from its rows' segments: the tile columns of
 // its segments as a bitmap, a warp per tile row, windows of ST_BITS tile
-// columns.  Tile row I's list starts at its first segment, so its place needs
+// columns, or merged where its few segments span many windows.  Tile row I's list starts at its first segment, so its place needs
 // no count of the tiles before it: tile_ptr[I] = seg_ptr[16 I], tile_end[I] one
 // past its last tile.  out[0] += tiles, out[1] = the most segments of a row.
-constexpr int ST_WARPS = 4, ST_WORDS = 256, ST_BITS = ST_WORDS * 32;
-__global__ void __launch_bounds__(ST_WARPS * 32)
+// One wave of ST_CTAS CTAs per SM (32 registers), not a CTA for every 4 tile
+// rows: the 156,000 of a matrix of 10 million short rows queued for the two words
+// of out.  That matrix 361 -> 198 us (10 and 12 CTAs per SM: 237), 96^3 stencil 51
+// -> 39; 200,000 rows of 5 entries among 10 million columns 472 -> 39, by the merge.
+constexpr int ST_WARPS = 4, ST_WORDS = 256, ST_BITS = ST_WORDS * 32, ST_CTAS = 16;
+__global__ void __launch_bounds__(ST_WARPS * 32, ST_CTAS)
     k_seg_tiles(int m, int tilem, const int *__restrict__ seg_ptr,
                 const unsigned long long *__restrict__ seg, int *__restrict__ tile_ptr,
-                int *__restrict__ tile_end, int *__restrict__ tile_col, int *out, const int *err,
-                const int *flags)
+                int *__restrict__ tile_end, int *__restrict__ tile_col, int *out, const int *unmade)
 {
     __shared__ uint32_t s_bits[ST_WARPS][ST_WORDS];
     __shared__ int s_count, s_max;
-    if (*(volatile const int *)err != 0 || *(volatile const int *)flags != 0)
-        return; // (as k_csr_segments)
+    const int stop = *(volatile const int *)unmade; // (looked at behind the first loads)
     const int lane = lane_id(), warp = threadIdx.x >> 5;
-    const int I = blockIdx.x * ST_WARPS + warp;
     uint32_t *bits = s_bits[warp];
+    int count = 0, longest = 0;
     if (threadIdx.x == 0)
         s_count = s_max = 0;
     __syncthreads();
-    if (I < tilem)
+    // (tile rows and columns number at most 2^27)
+    for (int I = blockIdx.x * ST_WARPS + warp; I < tilem; I += gridDim.x * ST_WARPS)
     {
         // lane r < 16: row r's segments
         const int r = min(I * TD + lane, m), r1 = min(r + 1, m);
         const int p = lane < TD ? __ldg(seg_ptr + r) : 0;
         const int e = lane < TD ? __ldg(seg_ptr + r1) : 0;
+        if (stop != 0)
+            break;
         const int s0 = __shfl_sync(FULL, p, 0), s1 = __shfl_sync(FULL, e, TD - 1);
         int lo = INT_MAX, hi = -1;
         if (p < e)
@@ -366,17 +380,46 @@ __global__ void __launch_bounds__(ST_WARPS * 32)
         hi = warp_max(hi);
         const int most = (int)__reduce_max_sync(FULL, (unsigned)(e - p));
         int n = 0;
-        for (long long w = lo; w <= hi; w += ST_BITS)
+        // a window costs its words (32 units) and a read of 32 segments per unit,
+        // the merge a step per segment (2 units: 4 left 20,000 rows of 600 entries
+        // among 10 million columns at 10.1 ms of set-up, 2 and 1 take 8.0)
+        const int windows = hi < 0 ? 0 : (hi - lo) / ST_BITS + 1;
+        const bool merge =
+            windows > 1 && (long long)windows * ((s1 - s0) / 32 + 32) > 2ll * (s1 - s0);
+        if (merge)
         {
-            const int nwords = (int)((min((long long)hi + 1, w + ST_BITS) - w + 31) >> 5);
+            // lane r walks row r's segments, one load ahead; the smallest
+            // column of the 16 is the next tile
+            int q = p;
+            int cur = q < e ? (int)(__ldg(seg + q) >> 16) : INT_MAX;
+            int next = q + 1 < e ? (int)(__ldg(seg + q + 1) >> 16) : INT_MAX;
+            for (;;)
+            {
+                const int T = warp_min(cur);
+                if (T == INT_MAX)
+                    break;
+                if (lane == 0)
+                    tile_col[s0 + n] = T;
+                ++n;
+                if (cur == T)
+                {
+                    cur = next;
+                    ++q;
+                    next = q + 1 < e ? (int)(__ldg(seg + q + 1) >> 16) : INT_MAX;
+                }
+            }
+        }
+        for (int w = lo; w <= hi && !merge; w += ST_BITS)
+        {
+            const int nwords = (min(hi + 1 - w, ST_BITS) + 31) >> 5;
             for (int i = lane; i < nwords; i += 32)
                 bits[i] = 0u;
             __syncwarp();
 #pragma unroll 4
-            for (int q = s0 + lane; q < s1; q += 32)
+            for (unsigned q = s0 + lane; q < (unsigned)s1; q += 32)
             {
-                const long long d = (long long)(__ldg(seg + q) >> 16) - w;
-                if (d >= 0 && d < 32ll * nwords)
+                const int d = (int)(__ldg(seg + q) >> 16) - w;
+                if ((unsigned)d < 32u * nwords)
                     atomicOr(&bits[d >> 5], 1u << (d & 31));
             }
             __syncwarp();
@@ -386,7 +429,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32)
                 const int v = __popc(word), incl = warp_incl_scan(v);
                 int at = s0 + n + incl - v;
                 for (; word != 0u; word &= word - 1u)
-                    tile_col[at++] = (int)w + (q0 + lane) * 32 + __ffs(word) - 1;
+                    tile_col[at++] = w + (q0 + lane) * 32 + __ffs(word) - 1;
                 n += __shfl_sync(FULL, incl, 31);
             }
             __syncwarp();
@@ -395,9 +438,14 @@ __global__ void __launch_bounds__(ST_WARPS * 32)
         {
             tile_ptr[I] = s0;
             tile_end[I] = s0 + n;
-            atomicAdd(&s_count, n);
-            atomicMax(&s_max, most);
         }
+        count += n;
+        longest = max(longest, most);
+    }
+    if (lane == 0)
+    {
+        atomicAdd(&s_count, count);
+        atomicMax(&s_max, longest);
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -1182,7 +1230,8 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     // [0..2] flags of the rows, [3] heavy tile rows listed, [4] tiles, [5] the
     // most segments of a row
     RTT_CHECK(out.tmp1.ensure(sizeof(int) * 8, s));
-    int *flags = out.tmp1.as<int>();
+    int *flags = out.tmp1.as<int>(), *unmade = ws.err.as<int>() + 1 + out.operand;
+    out.unmade = unmade;
     RTT_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * 6, s));
     if (m == 0)
     {
@@ -1218,7 +1267,8 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     int *cta_cnt = want_segs ? out.seg_cnt.as<int>() : nullptr;
     int *warp_cnt = want_segs ? cta_cnt + ch.ctas : nullptr;
     k_csr_scan<<<ch.grid(m), CS_THREADS, 0, s>>>(m, n, nnz, rowptr, col, ch.ctas, ch.blocks,
-                                                 cta_cnt, warp_cnt, ws.err.as<int>(), flags);
+                                                 cta_cnt, warp_cnt, ws.err.as<int>(), flags,
+                                                 want_segs ? unmade : nullptr);
     ws.launches++;
     // the segments and the tile index are made before the host sees the flags,
     // so that one synchronisation brings flags, errors and sizes
@@ -1228,7 +1278,7 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
         {
             k_csr_segments<<<ch.ctas, CS_THREADS, 0, s>>>(
                 m, nnz, rowptr, col, ch.blocks, cta_cnt, warp_cnt, out.seg_ptr.as<int>(),
-                out.seg.as<unsigned long long>(), ws.err.as<int>(), flags);
+                out.seg.as<unsigned long long>(), unmade);
             ws.launches++;
         }
         else
@@ -1236,10 +1286,11 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     }
     if (!payload)
     {
-        k_seg_tiles<<<ceil_div(tilem, ST_WARPS), ST_WARPS * 32, 0, s>>>(
+        const int sms = ws.sms;
+        k_seg_tiles<<<std::min(ceil_div(tilem, ST_WARPS), ST_CTAS * sms), ST_WARPS * 32, 0, s>>>(
             m, tilem, out.seg_ptr.as<int>(), out.seg.as<unsigned long long>(),
             out.tile_ptr.as<int>(), out.tile_end.as<int>(), out.tile_col.as<int>(), flags + 4,
-            ws.err.as<int>(), flags);
+            unmade);
         ws.launches++;
     }
     if (defer && !payload)
@@ -1262,6 +1313,8 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     out.generic = ws.h_scalars[2] != 0;
     out.has_segments = want_segs && !out.generic;
     out.max_row_segs = 0;
+    if (want_segs && out.generic)
+        RTT_CUDA(cudaMemsetAsync(unmade, 0, sizeof(int), s));
     return csr2tile_payload(ws, rowptr, col, val, out, packed_col, sort_within_rows && unsorted);
 }
 
@@ -1289,8 +1342,7 @@ int csr2tile_payload(Workspace &ws, const int *rowptr, const int *col, const dou
         k_c2t_heavy_mark<<<grid_for(tilem, 256), 256, 0, s>>>(m, tilem, rowptr, col, heavy,
                                                               hv_list, hv_count);
         ws.launches++;
-        int sms = 0;
-        RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+        const int sms = ws.sms;
         hv_grid = std::min(tilem, 2 * sms);
         RTT_CUDA(cudaFuncSetAttribute(k_c2t_heavy_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)hv_smem));
@@ -1393,8 +1445,7 @@ int csr2tile_refill_device(Workspace &ws, const int *rowptr, const int *col, con
             m, tilem, rowptr, col, val, t.tile_ptr.as<int>(), t.tile_col.as<int>(),
             t.tile_row.as<int>(), t.tile_nnz.as<int>(), t.ptr.as<uint8_t>(), t.col.as<uint8_t>(),
             t.val.as<double>(), t.mask.as<uint16_t>(), packed_col ? 1 : 0, ws.err.as<int>(), heavy);
-        int sms = 0;
-        RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+        const int sms = ws.sms;
         const size_t hv_smem = sizeof(HeavySmem);
         RTT_CUDA(cudaFuncSetAttribute(k_c2t_heavy_fill, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)hv_smem));
@@ -1424,7 +1475,8 @@ int validate_csr_device(Workspace &ws, int m, int n, int nnz, const int *rowptr,
     {
         const CsChunks ch(nnz);
         k_csr_scan<<<ch.grid(m), CS_THREADS, 0, ws.stream>>>(
-            m, n, nnz, rowptr, col, ch.ctas, ch.blocks, nullptr, nullptr, ws.err.as<int>(), flags);
+            m, n, nnz, rowptr, col, ch.ctas, ch.blocks, nullptr, nullptr, ws.err.as<int>(), flags,
+            nullptr);
         ws.launches++;
     }
     Publish pub;

@@ -1537,8 +1537,8 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
     if (glob)
     {
         // the global-row workers, on the side stream beside the tile-row CTAs
-        int per_sm = 0, sms = 0;
-        RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+        int per_sm = 0;
+        const int sms = ws.sms;
         RTT_CUDA(cudaEventRecord(ws.fork_ev, s));
         RTT_CUDA(cudaStreamWaitEvent(ws.side, ws.fork_ev, 0));
         if (cfg.global_rows == 2)
@@ -1585,10 +1585,10 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
                                             : k_numeric_flat<false, ACC_SMALL, CTAS_SMALL, true, true, true>)
                        : (cfg.conflict_safe ? k_numeric_flat<true, ACC_SMALL, CTAS_SMALL, true, true, false>
                                             : k_numeric_flat<false, ACC_SMALL, CTAS_SMALL, true, true, false>);
-        int per_sm = 0, sms = 0;
+        int per_sm = 0;
+        const int sms = ws.sms;
         RTT_CUDA(cudaFuncSetAttribute(wk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         RTT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wk, F_THREADS, smem));
-        RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
         const int grid = std::max(1, per_sm * sms);
         RTT_CHECK(S.w_cursor.ensure(sizeof(int) * (size_t)grid * cursor_cap(A), s));
         RTT_CUDA(cudaEventRecord(ws.fork_ev, s));
@@ -1621,10 +1621,10 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
         light = S.multi_window
                     ? k_numeric_flat<false, ACC_SMALL, CTAS_SMALL, false, true, true, false, true>
                     : k_numeric_flat<false, ACC_SMALL, CTAS_SMALL, false, false, true, false, true>;
-        int per_sm = 0, sms = 0;
+        int per_sm = 0;
+        const int sms = ws.sms;
         RTT_CUDA(cudaFuncSetAttribute(light, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         RTT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, light, F_THREADS, smem));
-        RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
         light_grid = std::max(1, std::min(per_sm * sms, S.tilem));
         if (!split)
             RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(WinQueue), s));

@@ -755,8 +755,8 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
         span *= 2;
     const size_t smem = RW_WARPS * row_smem_bytes<EW, TW>(span);
     // one wave of warps that take tasks from the queue
-    int sms = 0, per_sm = 0;
-    RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+    const int sms = ws.sms;
+    int per_sm = 0;
     for (auto k : {k_numeric_rowwin<EW, TW, true>, k_numeric_rowwin<EW, TW, false>})
         RTT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     RTT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_numeric_rowwin<EW, TW, true>,

@@ -68,9 +68,9 @@ struct DevTiles
     const int *seg_ptr;               // m + 1
     const unsigned long long *seg;    // seg_ptr[m]
     int max_row_segs;                 // most segments of one row (when seg_ptr is set)
-    // structure-only builds: a device word, not 0 when tile columns decrease in
-    // some row and the index was not made (nullptr: it was)
-    const int *unsorted;
+    // structure-only builds: the workspace's word for an index that was not made,
+    // for errors of the CSR or tile columns that decrease in a row (nullptr: it was)
+    const int *unmade;
 };
 
 // Tiles [b, e) of tile row I.
@@ -222,8 +222,9 @@ struct DevBuf
 struct Workspace
 {
     int device = 0;
+    int sms = 0; // the device's SMs
     cudaStream_t stream = nullptr;
-    DevBuf err;        // int device error word
+    DevBuf err;        // device error word, and operand i's index not made (word 1 + i)
     DevBuf scan_tmp;   // CUB temp storage
     DevBuf tmp[4];     // grow-only scratch of the transpose and the batch tables
     int *h_scalars = nullptr; // pinned, 64 ints
@@ -283,6 +284,8 @@ void freeze_growth(bool on);
 struct TileBufs
 {
     DevBuf tile_ptr, tile_col, tile_row, tile_nnz, ptr, col, val, mask;
+    int operand = 0; // its word in Workspace::err
+    int *unmade = nullptr;
     DevBuf tile_end; // structure-only builds: tile row I is [tile_ptr[I], tile_end[I])
     DevBuf csc_ptr, csc_row, csc_data, row_data;
     DevBuf tmp0, tmp1, tmp2, tmp3;

@@ -112,6 +112,7 @@ int Workspace::init(int dev)
         return fail(RTT_ERR_INVALID_ARGUMENT, "device index out of range");
     RTT_CUDA(cudaSetDevice(dev));
     int major = 0, minor = 0;
+    RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     RTT_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
     RTT_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
     if (major < 10)
@@ -294,7 +295,7 @@ int error_word_seen(Workspace &ws, const char *stage)
     int code = ws.h_scalars[8];
     if (code != 0)
     {
-        cudaMemsetAsync(ws.err.p, 0, sizeof(int), ws.stream);
+        cudaMemsetAsync(ws.err.p, 0, sizeof(int) * 4, ws.stream);
         return fail(RTT_ERR_DEVICE_CHECK,
                     std::string(stage) + ": device check failed, code " + std::to_string(code));
     }
@@ -383,7 +384,7 @@ DevTiles TileBufs::view() const
     t.seg_ptr = has_segments ? seg_ptr.as<int>() : nullptr;
     t.seg = has_segments ? seg.as<unsigned long long>() : nullptr;
     t.max_row_segs = has_segments ? max_row_segs : 0;
-    t.unsorted = payload ? nullptr : csr2tile_words(*this);
+    t.unmade = payload ? nullptr : unmade;
     return t;
 }
 

@@ -247,13 +247,12 @@ __device__ __forceinline__ void step1_out(const DevTiles &A, int I, int count, i
 __global__ void __launch_bounds__(SYM_WARPS * 32)
     k_sym_count(DevTiles A, DevTiles B, int *cnt, int *multi, uint8_t *heavy, int *list,
                 int *list_count, int *wide, int *wide_count, int *wlist, int *wlist_count,
-                int bit_words, const int *err)
+                int bit_words)
 {
     __shared__ WarpSmem1 sm[SYM_WARPS];
-    if (*(volatile const int *)err != 0 ||
-        (A.unsorted != nullptr && *(volatile const int *)A.unsorted != 0) ||
-        (B.unsorted != nullptr && *(volatile const int *)B.unsorted != 0))
-        return; // the operands' tile index was not made
+    // (looked at behind the first loads)
+    const int ua = A.unmade != nullptr ? *(volatile const int *)A.unmade : 0;
+    const int ub = B.unmade != nullptr ? *(volatile const int *)B.unmade : 0;
     const int lane = lane_id(), wi = threadIdx.x >> 5;
     const int I = blockIdx.x * SYM_WARPS + wi;
     if (I >= A.tilem)
@@ -261,6 +260,8 @@ __global__ void __launch_bounds__(SYM_WARPS * 32)
     WarpSmem1 &S = sm[wi];
     int a0, a1;
     tile_range(A, I, a0, a1);
+    if ((ua | ub) != 0)
+        return; // an operand's tile index was not made
     int lo, hi;
     long long pairs;
     row_window(A, B, a0, a1, lo, hi, pairs);
@@ -1230,8 +1231,7 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
     {
         int *flag = S.w_flag.as<int>();
         int *wlist = wide ? S.s2_wlist.as<int>() : nullptr;
-        int sms = 0;
-        RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+        const int sms = ws.sms;
         // B's tile rows as bitmaps, where they are not much larger than B's
         // tile lists (R-MAT 2^16: 2 MB, 2^20: 512 MB; the 96^3 stencil's 380 MB
         // against 1.3 million tiles are not built)
@@ -1266,8 +1266,7 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
         }
         k_sym_count<<<ceil_div(tilem, SYM_WARPS), SYM_WARPS * 32, 0, s>>>(
             A, B, cnt, flag, S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2,
-            S.s1_list.as<int>(), flag + 3, wlist, flag + 4, bits ? bit_words : 0,
-            ws.err.as<int>());
+            S.s1_list.as<int>(), flag + 3, wlist, flag + 4, bits ? bit_words : 0);
         ws.launches++;
         if (bits)
         {
@@ -1367,8 +1366,7 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
             // rows with dense masks: their windows add up the counts
             RTT_CUDA(cudaMemsetAsync(S.c_row_cnt.p, 0, sizeof(int) * (size_t)(S.m + 1), s));
             RTT_CUDA(cudaMemsetAsync(S.c_tr_nnz.p, 0, sizeof(int) * (size_t)(tilem + 1), s));
-            int sms = 0;
-            RTT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ws.device));
+            const int sms = ws.sms;
             RTT_CUDA(cudaFuncSetAttribute(k_sym_dense, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)sizeof(DenseSmem)));
             const long long items = (long long)n_dense * S.dense_windows;

@@ -84,3 +84,41 @@ def test_scan(case, shift, orc):
     # the context is as good as before
     assert ctx.symbolic(da, db)[0] == nnz
     ctx.close()
+
+
+# (rows of A, columns, rows' lengths): tile rows of few segments over one, two
+# and many windows of 8192 tile columns, merged or not; of many segments over a
+# few; runs of one tile column
+WIDE = {
+    "two_windows": (200, 16 * 8192 + 5, 6),
+    "merge_few": (200, 5_000_000, 5),
+    "merge_one": (100, 100_000_000, 1),
+    "merge_more": (40, 200_000_000, 120),
+    "windows": (40, 600_000, 900),
+    "last": (60, 2**31 - 1, 7),
+}
+
+
+@pytest.mark.parametrize("case", list(WIDE))
+def test_wide_tile_index(case):
+    """The tile index of wide, nearly empty rows: tiles counted and binned."""
+    m, n, per = WIDE[case]
+    rng = np.random.default_rng(m + per)
+    cols = rng.integers(0, n, (m, per))
+    cols[:, -1] = np.minimum(cols[:, 0] + rng.integers(0, 16, m), n - 1)  # runs of one tile
+    rows = [np.unique(r) for r in cols]
+    rows[m // 2] = np.zeros(0, np.int64)
+    rp = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
+    b = G.CSR(m, n, rp, np.concatenate(rows).astype(np.int32), np.ones(rp[-1]))
+    a = _csr([3] * 10, m, 1)
+    ctx = R.Context(0)
+    dev = (_dev(a), _dev(b))  # borrowed
+    ctx.symbolic(*dev)
+    assert ctx.stats()["tiles_b"] == _tiles(b)
+    tilem, tilen = -(-m // 16), -(-n // 16)
+    tiles = np.unique((np.repeat(np.arange(m), np.diff(rp)) // 16).astype(np.int64) * tilen +
+                      b.col // 16)
+    want = np.zeros((64, 64), np.int64)
+    np.add.at(want, (tiles // tilen * 64 // tilem, tiles % tilen * 64 // tilen), 1)
+    assert np.array_equal(np.asarray(ctx.tile_heatmap("B", 64)).reshape(64, 64), want)
+    ctx.close()
