@@ -31,7 +31,7 @@ namespace
 // ------------------------------------------------------------ validation
 // The checks and the row segments go over the entries, not the rows: a warp
 // takes a chunk of consecutive entries, 256 at a time, whatever rows they
-// belong to, so hub rows and empty rows cost what their entries cost.  (A warp
+// belong to, so a hub row costs what its entries cost.  (A warp
 // per 32 rows left the 32 hub rows of an R-MAT matrix to one warp: 460 us for
 // the checks of R-MAT 2^16's 1M entries and 1 ms for its segments; now 14 and
 // 19 us.  96^3 stencil, 23.4M entries: 45 us and 110 us before, 44 and 124 us.)  The row starts among the 256 entries are marked in a shared bitmap.
@@ -59,9 +59,37 @@ __device__ __forceinline__ int warp_lower_bound(const int *__restrict__ a, int n
     return lo;
 }
 
+// The rest of mark_rows where many rows are empty: every entry is looked up in the
+// row pointer.
+__device__ __forceinline__ int look_up_rows(uint32_t *bits, const int *__restrict__ rowptr, int rows,
+                                         int cursor, long long s0, long long end)
+{
+    const int lane = lane_id();
+    const int last = cursor + warp_lower_bound(rowptr + cursor, rows - cursor, end);
+    __syncwarp();
+    for (int i = 0; i < CS_WORDS; ++i)
+    {
+        const long long j = s0 + i * 32 + lane;
+        bool start = false;
+        if (j < end)
+        {
+            const int r = lower_bound(rowptr, cursor, last, (int)j);
+            start = r < last && __ldg(rowptr + r) == (int)j;
+        }
+        const unsigned st = __ballot_sync(FULL, start);
+        if (lane == 0)
+            bits[i] |= st;
+    }
+    return last;
+}
+
 // Marks the rows that start in [s0, end), from row `cursor` on (the first that
 // starts at or past s0), in the warp's cleared bitmap; returns the first row
-// that starts at or past end.
+// that starts at or past end.  The rows are walked, 32 and then 128 at a time;
+// past WALK_STEPS of those, among empty rows, the entries are looked up in the row
+// pointer instead (the walk alone left the 18 million empty rows of a matrix of 5
+// million entries to two warps: 276 ms of symbolic step, now 3.0).
+constexpr int WALK_STEPS = 4;
 __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__ rowptr, int rows,
                                          int cursor, long long s0, long long end)
 {
@@ -69,17 +97,33 @@ __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__
     if (lane < CS_WORDS)
         bits[lane] = 0u;
     __syncwarp();
-    for (;;)
-    {
-        const int r = cursor + lane;
+    auto mark = [&](int r) -> bool {
         const long long x = r < rows ? (long long)__ldg(rowptr + r) : LLONG_MAX;
         const bool in = x < end;
         if (in && x >= s0)
             atomicOr(&bits[(x - s0) >> 5], 1u << ((x - s0) & 31));
-        const int n = __popc(__ballot_sync(FULL, in));
-        cursor += n;
-        if (n < 32)
-            break;
+        return in;
+    };
+    int n = __popc(__ballot_sync(FULL, mark(cursor + lane)));
+    cursor += n;
+    if (n == 32)
+    {
+        for (int step = 0; step < WALK_STEPS; ++step)
+        {
+            bool in[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                in[q] = mark(cursor + q * 32 + lane);
+            n = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                n += __popc(__ballot_sync(FULL, in[q]));
+            cursor += n;
+            if (n < 128)
+                break;
+        }
+        if (n == 128)
+            cursor = look_up_rows(bits, rowptr, rows, cursor, s0, end);
     }
     __syncwarp();
     return cursor;
@@ -90,10 +134,10 @@ __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__
 // flags[0]: some row's tile column decreases (needs the generic path)
 // flags[1]: some row's column decreases (entries not sorted inside rows)
 // flags[2]: some row repeats a column
-// unmade: set for errors and flags[0]; what follows then makes no segments and no
+// unmade (one of two words beside the error word): set for errors and flags[0]; what follows then makes no segments and no
 // index.  A word of its own beside the error word, which is hardly ever written:
 // flags[0], cleared for every matrix, took the small products' kernels 0.5 us each.
-__global__ void __launch_bounds__(CS_THREADS)
+__global__ void __launch_bounds__(CS_THREADS, 4)
     k_csr_scan(int m, int n, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
                int ctas, int blocks, int *__restrict__ cta_cnt, int *__restrict__ warp_cnt,
                int *err, int *flags, int *unmade)
@@ -211,12 +255,13 @@ __global__ void __launch_bounds__(CS_THREADS)
 // 16-bit row mask in tile J, as csr2tile writes it into mask[].  A run's mask
 // is OR-ed over the lanes of its 32 entries by shuffles; what it has in the
 // next 32 is carried along, and past the warp's chunk it is followed entry by
-// entry.  seg_ptr[r] is the number of segments before row r's first entry.
+// entry.  word[i] = {segments that start in entries 32 i .. 32 i + 31, segments
+// before them}, for segments_before.
 // Nothing is written where unmade is set.
-__global__ void __launch_bounds__(CS_THREADS)
+__global__ void __launch_bounds__(CS_THREADS, 4)
     k_csr_segments(int m, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
                    int blocks, const int *__restrict__ cta_cnt, const int *__restrict__ warp_cnt,
-                   int *__restrict__ seg_ptr, unsigned long long *__restrict__ seg,
+                   uint2 *__restrict__ word, unsigned long long *__restrict__ seg,
                    const int *unmade)
 {
     __shared__ uint32_t s_bits[CS_WARPS][CS_WORDS], s_starts[CS_WARPS][CS_WORDS];
@@ -256,7 +301,6 @@ __global__ void __launch_bounds__(CS_THREADS)
         for (int i = 0; i < CS_WORDS; ++i)
             c[i] = s0 + i * 32 + lane < c1 ? __ldg(col + s0 + i * 32 + lane) : 0;
         int last = s0 > 0 ? __ldg(col + s0 - 1) : 0;
-        const int first = cursor;
         cursor = mark_rows(bits, rowptr, m, cursor, s0, min(c1, s0 + CS_BLOCK));
         int n = 0; // segments of the block so far
 #pragma unroll
@@ -303,11 +347,8 @@ __global__ void __launch_bounds__(CS_THREADS)
             }
         }
         __syncwarp();
-        for (int r = first + lane; r < cursor; r += 32)
-        {
-            const int d = (int)(__ldg(rowptr + r) - s0);
-            seg_ptr[r] = base + pre[d >> 5] + __popc(starts[d >> 5] & ((1u << (d & 31)) - 1u));
-        }
+        if (lane < CS_WORDS && s0 + lane * 32 < c1)
+            word[(s0 >> 5) + lane] = make_uint2(starts[lane], (unsigned)(base + pre[lane]));
         base += n;
         __syncwarp(); // before the bitmaps are written again
     }
@@ -330,25 +371,43 @@ __global__ void __launch_bounds__(CS_THREADS)
         if (lane == 0)
             seg[open_at] = ((unsigned long long)open_T << 16) | open_mk;
     }
-    // after the last entry: empty rows, and the total
-    if (c1 == nnz)
-        for (int r = cursor + lane; r <= m; r += 32)
-            seg_ptr[r] = base;
+    // rows that start past the last entry
+    if (c1 == nnz && (nnz & 31) == 0 && lane == 0)
+        word[nnz >> 5] = make_uint2(0u, (unsigned)base);
+}
+
+// Segments before row r's first entry (all of them for r = m).
+__device__ __forceinline__ int segments_before(const int *__restrict__ rowptr,
+                                               const uint2 *__restrict__ word, int r)
+{
+    const int d = __ldg(rowptr + r);
+    const uint2 w = __ldg(word + (d >> 5));
+    return (int)w.y + __popc(w.x & ((1u << (d & 31)) - 1u));
+}
+
+// seg_ptr where no tile index is made from the segments (k_seg_tiles writes it).
+__global__ void k_seg_rows(int m, const int *__restrict__ rowptr, const uint2 *__restrict__ word,
+                           int *__restrict__ seg_ptr, const int *unmade)
+{
+    const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (r <= m && *(volatile const int *)unmade == 0)
+        seg_ptr[r] = segments_before(rowptr, word, (int)r);
 }
 
 // Tile index of every tile row from its rows' segments: the tile columns of
 // its segments as a bitmap, a warp per tile row, windows of ST_BITS tile
 // columns, or merged where its few segments span many windows.  Tile row I's list starts at its first segment, so its place needs
 // no count of the tiles before it: tile_ptr[I] = seg_ptr[16 I], tile_end[I] one
-// past its last tile.  out[0] += tiles, out[1] = the most segments of a row.
+// past its last tile.  seg_ptr[r] is the number of segments before row r's first
+// entry.  out[0] += tiles, out[1] = the most segments of a row.
 // One wave of ST_CTAS CTAs per SM (32 registers), not a CTA for every 4 tile
 // rows: the 156,000 of a matrix of 10 million short rows queued for the two words
 // of out.  That matrix 361 -> 198 us (10 and 12 CTAs per SM: 237), 96^3 stencil 51
 // -> 39; 200,000 rows of 5 entries among 10 million columns 472 -> 39, by the merge.
 constexpr int ST_WARPS = 4, ST_WORDS = 256, ST_BITS = ST_WORDS * 32, ST_CTAS = 16;
 __global__ void __launch_bounds__(ST_WARPS * 32, ST_CTAS)
-    k_seg_tiles(int m, int tilem, const int *__restrict__ seg_ptr,
-                const unsigned long long *__restrict__ seg, int *__restrict__ tile_ptr,
+    k_seg_tiles(int m, int tilem, const int *__restrict__ rowptr, const uint2 *__restrict__ word,
+                int *__restrict__ seg_ptr, const unsigned long long *__restrict__ seg, int *__restrict__ tile_ptr,
                 int *__restrict__ tile_end, int *__restrict__ tile_col, int *out, const int *unmade)
 {
     __shared__ uint32_t s_bits[ST_WARPS][ST_WORDS];
@@ -364,11 +423,16 @@ __global__ void __launch_bounds__(ST_WARPS * 32, ST_CTAS)
     for (int I = blockIdx.x * ST_WARPS + warp; I < tilem; I += gridDim.x * ST_WARPS)
     {
         // lane r < 16: row r's segments
-        const int r = min(I * TD + lane, m), r1 = min(r + 1, m);
-        const int p = lane < TD ? __ldg(seg_ptr + r) : 0;
-        const int e = lane < TD ? __ldg(seg_ptr + r1) : 0;
+        const int d = lane <= TD ? __ldg(rowptr + min(I * TD + lane, m)) : 0;
         if (stop != 0)
             break;
+        const uint2 wd = __ldg(word + (d >> 5));
+        int p = (int)wd.y + __popc(wd.x & ((1u << (d & 31)) - 1u));
+        int e = __shfl_down_sync(FULL, p, 1);
+        if ((lane < TD || I == tilem - 1) && lane <= TD && I * TD + lane <= m)
+            seg_ptr[I * TD + lane] = p;
+        if (lane >= TD)
+            p = e = 0;
         const int s0 = __shfl_sync(FULL, p, 0), s1 = __shfl_sync(FULL, e, TD - 1);
         int lo = INT_MAX, hi = -1;
         if (p < e)
@@ -1231,7 +1295,6 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     // most segments of a row
     RTT_CHECK(out.tmp1.ensure(sizeof(int) * 8, s));
     int *flags = out.tmp1.as<int>(), *unmade = ws.err.as<int>() + 1 + out.operand;
-    out.unmade = unmade;
     RTT_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * 6, s));
     if (m == 0)
     {
@@ -1254,6 +1317,7 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
     {
         RTT_CHECK(out.seg_cnt.ensure(sizeof(int) * ((size_t)ch.ctas * (CS_WARPS + 1) + 1), s));
         RTT_CHECK(out.seg_ptr.ensure(sizeof(int) * ((size_t)m + 1), s));
+        RTT_CHECK(out.seg_word.ensure(sizeof(uint2) * ((size_t)nnz / 32 + 1), s));
         // at most one segment per entry: sized by nnz, no host read
         RTT_CHECK(out.seg.ensure(sizeof(unsigned long long) * ((size_t)nnz + 1), s));
     }
@@ -1277,18 +1341,25 @@ int csr2tile_device(Workspace &ws, int m, int n, int nnz, const int *rowptr, con
         if (nnz > 0)
         {
             k_csr_segments<<<ch.ctas, CS_THREADS, 0, s>>>(
-                m, nnz, rowptr, col, ch.blocks, cta_cnt, warp_cnt, out.seg_ptr.as<int>(),
+                m, nnz, rowptr, col, ch.blocks, cta_cnt, warp_cnt, out.seg_word.as<uint2>(),
                 out.seg.as<unsigned long long>(), unmade);
             ws.launches++;
         }
         else
-            RTT_CUDA(cudaMemsetAsync(out.seg_ptr.p, 0, sizeof(int) * ((size_t)m + 1), s));
+            RTT_CUDA(cudaMemsetAsync(out.seg_word.p, 0, sizeof(uint2), s));
+        if (payload)
+        {
+            k_seg_rows<<<grid_for((long long)m + 1, 256), 256, 0, s>>>(
+                m, rowptr, out.seg_word.as<uint2>(), out.seg_ptr.as<int>(), unmade);
+            ws.launches++;
+        }
     }
     if (!payload)
     {
         const int sms = ws.sms;
         k_seg_tiles<<<std::min(ceil_div(tilem, ST_WARPS), ST_CTAS * sms), ST_WARPS * 32, 0, s>>>(
-            m, tilem, out.seg_ptr.as<int>(), out.seg.as<unsigned long long>(),
+            m, tilem, rowptr, out.seg_word.as<uint2>(), out.seg_ptr.as<int>(),
+            out.seg.as<unsigned long long>(),
             out.tile_ptr.as<int>(), out.tile_end.as<int>(), out.tile_col.as<int>(), flags + 4,
             unmade);
         ws.launches++;

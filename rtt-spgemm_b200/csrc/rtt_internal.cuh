@@ -68,9 +68,6 @@ struct DevTiles
     const int *seg_ptr;               // m + 1
     const unsigned long long *seg;    // seg_ptr[m]
     int max_row_segs;                 // most segments of one row (when seg_ptr is set)
-    // structure-only builds: the workspace's word for an index that was not made,
-    // for errors of the CSR or tile columns that decrease in a row (nullptr: it was)
-    const int *unmade;
 };
 
 // Tiles [b, e) of tile row I.
@@ -224,7 +221,7 @@ struct Workspace
     int device = 0;
     int sms = 0; // the device's SMs
     cudaStream_t stream = nullptr;
-    DevBuf err;        // device error word, and operand i's index not made (word 1 + i)
+    DevBuf err;        // device error word; words 1 and 2: A's, B's index was not made
     DevBuf scan_tmp;   // CUB temp storage
     DevBuf tmp[4];     // grow-only scratch of the transpose and the batch tables
     int *h_scalars = nullptr; // pinned, 64 ints
@@ -285,11 +282,10 @@ struct TileBufs
 {
     DevBuf tile_ptr, tile_col, tile_row, tile_nnz, ptr, col, val, mask;
     int operand = 0; // its word in Workspace::err
-    int *unmade = nullptr;
     DevBuf tile_end; // structure-only builds: tile row I is [tile_ptr[I], tile_end[I])
     DevBuf csc_ptr, csc_row, csc_data, row_data;
     DevBuf tmp0, tmp1, tmp2, tmp3;
-    DevBuf seg_ptr, seg, seg_cnt; // row segments (csr2tile_device with segments = true)
+    DevBuf seg_ptr, seg, seg_cnt, seg_word; // row segments (csr2tile_device with segments = true)
     int m = 0, n = 0, tilem = 0, tilen = 0, numtile = 0, nnz = 0;
     bool has_segments = false;
     int max_row_segs = 0; // most segments of one row (structure-only builds; else 0 = unknown)
@@ -305,7 +301,7 @@ struct TileBufs
         const DevBuf *all[] = {&tile_ptr, &tile_col, &tile_row, &tile_nnz, &ptr,  &col,
                                &val,      &mask,     &csc_ptr,  &csc_row,  &csc_data,
                                &row_data, &tmp0,     &tmp1,     &tmp2,     &tmp3,
-                               &seg_ptr,  &seg,      &seg_cnt,  &tile_end};
+                               &seg_ptr,  &seg,      &seg_cnt,  &seg_word, &tile_end};
         for (const DevBuf *b : all)
             f(*b);
     }

@@ -384,7 +384,6 @@ DevTiles TileBufs::view() const
     t.seg_ptr = has_segments ? seg_ptr.as<int>() : nullptr;
     t.seg = has_segments ? seg.as<unsigned long long>() : nullptr;
     t.max_row_segs = has_segments ? max_row_segs : 0;
-    t.unmade = payload ? nullptr : unmade;
     return t;
 }
 

@@ -247,12 +247,11 @@ __device__ __forceinline__ void step1_out(const DevTiles &A, int I, int count, i
 __global__ void __launch_bounds__(SYM_WARPS * 32)
     k_sym_count(DevTiles A, DevTiles B, int *cnt, int *multi, uint8_t *heavy, int *list,
                 int *list_count, int *wide, int *wide_count, int *wlist, int *wlist_count,
-                int bit_words)
+                int bit_words, const int *err)
 {
     __shared__ WarpSmem1 sm[SYM_WARPS];
     // (looked at behind the first loads)
-    const int ua = A.unmade != nullptr ? *(volatile const int *)A.unmade : 0;
-    const int ub = B.unmade != nullptr ? *(volatile const int *)B.unmade : 0;
+    const int ua = *(volatile const int *)(err + 1), ub = *(volatile const int *)(err + 2);
     const int lane = lane_id(), wi = threadIdx.x >> 5;
     const int I = blockIdx.x * SYM_WARPS + wi;
     if (I >= A.tilem)
@@ -1266,7 +1265,8 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
         }
         k_sym_count<<<ceil_div(tilem, SYM_WARPS), SYM_WARPS * 32, 0, s>>>(
             A, B, cnt, flag, S.s2_heavy.as<uint8_t>(), S.s2_list.as<int>(), flag + 2,
-            S.s1_list.as<int>(), flag + 3, wlist, flag + 4, bits ? bit_words : 0);
+            S.s1_list.as<int>(), flag + 3, wlist, flag + 4, bits ? bit_words : 0,
+            ws.err.as<int>());
         ws.launches++;
         if (bits)
         {

@@ -51,16 +51,28 @@ CASES = {
     "one_row": lambda: _csr([5000], 9000, 4),                   # one row over many warps
     "long_run": lambda: _csr([0, 900, 0, 1100, 3], 1200, 5, runs=True),
     "empty": lambda: _csr([3] + [0] * 4000 + [5] * 60 + [0] * 3000, 500, 6),
+    # empty rows: walked, and past 544 of them among 256 entries looked up
+    "gap40": lambda: _csr(([3] + [0] * 40) * 300, 500, 9),
+    "gap600": lambda: _csr(([2] + [0] * 600) * 40 + [5] * 100, 500, 10),
+    "gap5000": lambda: _csr(([37] + [0] * 5000 + [1]) * 9, 400, 11, runs=True),
+    "front": lambda: _csr([0] * 30000 + [7] * 100, 300, 12),
+    "back": lambda: _csr([8] * 64 + [0] * 30000, 300, 13),     # 512 entries: the last word is full
+    "middle": lambda: _csr([4] * 100 + [0] * 30000 + [9] * 100, 300, 14),
     "many": lambda: _csr([24] * 120000, 5000, 7, runs=True),    # several blocks to a warp
 }
 
 
-@pytest.mark.parametrize("shift", [0, 1])
+# (payload: segments beside the tiles, without the tile index from them)
+@pytest.mark.parametrize("shift,cfg", [(0, {}), (1, {}), (0, dict(dmma_pair_cutoff=4000))])
 @pytest.mark.parametrize("case", list(CASES))
-def test_scan(case, shift, orc):
+def test_scan(case, shift, cfg, orc):
     a = CASES[case]()
     b = _csr([2] * a.n, 200, 8)
-    ctx = R.Context(0)
+    if cfg:  # the segments that step 2 reads are B's
+        filled = np.flatnonzero(np.diff(a.rowptr))
+        pick = _csr([min(2, filled.size)] * 50, filled.size, 8)
+        a, b = G.CSR(50, a.m, pick.rowptr, filled[pick.col].astype(np.int32), pick.val), a
+    ctx = R.Context(0, cfg)
     da, db = _dev(a, shift), _dev(b)
     nnz, _ = ctx.symbolic(da, db)
     out = (torch.empty(a.m + 1, dtype=torch.int32, device=DEV),
@@ -71,7 +83,7 @@ def test_scan(case, shift, orc):
     assert st["tiles_a"] == _tiles(a) and st["tiles_b"] == _tiles(b)
     assert_csr_close(*(x.cpu().numpy() for x in out), *orc.spgemm_csr(a, b), case)
     # the last entry's column, or the row pointer's end, out of range
-    for bad in ("col", "rowptr"):
+    for bad in () if cfg else ("col", "rowptr"):
         a2 = G.CSR(a.m, a.n, a.rowptr.copy(), a.col.copy(), a.val)
         if bad == "col":
             a2.col[-1] = a.n
