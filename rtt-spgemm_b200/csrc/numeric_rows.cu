@@ -671,7 +671,7 @@ int numeric_rows_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
         RTT_CHECK(S.c_col.ensure(nnz + 16, s));
         RTT_CHECK(S.c_val.ensure(sizeof(double) * nnz + 16, s));
     }
-    if (cfg.csr_col != nullptr)
+    if (cfg.csr_rowptr != nullptr)
         RTT_CHECK(csr_rowptr_device(ws, S, cfg.csr_rowptr));
     if (S.numtile == 0 || S.tilem == 0)
         return RTT_OK;

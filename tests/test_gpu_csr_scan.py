@@ -134,3 +134,32 @@ def test_wide_tile_index(case):
     np.add.at(want, (tiles // tilen * 64 // tilem, tiles % tilen * 64 // tilen), 1)
     assert np.array_equal(np.asarray(ctx.tile_heatmap("B", 64)).reshape(64, 64), want)
     ctx.close()
+
+
+@pytest.mark.parametrize("cfg", [{}, dict(keep_tiles=1), dict(fused_csr_output=0), dict(b_staging=1),
+                                 dict(dmma_pair_cutoff=1), dict(leaf_dmma=1)],
+                         ids=lambda c: "_".join(c) or "default")
+@pytest.mark.parametrize("empty", ["rows", "product"])
+def test_empty_product(empty, cfg):
+    """C without entries, its columns and values NULL: the row pointer is
+    written all the same.  No entries at all, or tiles that meet where no row
+    and column do."""
+    a = _csr([0] * 500, 300, 15) if empty == "rows" else _csr([1] * 500, 300, 15)
+    if empty == "product":
+        a.col[:] = 16 * (a.col // 16)  # first rows of B's tiles, which are empty
+    b = _csr([0 if k % 16 == 0 else 3 for k in range(300)], 200, 16)
+    ctx = R.Context(0, cfg)
+    dev = (_dev(a), _dev(b))
+    nnz, tiles = ctx.symbolic(*dev)
+    assert nnz == 0 and (tiles > 0) == (empty == "product")
+    out = (torch.full((501,), -1, dtype=torch.int32, device=DEV),
+           torch.empty(0, dtype=torch.int32, device=DEV),
+           torch.empty(0, dtype=torch.float64, device=DEV))
+    for _ in range(3):  # the third replays a graph
+        ctx.numeric(*out)
+        assert not out[0].any()
+        out[0].fill_(-1)
+    if empty == "product":
+        ctx.numeric_values(dev[0][4], dev[1][4], *out)
+        assert not out[0].any()
+    ctx.close()
