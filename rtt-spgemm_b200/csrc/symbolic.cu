@@ -363,8 +363,10 @@ __global__ void __launch_bounds__(S1_WIDE_WARPS * 32)
 }
 
 // B's tile rows as bitmaps of tile columns, bit_words (a multiple of
-// DENSE_WORDS) words each, when step 1 listed wide rows: a warp per tile row.
-constexpr int BITS_WARPS = 4;
+// DENSE_WORDS) words each, when step 1 listed wide rows: a warp per tile row, one
+// wave of CTAs (the 156,000 of a B of 10 million rows took 162 us to find nothing
+// listed).
+constexpr int BITS_WARPS = 4, BITS_CTAS = 16;
 __global__ void __launch_bounds__(BITS_WARPS * 32)
     k_tile_bitmaps(DevTiles B, int bit_words, const int *wide_count, uint32_t *__restrict__ bits)
 {
@@ -372,32 +374,33 @@ __global__ void __launch_bounds__(BITS_WARPS * 32)
     if (*(volatile const int *)wide_count == 0)
         return;
     const int lane = lane_id();
-    const int K = blockIdx.x * BITS_WARPS + (threadIdx.x >> 5);
-    if (K >= B.tilem)
-        return;
     uint32_t *sb = s_bits[threadIdx.x >> 5];
-    uint32_t *out = bits + (size_t)K * bit_words;
-    int b0, b1;
-    tile_range(B, K, b0, b1);
-    for (int w0 = 0; w0 < bit_words; w0 += WWORDS)
+    for (int K = blockIdx.x * BITS_WARPS + (threadIdx.x >> 5); K < B.tilem;
+         K += gridDim.x * BITS_WARPS)
     {
-        const int nw = min(WWORDS, bit_words - w0);
-        for (int i = lane; i < nw; i += 32)
-            sb[i] = 0u;
-        __syncwarp();
-        // the list's part in these words (tile columns increase)
-        const int lo = lower_bound(B.tile_col, b0, b1, w0 * 32);
-        for (int b = lo + lane; b < b1; b += 32)
+        uint32_t *out = bits + (size_t)K * bit_words;
+        int b0, b1;
+        tile_range(B, K, b0, b1);
+        for (int w0 = 0; w0 < bit_words; w0 += WWORDS)
         {
-            const int d = __ldg(B.tile_col + b) - w0 * 32;
-            if (d >= nw * 32)
-                break;
-            atomicOr(&sb[d >> 5], 1u << (d & 31));
+            const int nw = min(WWORDS, bit_words - w0);
+            for (int i = lane; i < nw; i += 32)
+                sb[i] = 0u;
+            __syncwarp();
+            // the list's part in these words (tile columns increase)
+            const int lo = lower_bound(B.tile_col, b0, b1, w0 * 32);
+            for (int b = lo + lane; b < b1; b += 32)
+            {
+                const int d = __ldg(B.tile_col + b) - w0 * 32;
+                if (d >= nw * 32)
+                    break;
+                atomicOr(&sb[d >> 5], 1u << (d & 31));
+            }
+            __syncwarp();
+            for (int i = lane; i < nw; i += 32)
+                out[w0 + i] = sb[i];
+            __syncwarp();
         }
-        __syncwarp();
-        for (int i = lane; i < nw; i += 32)
-            out[w0 + i] = sb[i];
-        __syncwarp();
     }
 }
 
@@ -1270,7 +1273,8 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
         ws.launches++;
         if (bits)
         {
-            k_tile_bitmaps<<<ceil_div(B.tilem, BITS_WARPS), BITS_WARPS * 32, 0, s>>>(
+            k_tile_bitmaps<<<std::min(ceil_div(B.tilem, BITS_WARPS), BITS_CTAS * sms),
+                             BITS_WARPS * 32, 0, s>>>(
                 B, bit_words, flag + 3, S.s1_bits.as<uint32_t>());
             k_sym_count_bits<<<std::min(tilem, 8 * sms), SB_WARPS * 32, 0, s>>>(
                 A, bit_words, S.s1_bits.as<uint32_t>(), cnt, S.s1_wcnt.as<int>(),
