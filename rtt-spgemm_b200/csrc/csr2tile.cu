@@ -89,7 +89,7 @@ __device__ __forceinline__ int look_up_rows(uint32_t *bits, const int *__restric
 // past WALK_STEPS of those, among empty rows, the entries are looked up in the row
 // pointer instead (the walk alone left the 18 million empty rows of a matrix of 5
 // million entries to two warps: 276 ms of symbolic step, now 3.0).
-constexpr int WALK_STEPS = 4;
+constexpr int WALK_STEPS = 16;
 __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__ rowptr, int rows,
                                          int cursor, long long s0, long long end)
 {
@@ -479,12 +479,20 @@ __global__ void __launch_bounds__(ST_WARPS * 32, ST_CTAS)
             for (int i = lane; i < nwords; i += 32)
                 bits[i] = 0u;
             __syncwarp();
-#pragma unroll 4
-            for (unsigned q = s0 + lane; q < (unsigned)s1; q += 32)
+            // (four loads in flight: a hub's tile row has tens of thousands)
+            for (unsigned q = s0 + lane; q < (unsigned)s1; q += 128)
             {
-                const int d = (int)(__ldg(seg + q) >> 16) - w;
-                if ((unsigned)d < 32u * nwords)
-                    atomicOr(&bits[d >> 5], 1u << (d & 31));
+                unsigned long long v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    v[u] = q + 32 * u < (unsigned)s1 ? __ldg(seg + q + 32 * u) : ~0ull;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const int d = (int)(v[u] >> 16) - w;
+                    if ((unsigned)d < 32u * nwords)
+                        atomicOr(&bits[d >> 5], 1u << (d & 31));
+                }
             }
             __syncwarp();
             for (int q0 = 0; q0 < nwords; q0 += 32)

@@ -51,7 +51,7 @@ CASES = {
     "one_row": lambda: _csr([5000], 9000, 4),                   # one row over many warps
     "long_run": lambda: _csr([0, 900, 0, 1100, 3], 1200, 5, runs=True),
     "empty": lambda: _csr([3] + [0] * 4000 + [5] * 60 + [0] * 3000, 500, 6),
-    # empty rows: walked, and past 544 of them among 256 entries looked up
+    # empty rows: walked, and past 2,080 of them among 256 entries looked up
     "gap40": lambda: _csr(([3] + [0] * 40) * 300, 500, 9),
     "gap600": lambda: _csr(([2] + [0] * 600) * 40 + [5] * 100, 500, 10),
     "gap5000": lambda: _csr(([37] + [0] * 5000 + [1]) * 9, 400, 11, runs=True),
