@@ -256,10 +256,10 @@ struct Publish
 };
 // enqueue the publication
 int publish(Workspace &ws, const Publish &p);
-// exclusive scan of n ints in place into out (n + 1 entries: out[n] = total),
-// then the publication, if any
+// exclusive scan of n ints into out (n + 1 entries, not overlapping in: out[n] =
+// total), then the publication, if any
 int scan_exclusive_int(Workspace &ws, const int *in, int *out, int n, const Publish *pub = nullptr);
-// exclusive scan of n ints into int64 offsets (n + 1 entries)
+// the same into int64 offsets
 int scan_exclusive_i64(Workspace &ws, const int *in, long long *out, int n,
                        const Publish *pub = nullptr);
 // adds the device error word to p; wait_published then syncs and returns

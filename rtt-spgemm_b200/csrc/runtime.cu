@@ -189,12 +189,21 @@ __device__ void publish_words(const Publish &p)
 
 __global__ void k_publish(Publish p) { publish_words(p); }
 
-// Scans of up to SCAN_ONE values in one CTA: one launch in place of the
-// library scan's two, its zero and the copies of its results.  With the
-// publication 256 values take 6 us, 4,096 (one round) 7.5 us, 12,500 12 to 17
-// us; the library's launches and a publication about 11 us.  (16 neighbouring
-// values per thread in one round took 16 us for the 12,500.)
-constexpr int SCAN_ONE = 16384, SCAN_THREADS = 1024, SCAN_PER = 4;
+// Short scans in one CTA: one launch in place of the library scan's two, its
+// zero and the publication, up to where those take as long.  Scan after scan on one
+// B200, one CTA against the library: 4-byte sums with a publication 8.3 and 12.7 us
+// at 4,096 values, 12.5 and 14.6 at 16,384, 14.5 and 14.6 at 20,000; without one
+// 6.3 and 9.5, 10.4 and 11.5 at 12,500, 12.2 and 11.1 at 16,384 (where fewer
+// launches still count: a limit of 12,800 there took the 256^2 5-point product from
+// 178 to 179 us); 8-byte sums with one 8.5 and 12.8, 14.5 and 14.4 at 10,000;
+// without 8.4 and 9.7 at 5,000, 10.3 and 9.5 at 6,000.  (16 neighbouring values per
+// thread in one round took 16 us for 12,500.)
+constexpr int SCAN_THREADS = 1024, SCAN_PER = 4;
+template <typename T>
+constexpr int scan_one_limit(bool publication)
+{
+    return sizeof(T) == 4 ? 16384 : publication ? 10240 : 5120;
+}
 template <typename T>
 __global__ void __launch_bounds__(SCAN_THREADS)
     k_scan_one(const int *__restrict__ in, T *__restrict__ out, int n, Publish p)
@@ -238,11 +247,11 @@ struct ToI64
     __host__ __device__ long long operator()(int v) const { return (long long)v; }
 };
 
-// n <= SCAN_ONE (or none): true when done
+// Short ones (or none): true when done
 template <typename T>
 bool scan_one(Workspace &ws, const int *in, T *out, int n, const Publish *pub)
 {
-    if (n > SCAN_ONE)
+    if (n > scan_one_limit<T>(pub != nullptr))
         return false;
     k_scan_one<T><<<1, SCAN_THREADS, 0, ws.stream>>>(in, out, std::max(n, 0),
                                                      pub != nullptr ? *pub : Publish());

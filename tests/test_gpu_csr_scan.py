@@ -163,3 +163,24 @@ def test_empty_product(empty, cfg):
         ctx.numeric_values(dev[0][4], dev[1][4], *out)
         assert not out[0].any()
     ctx.close()
+
+
+@pytest.mark.parametrize("tiles", [4096, 5120, 5121, 10240, 10241, 16384, 16385])
+def test_scan_lengths(tiles):
+    """Sums of as many tile rows and C tiles as one CTA scans, and one more: a
+    diagonal matrix, squared."""
+    m = 16 * tiles - 3
+    v = torch.rand(m, dtype=torch.float64, device=DEV)
+    i = torch.arange(m + 1, dtype=torch.int32, device=DEV)
+    a = (m, m, i, i[:m].contiguous(), v)
+    for wide in (False, True):
+        ctx = R.Context(0)
+        nnz = ctx.symbolic64(a) if wide else ctx.symbolic(a)[0]
+        assert nnz == m
+        out = (torch.empty(m + 1, dtype=torch.int64 if wide else torch.int32, device=DEV),
+               torch.empty(m, dtype=torch.int32, device=DEV),
+               torch.empty(m, dtype=torch.float64, device=DEV))
+        (ctx.numeric64 if wide else ctx.numeric)(*out)
+        assert torch.equal(out[0], i.to(out[0].dtype)) and torch.equal(out[1], i[:m])
+        assert torch.equal(out[2], v * v)
+        ctx.close()
