@@ -470,14 +470,6 @@ struct WinTask
 };
 static_assert(sizeof(WinTask) == 80, "task record layout");
 
-struct WinQueue
-{
-    int count;    // tasks written by the plan
-    int head;     // next task to take
-    int overflow; // some heavy tile row found no room and kept its own CTA
-    int next;     // next tile row for the persistent tile-row CTAs
-};
-
 constexpr int PLAN_WARPS = 8;
 // Products walked by one window task (about a millisecond of one CTA): tile
 // rows whose windows together walk fewer are not split.
@@ -538,7 +530,7 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32)
                const int *__restrict__ c_tile_nnz,
                const uint16_t *__restrict__ c_mask, const int *__restrict__ csr_rowptr,
                uint8_t *__restrict__ heavy, WinTask *__restrict__ tasks, int cap,
-               long long target, WinQueue *q, long long *counters)
+               long long target, TaskQueue *q, long long *counters)
 {
     const int lane = lane_id();
     const int I = blockIdx.x * PLAN_WARPS + (threadIdx.x >> 5);
@@ -752,7 +744,7 @@ __global__ void __launch_bounds__(F_THREADS, MIN_CTAS)
                    double *__restrict__ c_val, const int *__restrict__ csr_rowptr,
                    int *__restrict__ csr_col, double *__restrict__ csr_val, long long *counters,
                    int *err, const uint8_t *__restrict__ heavy, const WinTask *__restrict__ tasks,
-                   WinQueue *q, int *__restrict__ cursors)
+                   TaskQueue *q, int *__restrict__ cursors)
 {
     extern __shared__ __align__(128) unsigned char dyn[];
     FlatSmem<ACC> &S = *reinterpret_cast<FlatSmem<ACC> *>(dyn);
@@ -1095,7 +1087,7 @@ __global__ void __launch_bounds__(F_THREADS)
     k_numeric_glob(DevTiles A, DevTiles B, int tilem, long long nnzC,
                    const int *__restrict__ c_tile_col, const uint16_t *__restrict__ c_mask,
                    const int *__restrict__ csr_rowptr, int *__restrict__ csr_col,
-                   double *__restrict__ csr_val, const WinTask *__restrict__ tasks, WinQueue *q,
+                   double *__restrict__ csr_val, const WinTask *__restrict__ tasks, TaskQueue *q,
                    int cap, int tilen, int *__restrict__ slot_all, int *__restrict__ rel_all,
                    int *err)
 {
@@ -1272,7 +1264,7 @@ __global__ void __launch_bounds__(F_THREADS)
     k_numeric_glob2(DevTiles A, DevTiles B, int tilem, long long nnzC,
                     const int *__restrict__ c_tile_col, const uint16_t *__restrict__ c_mask,
                     const int *__restrict__ csr_rowptr, int *__restrict__ csr_col,
-                    double *__restrict__ csr_val, const WinTask *__restrict__ tasks, WinQueue *q,
+                    double *__restrict__ csr_val, const WinTask *__restrict__ tasks, TaskQueue *q,
                     int cap, int *err)
 {
     extern __shared__ __align__(16) unsigned char g2_raw[];
@@ -1469,7 +1461,7 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
     const int cap = (int)std::min<long long>(cap_ll, 1 << 26);
     RTT_CHECK(S.w_task.ensure(sizeof(WinTask) * (size_t)cap, s));
     RTT_CHECK(S.w_heavy.ensure((size_t)S.tilem + 16, s));
-    RTT_CHECK(S.w_queue.ensure(sizeof(WinQueue), s));
+    RTT_CHECK(S.w_queue.ensure(sizeof(TaskQueue), s));
     if (cfg.ev_begin != nullptr)
         RTT_CUDA(cudaEventRecord(cfg.ev_begin, s));
     const int *fused_rowptr = cfg.csr_col ? cfg.csr_rowptr : nullptr;
@@ -1499,7 +1491,7 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
     }
     if (split && !rowwin)
     {
-        RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(WinQueue), s));
+        RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(TaskQueue), s));
         auto plan = !glob                  ? k_win_plan<ACC_SMALL, 0>
                     : cfg.global_rows == 2 ? k_win_plan<ACC_SMALL, 2>
                                            : k_win_plan<ACC_SMALL, 1>;
@@ -1507,7 +1499,7 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
             S.tilem, S.m, A, B, S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(),
             S.c_tile_nnz.as<int>(),
             S.c_mask.as<uint16_t>(), fused_rowptr, S.w_heavy.as<uint8_t>(),
-            S.w_task.as<WinTask>(), cap, target, S.w_queue.as<WinQueue>(), cfg.counters);
+            S.w_task.as<WinTask>(), cap, target, S.w_queue.as<TaskQueue>(), cfg.counters);
         ws.launches++;
     }
     auto launch = [&](auto kern, int grid, cudaStream_t st, size_t smem, int *cursors) -> int {
@@ -1519,7 +1511,7 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
             cfg.write_tiles ? S.c_val.as<double>() : nullptr, fused_rowptr, cfg.csr_col,
             cfg.csr_val, cfg.counters, ws.err.as<int>(),
             split ? S.w_heavy.as<uint8_t>() : nullptr, S.w_task.as<WinTask>(),
-            S.w_queue.as<WinQueue>(), cursors);
+            S.w_queue.as<TaskQueue>(), cursors);
         ws.launches++;
         return RTT_OK;
     };
@@ -1553,7 +1545,7 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
             k_numeric_glob2<<<grid, F_THREADS, gsm, ws.side>>>(
                 A, B, S.tilem, S.nnz, S.c_tile_col.as<int>(), S.c_mask.as<uint16_t>(),
                 fused_rowptr, cfg.csr_col, cfg.csr_val, S.w_task.as<WinTask>(),
-                S.w_queue.as<WinQueue>(), cap, ws.err.as<int>());
+                S.w_queue.as<TaskQueue>(), cap, ws.err.as<int>());
         }
         else
         {
@@ -1566,7 +1558,7 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
             gk<<<grid, F_THREADS, 0, ws.side>>>(A, B, S.tilem, S.nnz, S.c_tile_col.as<int>(),
                                                 S.c_mask.as<uint16_t>(), fused_rowptr, cfg.csr_col,
                                                 cfg.csr_val, S.w_task.as<WinTask>(),
-                                                S.w_queue.as<WinQueue>(), cap, tilen,
+                                                S.w_queue.as<TaskQueue>(), cap, tilen,
                                                 S.g_slot.as<int>(), S.g_rel.as<int>(),
                                                 ws.err.as<int>());
         }
@@ -1627,7 +1619,7 @@ int numeric_flat_device(Workspace &ws, const DevTiles &A, const DevTiles &B, Sym
         RTT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, light, F_THREADS, smem));
         light_grid = std::max(1, std::min(per_sm * sms, S.tilem));
         if (!split)
-            RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(WinQueue), s));
+            RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(TaskQueue), s));
     }
     RTT_CHECK(launch(light, light_grid, s, smem, nullptr));
     if (split)

@@ -83,14 +83,6 @@ struct RowTask
     int t0, t1;     // one row's piece: C tiles [t0, t1); t0 < 0: whole rows
 };
 
-struct RowQueue
-{
-    int big, normal; // tasks written (pieces of long rows; groups of rows)
-    int head;        // next task to take, pieces first
-    int pad;         // (the tile-row kernel's queue of persistent CTAs)
-    int want;        // pieces asked for
-};
-
 // cut_tile[g]: first tile column of part g (g = CUTS: tilen).  The parts hold
 // about as many of B's entries each, from about WEIGHT_SAMPLES of them counted
 // per bin of tile columns (one bin per tile column up to WEIGHT_BINS): the
@@ -158,7 +150,7 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32)
                const int *__restrict__ c_tile_nnz, const int *__restrict__ csr_rowptr,
                const int *__restrict__ cut_tile, uint8_t *__restrict__ heavy,
                RowTask *__restrict__ big, int big_cap, RowTask *__restrict__ normal, int group,
-               long long target, RowQueue *q, long long *counters)
+               long long target, TaskQueue *q, long long *counters)
 {
     const int lane = lane_id();
     const int I = blockIdx.x * PLAN_WARPS + (threadIdx.x >> 5);
@@ -299,7 +291,7 @@ __global__ void __launch_bounds__(PREP_THREADS)
     k_row_prepare(int tilem, const int *__restrict__ c_tile_ptr,
                   const uint16_t *__restrict__ c_mask, const uint8_t *__restrict__ heavy,
                   uint16_t *__restrict__ maskt, DevTiles B, const int *__restrict__ cut_tile,
-                  const RowQueue *q, int *__restrict__ part)
+                  const TaskQueue *q, int *__restrict__ part)
 {
     const int I = blockIdx.x;
     if (I >= tilem)
@@ -377,7 +369,7 @@ __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
                      const int *__restrict__ c_tile_col, const uint16_t *__restrict__ maskt,
                      const int *__restrict__ csr_rowptr, int *__restrict__ csr_col,
                      double *__restrict__ csr_val, const RowTask *__restrict__ big,
-                     const RowTask *__restrict__ normal, RowQueue *q, int span,
+                     const RowTask *__restrict__ normal, TaskQueue *q, int span,
                      const int *__restrict__ part, const int *__restrict__ cut_tile, int2 *cursors,
                      int *err)
 {
@@ -770,7 +762,7 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     RTT_CHECK(S.r_mask.ensure(sizeof(uint16_t) * row_masks(S.numtile, S.tilem, 0, 0), s));
     RTT_CHECK(S.r_cut.ensure(sizeof(int) * (CUTS + 1), s));
     RTT_CHECK(S.r_cursor.ensure(sizeof(int2) * (size_t)grid * RW_WARPS * ROW_CURSORS, s));
-    RTT_CHECK(S.w_queue.ensure(sizeof(RowQueue), s));
+    RTT_CHECK(S.w_queue.ensure(sizeof(TaskQueue), s));
     // the table of B's parts where it is small enough and can be had
     const size_t part_bytes = sizeof(int) * (size_t)B.m * (CUTS + 1) + 16;
     bool table = part_bytes <= PART_BYTES_MAX;
@@ -782,7 +774,7 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
             return st;
     }
     int *part = table ? S.r_part.as<int>() : nullptr;
-    RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(RowQueue), s));
+    RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(TaskQueue), s));
     int *cut_tile = S.r_cut.as<int>();
     k_cut_tiles<<<1, CUT_THREADS, 0, s>>>(B, S.tilen, cut_tile);
     // a task per row when the groups would leave warps without work
@@ -794,10 +786,10 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
         S.tilem, S.m, A, B, S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(),
         S.c_tile_nnz.as<int>(), cfg.csr_rowptr, cut_tile, S.w_heavy.as<uint8_t>(),
         S.r_big.as<RowTask>(), big_cap, S.r_normal.as<RowTask>(), group,
-        target, S.w_queue.as<RowQueue>(), cfg.counters);
+        target, S.w_queue.as<TaskQueue>(), cfg.counters);
     k_row_prepare<<<S.tilem + (table ? 8 * sms : 0), PREP_THREADS, 0, s>>>(
         S.tilem, S.c_tile_ptr.as<int>(), S.c_mask.as<uint16_t>(), S.w_heavy.as<uint8_t>(),
-        S.r_mask.as<uint16_t>(), B, cut_tile, S.w_queue.as<RowQueue>(), part);
+        S.r_mask.as<uint16_t>(), B, cut_tile, S.w_queue.as<TaskQueue>(), part);
     ws.launches += 3;
     auto kern = table ? k_numeric_rowwin<EW, TW, true> : k_numeric_rowwin<EW, TW, false>;
     // on the side stream, beside the tile-row CTAs of the other tile rows
@@ -806,7 +798,7 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     kern<<<grid, RW_WARPS * 32, smem, ws.side>>>(
         A, B, S.nnz, S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(), S.r_mask.as<uint16_t>(),
         cfg.csr_rowptr, cfg.csr_col, cfg.csr_val, S.r_big.as<RowTask>(), S.r_normal.as<RowTask>(),
-        S.w_queue.as<RowQueue>(), span, part, cut_tile, S.r_cursor.as<int2>(), ws.err.as<int>());
+        S.w_queue.as<TaskQueue>(), span, part, cut_tile, S.r_cursor.as<int2>(), ws.err.as<int>());
     ws.launches++;
     RTT_CUDA(cudaEventRecord(ws.join_ev, ws.side));
     return RTT_OK;

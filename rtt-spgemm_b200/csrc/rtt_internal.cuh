@@ -77,6 +77,18 @@ __device__ __forceinline__ void tile_range(const DevTiles &T, int I, int &b, int
     e = T.tile_end != nullptr ? __ldg(T.tile_end + I) : __ldg(T.tile_ptr + I + 1);
 }
 
+// The numeric step's work queue in device memory (SymbolicOut::w_queue), cleared
+// for every product: one of window tasks or row tasks, beside tile rows.
+struct TaskQueue
+{
+    int count;       // window tasks written by the plan
+    int big, normal; // row tasks written (pieces of long rows; groups of rows)
+    int want;        // pieces asked for
+    int head;        // next task to take (pieces before groups)
+    int overflow;    // some heavy tile row found no room and kept its own CTA
+    int next;        // next tile row for the persistent tile-row CTAs
+};
+
 // C tile structure produced by the symbolic phase.
 struct DevCTiles
 {
@@ -247,8 +259,12 @@ struct Publish
     int *dst[MAX];
     int words[MAX];
     int count = 0;
+    bool full = false; // more than MAX were added: publishing fails
     void add(const void *from, int *to, int n)
     {
+        full = full || count == MAX;
+        if (full)
+            return;
         src[count] = static_cast<const int *>(from);
         dst[count] = to;
         words[count++] = n;

@@ -251,7 +251,7 @@ struct ToI64
 template <typename T>
 bool scan_one(Workspace &ws, const int *in, T *out, int n, const Publish *pub)
 {
-    if (n > scan_one_limit<T>(pub != nullptr))
+    if (n > scan_one_limit<T>(pub != nullptr) || (pub != nullptr && pub->full))
         return false;
     k_scan_one<T><<<1, SCAN_THREADS, 0, ws.stream>>>(in, out, std::max(n, 0),
                                                      pub != nullptr ? *pub : Publish());
@@ -262,6 +262,8 @@ bool scan_one(Workspace &ws, const int *in, T *out, int n, const Publish *pub)
 
 int publish(Workspace &ws, const Publish &p)
 {
+    if (p.full)
+        return fail(RTT_ERR_STATE, "too many words to publish");
     k_publish<<<1, 32, 0, ws.stream>>>(p);
     ws.launches++;
     return RTT_OK;
