@@ -58,7 +58,10 @@ CASES = {
     "front": lambda: _csr([0] * 30000 + [7] * 100, 300, 12),
     "back": lambda: _csr([8] * 64 + [0] * 30000, 300, 13),     # 512 entries: the last word is full
     "middle": lambda: _csr([4] * 100 + [0] * 30000 + [9] * 100, 300, 14),
-    "many": lambda: _csr([24] * 120000, 5000, 7, runs=True),    # several blocks to a warp
+    # two blocks to a warp (more than 2 * 1200 CTAs of 8 warps' blocks): runs over
+    # their ends, rows longer than both, empty rows among them
+    "many": lambda: _csr([24] * 100000 + [5000] + [0] * 9000 + [37] * 3000 + [24] * 105000 + [3],
+                         9000, 7, runs=True),
 }
 
 
@@ -67,6 +70,7 @@ CASES = {
 @pytest.mark.parametrize("case", list(CASES))
 def test_scan(case, shift, cfg, orc):
     a = CASES[case]()
+    assert case != "many" or a.nnz > 2 * 1200 * 8 * 256
     b = _csr([2] * a.n, 200, 8)
     if cfg:  # the segments that step 2 reads are B's
         filled = np.flatnonzero(np.diff(a.rowptr))

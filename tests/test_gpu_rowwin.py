@@ -33,7 +33,7 @@ def _pick(m, per, k, seed):
 
 
 def _entries():
-    # C rows of 511 .. 1025 entries (windows of 512 or 1024), two B rows each
+    # C rows of 511 .. 1025 entries (windows of 512), two B rows each
     sizes = [511, 512, 513, 1023, 1024, 1025, 600, 1] * 4
     b = _rows([np.arange(7 * i, 7 * i + s) for i, s in enumerate(sizes)] +
               [np.arange(7 * i, 7 * i + s, 3) for i, s in enumerate(sizes)], 1300, 1)
@@ -41,7 +41,7 @@ def _entries():
 
 
 def _tiles():
-    # C rows of 255 .. 513 tiles with one entry each (windows of 256 or 512)
+    # C rows of 255 .. 513 tiles with one entry each (windows of 256)
     sizes = [255, 256, 257, 511, 512, 513, 8, 7] * 4
     b = _rows([16 * np.arange(i, i + s) + i % 16 for i, s in enumerate(sizes)], 16 * 700, 3)
     return _rows([[i] for i in range(32)], 32, 4), b
@@ -71,7 +71,34 @@ def _hub():
     return a, a
 
 
-CASES = {"entries": _entries, "tiles": _tiles, "spans": _spans, "long": _long, "hub": _hub}
+def _entries_long():
+    # more than 1,024 entries a row: windows of 1024, rows of one and two of them
+    sizes = [1023, 1024, 1025, 2047, 2048, 2049, 600, 1] * 4
+    b = _rows([np.arange(7 * i, 7 * i + s) for i, s in enumerate(sizes)] +
+              [np.arange(7 * i, 7 * i + s, 3) for i, s in enumerate(sizes)], 2400, 14)
+    return _rows([[i, i + 32] for i in range(32)], 64, 15), b
+
+
+def _tiles_long():
+    # the same windows, of 512 tiles: rows of 511 .. 1025 tiles with one entry
+    # each between rows of 3,000 entries
+    sizes = [511, 512, 513, 1023, 1024, 1025, 8, 7] * 4
+    b = _rows([16 * np.arange(i, i + s) + i % 16 for i, s in enumerate(sizes)] +
+              [np.arange(9 * i, 9 * i + 3000) for i in range(32)], 16 * 1100, 16)
+    return _rows([[i // 2 + 32 * (i % 2)] for i in range(64)], 64, 17), b
+
+
+def _groups(m, n):
+    # rows of little work, in tasks of neighbours: two from 9,472 rows (64 an SM),
+    # four from 37,888
+    return _pick(m, 3, 48, 18), _pick(48, 40, n, 19)
+
+
+CASES = {"entries": _entries, "tiles": _tiles, "spans": _spans, "long": _long, "hub": _hub,
+         "entries_long": _entries_long, "tiles_long": _tiles_long,
+         "groups2": lambda: _groups(9473, 20000),
+         # (and columns further apart than one column index spans)
+         "groups4": lambda: _groups(38001, 16 * 300000)}
 
 
 def _run(a, b, cfg):
@@ -95,9 +122,13 @@ def test_row_windows(case, orc):
     for target in (0, 1, 1 << 16):
         got, st = _run(a, b, dict(split_target=target))
         assert st["split_windows"] > 0 and st["nnz_cub"] == st0["nnz_cub"]
+        assert target or not case.startswith("groups") or \
+            st["split_windows"] == -(-a.m // int(case[6:]))
         for g, w in zip(got, want):
             assert np.array_equal(g.view(np.int32), w.view(np.int32)), (case, target)
     assert_csr_close(*want, *orc.spgemm_csr(a, b), case)
+    if case.endswith("_long"):
+        assert want[1].size > 1024 * a.m
 
 
 def test_last_columns(orc):
