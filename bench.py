@@ -105,14 +105,33 @@ def load_peaks() -> dict:
     return {"hbm_gbs": 6650.0, "source": "fallback"}
 
 
-def load_traffic(workload: str):
+def load_traffic(workload: str, kernel: str):
+    """DRAM bytes of one launch of the kernel on the workload, where they were
+    measured (profiles/numeric_traffic.json), else None."""
     p = ROOT / "profiles" / "numeric_traffic.json"
     if p.exists():
-        d = json.loads(p.read_text())
-        e = d.get(workload)
-        if e:
-            return e.get("dram_bytes_per_launch")
+        e = json.loads(p.read_text()).get(workload)
+        if e and e["kernel"].split("<")[0] == kernel:
+            return e["dram_bytes_per_launch"]
     return None
+
+
+def numeric_kernel(cfg: dict, stats: dict, b_increasing: bool) -> str:
+    """The kernel that does the numeric step's products under this configuration
+    (a context's config and the product's stats; b_increasing: B's rows have
+    strictly increasing columns), for the tile rows that are most of the work."""
+    if cfg["leaf_dmma"]:
+        return "k_numeric_leaf"
+    if cfg["b_staging"] or (cfg["dmma_pair_cutoff"] > 0 and stats["dmma_pairs"]):
+        return "k_numeric_rows"
+    csr_alone = cfg["fused_csr_output"] and not cfg["keep_tiles"] and b_increasing
+    if not csr_alone:
+        return "k_numeric_flat"
+    if stats["split_windows"] > 0:  # heavy tile rows in tasks
+        return {0: "k_numeric_rowwin", 1: "k_numeric_glob", 2: "k_numeric_glob2"}[cfg["global_rows"]]
+    if cfg["segment_walk"] or cfg["persistent_rows"] or cfg["split_target"] < 0:
+        return "k_numeric_flat"
+    return "k_numeric_tilerow"
 
 
 class ClockSampler:
@@ -763,8 +782,11 @@ def run_ours(args) -> None:
     abytes = alg_bytes(A.m, A.nnz, A.nnz, nnz_c)
     num_ms = statistics.mean(stage["numeric_kernel_ms"])
     achieved = abytes / (num_ms * 1e-3) / 1e9
-    traffic = (None if args.staging or args.unfused or args.leaf_dmma
-               else load_traffic(args.workload))
+    rows = np.repeat(np.arange(A.m), np.diff(A.rowptr))
+    # (A^T's columns are A's rows: repeated where A repeats a column)
+    increasing = not np.any((np.diff(rows) == 0) & (np.diff(A.col) <= 0))
+    kernel = numeric_kernel(ctx.config, st, increasing)
+    traffic = load_traffic(args.workload, kernel)
 
     # repeated product with the same structure and new values (values-only
     # update, rtt_spgemm_numeric_values): no csr2tile counting, no symbolic
@@ -889,11 +911,10 @@ def run_ours(args) -> None:
                    "dmma_pair_cutoff": args.dmma_cutoff, "fused_tile2csr": not args.unfused,
                    "b_staging": bool(args.staging)},
         "roofline": {"bound": "hbm",
-                     "kernel": ("k_numeric_rows (TMA-staged numeric + fused tile2csr)" if args.staging
-                                else "k_numeric_leaf (FP64 DMMA from hybrid leaves; the leaf "
-                                     "build and tile2csr outside the kernel time)" if args.leaf_dmma
-                                else ("k_numeric_rowwin" if "rmat" in args.workload
-                                      else "k_numeric_tilerow") + " (numeric + fused tile2csr)"),
+                     "kernel": kernel + (" (FP64 DMMA from hybrid leaves; the leaf build and "
+                                         "tile2csr outside the kernel time)" if args.leaf_dmma
+                                         else " (numeric)" if args.unfused
+                                         else " (numeric + fused tile2csr)"),
                      "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
                      "peak_source": peaks["source"], "kernel_ms": num_ms,
