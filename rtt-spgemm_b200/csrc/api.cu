@@ -839,17 +839,6 @@ int numeric_args_ok(rtt_context c, const int *c_row_ptr, const int *c_col_idx,
 
 } // namespace
 
-// Symbolic step 2 reads A's entries from its CSR rows where it walks B's row
-// segments, else from A's tiles: a B whose rows list no segments (tile columns
-// that decrease) needs them also where A's own rows do not.  (A's and B's rows
-// have been checked.)
-int payload_without_segments(rtt_context c)
-{
-    if (c->B.has_segments || c->B.m == 0 || c->A.payload)
-        return RTT_OK;
-    return map_device_error(csr2tile_payload(c->ws, c->a_rp, c->a_ci, c->a_va, c->A, true));
-}
-
 // The device views that the symbolic and numeric steps take.
 void operand_views(rtt_context c, DevTiles &dA, DevTiles &dB)
 {
@@ -935,8 +924,6 @@ int prepare_operands(rtt_context c, const rtt_csr_view *A, const rtt_csr_view *B
             c->b_nnz = B->nnz;
         }
         c->b_dups = c->B.dup_cols;
-        if (!defer)
-            RTT_CHECK(payload_without_segments(c));
     }
     operand_views(c, dA, dB);
     return RTT_OK;
@@ -974,8 +961,6 @@ int operands_and_step1(rtt_context c, const rtt_csr_view *A, const rtt_csr_view 
             RTT_CHECK(map_device_error(csr2tile_payload(ws, c->a_rp, c->a_ci, c->a_va, c->A, true)));
         if (wait_b && c->B.generic)
             RTT_CHECK(map_device_error(csr2tile_payload(ws, c->b_rp, c->b_ci, c->b_va, c->B, true)));
-        if (!c->b_alias)
-            RTT_CHECK(payload_without_segments(c));
         operand_views(c, dA, dB);
         return map_device_error(symbolic_step1(ws, dA, dB, c->S));
     }
@@ -1798,7 +1783,6 @@ int rtt_spgemm_update_b(rtt_context c, const rtt_csr_view *B, const int *row_new
     c->b_va = b.values;
     c->b_nnz = b.nnz;
     c->b_dups = c->B.dup_cols;
-    RTT_CHECK(payload_without_segments(c));
     DevTiles dA, dB;
     operand_views(c, dA, dB);
     RTT_CHECK(map_device_error(symbolic_device(ws, dA, dB, c->S, !c->b_dups)));

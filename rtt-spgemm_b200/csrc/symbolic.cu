@@ -682,7 +682,8 @@ __global__ void __launch_bounds__(SD_THREADS, 4)
 // single-window walk registers and issue slots).  NW warps per CTA: 8 for
 // the tile rows in order (a heavy one is skipped when heavy[] marks it), or
 // S2_HEAVY_WARPS for the heavy rows of list[] (all warps share the walk).
-template <bool NARROW, int NW, bool SEGS, bool WIDE = false>
+// ACSR: A's entries from its CSR rows (always with SEGS), else from its tiles.
+template <bool NARROW, int NW, bool SEGS, bool WIDE = false, bool ACSR = SEGS>
 __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW == S2_SEG_WARPS ? 10 : NW == S2_WIDE_WARPS ? 2 : 1)
     k_sym_rows(DevTiles A, DevTiles B, const int *__restrict__ c_tile_ptr,
                int *__restrict__ c_tile_col, int *__restrict__ c_tile_row,
@@ -745,7 +746,7 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
             atomicMax(&S.hi, hi);
         }
     }
-    if (SEGS && tid <= nrows)
+    if (ACSR && tid <= nrows)
         S.rp[tid] = __ldg(A.csr_rowptr + I * TD + tid);
     __syncthreads();
     const int lo = S.lo, hi = S.hi;
@@ -947,6 +948,69 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
             // seven wait, so all warps share the tile row's A entries (the
             // masks combine by OR, in any order); warp w takes every
             // NW-th A tile, so short tile rows are shared too
+            auto batch = [&](int n, int fs, int len, int sh, int rb) {
+                int nbat = n;
+                if (NARROW)
+                {
+                    // B rows with nothing in this window leave the list
+                    const unsigned live = __ballot_sync(FULL, len > 0);
+                    if (len > 0)
+                        ent[__popc(live & ((1u << lane) - 1u))] = make_int4(fs, len, sh, rb);
+                    nbat = __popc(live);
+                }
+                else
+                    ent[lane] = make_int4(fs, len, sh, rb);
+                __syncwarp();
+                auto mark = [&](int col, int sh, int rb) {
+                    const int d = (col >> 4) - w;
+                    if ((unsigned)d < (unsigned)wlen)
+                    {
+                        const int sl = S.slot[d];
+                        if (sl != NONE)
+                            atomicOr(&MW[rb + sl], (0x8000u >> (col & 15)) << sh);
+                    }
+                };
+                for (int j = 0; j < nbat; j += 2)
+                {
+                    int4 e0 = ent[j], e1 = ent[(j + 1) & 31];
+                    if (j + 1 >= nbat)
+                        e1.y = 0;
+                    const int c0 = lane < e0.y ? __ldg(B.csr_col + e0.x + lane) : -1;
+                    const int c1 = lane < e1.y ? __ldg(B.csr_col + e1.x + lane) : -1;
+                    if (c0 >= 0)
+                        mark(c0, e0.z, e0.w);
+                    if (e0.y > 32) // rows longer than a warp (uniform branch)
+                        for (int f = 32 + lane; f < e0.y; f += 32)
+                            mark(__ldg(B.csr_col + e0.x + f), e0.z, e0.w);
+                    if (c1 >= 0)
+                        mark(c1, e1.z, e1.w);
+                    if (e1.y > 32)
+                        for (int f = 32 + lane; f < e1.y; f += 32)
+                            mark(__ldg(B.csr_col + e1.x + f), e1.z, e1.w);
+                }
+                __syncwarp(); // the next batch overwrites this warp's list
+            };
+            if constexpr (ACSR)
+                for (int q0 = S.rp[0] + warp * 32; q0 < S.rp[nrows]; q0 += NW * 32)
+                {
+                    const int e = q0 + lane;
+                    int fs = 0, len = 0, r = 0;
+                    if (e < S.rp[nrows])
+                    {
+#pragma unroll
+                        for (int h = 8; h > 0; h >>= 1)
+                            if (r + h < nrows && S.rp[r + h] <= e)
+                                r += h;
+                        const int k = __ldg(A.csr_col + e);
+                        if ((unsigned)k < (unsigned)B.m)
+                        {
+                            fs = min(max(__ldg(B.csr_rowptr + k), 0), B.nnz);
+                            len = min(max(__ldg(B.csr_rowptr + k + 1), fs), B.nnz) - fs;
+                        }
+                    }
+                    batch(min(32, S.rp[nrows] - q0), fs, len, (r & 1) * 16, (r >> 1) * STRIDE);
+                }
+            else
             for (int t0 = a0; t0 < a1; t0 += NW * 32)
             {
                 const int t = t0 + lane * NW + warp;
@@ -991,46 +1055,7 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
                             rb = (r >> 1) * STRIDE;
                         }
                     }
-                    int nbat = min(32, total - q0);
-                    if (NARROW)
-                    {
-                        // B rows with nothing in this window leave the list
-                        const unsigned live = __ballot_sync(FULL, len > 0);
-                        if (len > 0)
-                            ent[__popc(live & ((1u << lane) - 1u))] = make_int4(fs, len, sh, rb);
-                        nbat = __popc(live);
-                    }
-                    else
-                        ent[lane] = make_int4(fs, len, sh, rb);
-                    __syncwarp();
-                    auto mark = [&](int col, int sh, int rb) {
-                        const int d = (col >> 4) - w;
-                        if ((unsigned)d < (unsigned)wlen)
-                        {
-                            const int sl = S.slot[d];
-                            if (sl != NONE)
-                                atomicOr(&MW[rb + sl], (0x8000u >> (col & 15)) << sh);
-                        }
-                    };
-                    for (int j = 0; j < nbat; j += 2)
-                    {
-                        int4 e0 = ent[j], e1 = ent[(j + 1) & 31];
-                        if (j + 1 >= nbat)
-                            e1.y = 0;
-                        const int c0 = lane < e0.y ? __ldg(B.csr_col + e0.x + lane) : -1;
-                        const int c1 = lane < e1.y ? __ldg(B.csr_col + e1.x + lane) : -1;
-                        if (c0 >= 0)
-                            mark(c0, e0.z, e0.w);
-                        if (e0.y > 32) // rows longer than a warp (uniform branch)
-                            for (int f = 32 + lane; f < e0.y; f += 32)
-                                mark(__ldg(B.csr_col + e0.x + f), e0.z, e0.w);
-                        if (c1 >= 0)
-                            mark(c1, e1.z, e1.w);
-                        if (e1.y > 32)
-                            for (int f = 32 + lane; f < e1.y; f += 32)
-                                mark(__ldg(B.csr_col + e1.x + f), e1.z, e1.w);
-                    }
-                    __syncwarp(); // the next batch overwrites this warp's list
+                    batch(min(32, total - q0), fs, len, sh, rb);
                 }
             }
             __syncthreads(); // every warp's rows are complete
@@ -1038,6 +1063,69 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
         else if (NW == S2_WARPS && r0 < nrows)
         {
             // one window: warp-private walk over the warp's own A entries
+            auto batch = [&](int n, int fs, int len, int sh) {
+                int nbat = n;
+                if (NARROW)
+                {
+                    // B rows with nothing in this window leave the list
+                    const unsigned live = __ballot_sync(FULL, len > 0);
+                    if (len > 0)
+                        ent[__popc(live & ((1u << lane) - 1u))] = make_int4(fs, len, sh, 0);
+                    nbat = __popc(live);
+                }
+                else
+                    ent[lane] = make_int4(fs, len, sh, 0);
+                __syncwarp();
+                // one column of B row k into the mask of row r's C tile
+                auto mark = [&](int col, int sh) {
+                    const int d = (col >> 4) - w;
+                    if ((unsigned)d < (unsigned)wlen)
+                    {
+                        const int sl = S.slot[d];
+                        if (sl != NONE)
+                            atomicOr(&mw[sl], (0x8000u >> (col & 15)) << sh);
+                    }
+                };
+                for (int j = 0; j < nbat; j += 2)
+                {
+                    int4 e0 = ent[j], e1 = ent[(j + 1) & 31];
+                    if (j + 1 >= nbat)
+                        e1.y = 0;
+                    const int c0 = lane < e0.y ? __ldg(B.csr_col + e0.x + lane) : -1;
+                    const int c1 = lane < e1.y ? __ldg(B.csr_col + e1.x + lane) : -1;
+                    if (c0 >= 0)
+                        mark(c0, e0.z);
+                    if (e0.y > 32) // rows longer than a warp (uniform branch)
+                        for (int f = 32 + lane; f < e0.y; f += 32)
+                            mark(__ldg(B.csr_col + e0.x + f), e0.z);
+                    if (c1 >= 0)
+                        mark(c1, e1.z);
+                    if (e1.y > 32)
+                        for (int f = 32 + lane; f < e1.y; f += 32)
+                            mark(__ldg(B.csr_col + e1.x + f), e1.z);
+                }
+                __syncwarp(); // the next batch overwrites this warp's list
+            };
+            if constexpr (ACSR)
+            {
+                const int em = S.rp[min(r1, nrows)], ee = S.rp[min(r0 + 2, nrows)];
+                for (int q0 = S.rp[r0]; q0 < ee; q0 += 32)
+                {
+                    const int e = q0 + lane;
+                    int fs = 0, len = 0;
+                    if (e < ee)
+                    {
+                        const int k = __ldg(A.csr_col + e);
+                        if ((unsigned)k < (unsigned)B.m)
+                        {
+                            fs = min(max(__ldg(B.csr_rowptr + k), 0), B.nnz);
+                            len = min(max(__ldg(B.csr_rowptr + k + 1), fs), B.nnz) - fs;
+                        }
+                    }
+                    batch(min(32, ee - q0), fs, len, e < em ? 0 : 16);
+                }
+            }
+            else
             for (int t0 = a0; t0 < a1; t0 += 32)
             {
                 const int t = t0 + lane;
@@ -1088,47 +1176,7 @@ __global__ void __launch_bounds__(NW * 32, NW == S2_WARPS ? (WIDE ? 2 : 5) : NW 
                             fs = sb;
                         }
                     }
-                    int nbat = min(32, total - q0);
-                    if (NARROW)
-                    {
-                        // B rows with nothing in this window leave the list
-                        const unsigned live = __ballot_sync(FULL, len > 0);
-                        if (len > 0)
-                            ent[__popc(live & ((1u << lane) - 1u))] = make_int4(fs, len, sh, 0);
-                        nbat = __popc(live);
-                    }
-                    else
-                        ent[lane] = make_int4(fs, len, sh, 0);
-                    __syncwarp();
-                    // one column of B row k into the mask of row r's C tile
-                    auto mark = [&](int col, int sh) {
-                        const int d = (col >> 4) - w;
-                        if ((unsigned)d < (unsigned)wlen)
-                        {
-                            const int sl = S.slot[d];
-                            if (sl != NONE)
-                                atomicOr(&mw[sl], (0x8000u >> (col & 15)) << sh);
-                        }
-                    };
-                    for (int j = 0; j < nbat; j += 2)
-                    {
-                        int4 e0 = ent[j], e1 = ent[(j + 1) & 31];
-                        if (j + 1 >= nbat)
-                            e1.y = 0;
-                        const int c0 = lane < e0.y ? __ldg(B.csr_col + e0.x + lane) : -1;
-                        const int c1 = lane < e1.y ? __ldg(B.csr_col + e1.x + lane) : -1;
-                        if (c0 >= 0)
-                            mark(c0, e0.z);
-                        if (e0.y > 32) // rows longer than a warp (uniform branch)
-                            for (int f = 32 + lane; f < e0.y; f += 32)
-                                mark(__ldg(B.csr_col + e0.x + f), e0.z);
-                        if (c1 >= 0)
-                            mark(c1, e1.z);
-                        if (e1.y > 32)
-                            for (int f = 32 + lane; f < e1.y; f += 32)
-                                mark(__ldg(B.csr_col + e1.x + f), e1.z);
-                    }
-                    __syncwarp(); // the next batch overwrites this warp's list
+                    batch(min(32, total - q0), fs, len, sh);
                 }
             }
         }
@@ -1348,8 +1396,8 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
     RTT_CHECK(S.c_tr_nnz.ensure(sizeof(int) * (size_t)(tilem + 1), s));
     RTT_CHECK(S.tile_cnt.ensure(sizeof(int) * (nt + 1), s));
     // step 2 from B's row segments when they and A's CSR rows are at hand
-    const bool segs = B.seg_ptr != nullptr && B.seg != nullptr && A.csr_rowptr != nullptr &&
-                      A.csr_col != nullptr;
+    const bool acsr = A.csr_rowptr != nullptr && A.csr_col != nullptr;
+    const bool segs = B.seg_ptr != nullptr && B.seg != nullptr && acsr;
     if (tilem > 0)
     {
         auto go = [&](auto kern, int grid, int threads, size_t smem, cudaStream_t st,
@@ -1394,6 +1442,7 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
         if (n_heavy > 0 && S.sym_window_slots >= 0)
         {
             auto hk = segs ? k_sym_rows<false, S2_HEAVY_WARPS, true, true>
+                      : acsr ? k_sym_rows<false, S2_HEAVY_WARPS, false, true, true>
                            : b_sorted ? k_sym_rows<true, S2_HEAVY_WARPS, false, true>
                                       : k_sym_rows<false, S2_HEAVY_WARPS, false, true>;
             RTT_CHECK(go(hk, n_heavy, S2_HEAVY_WARPS * 32, segs ? smem2_bytes<S2_HEAVY_WARPS, true, true>(wstride)
@@ -1403,6 +1452,7 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
         else if (n_heavy > 0)
         {
             auto hk = segs ? k_sym_rows<false, S2_HEAVY_WARPS, true>
+                      : acsr ? k_sym_rows<false, S2_HEAVY_WARPS, false, false, true>
                            : b_sorted ? k_sym_rows<true, S2_HEAVY_WARPS, false>
                                       : k_sym_rows<false, S2_HEAVY_WARPS, false>;
             RTT_CHECK(go(hk, n_heavy, S2_HEAVY_WARPS * 32,
@@ -1418,8 +1468,9 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
                              S2_WIDE_WARPS * 32, smem2_bytes<S2_WIDE_WARPS, true, true>(wstride),
                              ws.side, nullptr, S.s2_wlist.as<int>(), wslots));
             else
-                RTT_CHECK(go(b_sorted ? k_sym_rows<true, S2_WARPS, false, true>
-                                      : k_sym_rows<false, S2_WARPS, false, true>,
+                RTT_CHECK(go(acsr ? k_sym_rows<false, S2_WARPS, false, true, true>
+                             : b_sorted ? k_sym_rows<true, S2_WARPS, false, true>
+                                        : k_sym_rows<false, S2_WARPS, false, true>,
                              n_wide, S2_THREADS, smem2_bytes<S2_WARPS, true, false>(wstride),
                              ws.side, nullptr, S.s2_wlist.as<int>(), wslots));
         }
@@ -1435,6 +1486,7 @@ int symbolic_step2(Workspace &ws, const DevTiles &A, const DevTiles &B, Symbolic
         else
         {
             auto kern = segs ? k_sym_rows<false, S2_WARPS, true>
+                        : acsr ? k_sym_rows<false, S2_WARPS, false, false, true>
                              : b_sorted && sym_multi ? k_sym_rows<true, S2_WARPS, false>
                                                      : k_sym_rows<false, S2_WARPS, false>;
             RTT_CHECK(go(kern, tilem, S2_THREADS,

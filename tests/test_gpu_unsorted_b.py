@@ -1,6 +1,5 @@
 """C = A * B where A's rows are sorted and B's are not: B then lists no row
-segments, and symbolic step 2 walks A's tiles, which a sorted A keeps only for
-such a B.  One and several windows per tile row, hub rows, the 64-bit products
+segments, and symbolic step 2 walks B's rows for A's entries.  One and several windows per tile row, hub rows, the 64-bit products
 in chunks, batches, another B for the same A, and new values."""
 from __future__ import annotations
 
@@ -109,4 +108,22 @@ def test_batched(orc):
     As, Bs = [_dev(a) for a, _ in hosts], [_dev(b) for _, b in hosts]
     for (a, b), c in zip(hosts, R.spgemm_batched(ctx, As, Bs)):
         _close(c, a, b, orc, "batched")
+    ctx.close()
+
+
+@pytest.mark.parametrize("n", [40, 60000])
+def test_tiles_of_repeated_columns(n, orc):
+    """Rows that are unsorted and repeat columns until a tile holds more than 255
+    entries, which a tile's byte offsets cannot count: one window, and several."""
+    rng = np.random.default_rng(20)
+    a_cols = [np.concatenate([rng.integers(0, 16, 40), rng.integers(0, 300, 5)]) for _ in range(50)]
+    rp = np.arange(51, dtype=np.int32) * 45
+    a = G.CSR(50, 300, rp, np.concatenate(a_cols).astype(np.int32), rng.uniform(-1, 1, 50 * 45))
+    b = _shuffled(G.random_csr(300, n, min(0.2, 1200 / n), seed=21), 22)
+    ctx = R.Context(0)
+    dev = (_dev(a), _dev(b))
+    nnz, _ = ctx.symbolic(*dev)
+    out = _out(50, nnz)
+    ctx.numeric(*out)
+    _close(out, a, b, orc, "repeated columns")
     ctx.close()
