@@ -94,6 +94,7 @@ struct rtt_context_s
     rtt::GraphSlot graph[4]; // numeric, values-only, batched, batched values-only
     cudaStream_t cap_stream = nullptr; // capture stream (never the legacy one)
     int cut_cached = -1; // effective DMMA cutoff of the current tiles (-1: unknown)
+    bool tiles_count = true, count_cached = true; // the tiles' byte offsets hold
     // 64-bit products: step-1 counts, per-row counts of C, its int64 row
     // pointer, a chunk's local row pointer; chunks of A's tile rows
     rtt::DevBuf w_cnt, w_rowcnt, w_rowptr, w_local;
@@ -573,18 +574,21 @@ int upload_tiles(rtt_context c, const SMatrix *M, bool col_major, TileBufs &T)
 }
 
 // The DMMA variant of the numeric kernel reserves extra shared memory; use it
-// only when some tile pair can reach the configured cutoff.
+// only when some tile pair can reach the configured cutoff.  It and the staged
+// kernel read the tiles, whose row offsets are bytes: not where columns repeat
+// until a tile holds more than 255 entries.
 int effective_cutoff(rtt_context c, const DevTiles &A, const DevTiles &B, int *cutoff)
 {
-    *cutoff = c->cfg.dmma_pair_cutoff;
-    if (*cutoff <= 0 || !A.tile_nnz || !B.tile_nnz)
-    {
-        *cutoff = 0;
+    const bool tiles = A.tile_nnz != nullptr && B.tile_nnz != nullptr;
+    const bool repeats = c->A.dup_cols || c->b_dups;
+    *cutoff = tiles ? std::max(0, c->cfg.dmma_pair_cutoff) : 0;
+    c->tiles_count = true;
+    if (*cutoff == 0 && !(tiles && repeats && c->cfg.b_staging != 0))
         return RTT_OK;
-    }
     if (c->cut_cached >= 0)
     {
         *cutoff = c->cut_cached;
+        c->tiles_count = c->count_cached;
         return RTT_OK;
     }
     RTT_CHECK(c->counters.ensure(sizeof(long long) * 4, c->ws.stream));
@@ -595,7 +599,10 @@ int effective_cutoff(rtt_context c, const DevTiles &A, const DevTiles &B, int *c
                              cudaMemcpyDeviceToHost, c->ws.stream));
     RTT_CUDA(cudaStreamSynchronize(c->ws.stream));
     c->ws.syncs++;
-    if ((long long)c->ws.h_scalars[10] * c->ws.h_scalars[11] < (long long)*cutoff)
+    c->tiles_count = !repeats || std::max(c->ws.h_scalars[10], c->ws.h_scalars[11]) <= 255;
+    c->count_cached = c->tiles_count;
+    if ((long long)c->ws.h_scalars[10] * c->ws.h_scalars[11] < (long long)*cutoff ||
+        !c->tiles_count)
         *cutoff = 0;
     c->cut_cached = *cutoff; // tile sizes change only with a new symbolic
     return RTT_OK;
@@ -629,7 +636,7 @@ void numeric_key(rtt_context c, std::vector<long long> &k)
     for (long long v : {as_key(c->b_rp), as_key(c->b_ci), as_key(c->b_va), c->b_nnz,
                         (long long)c->b_dups, (long long)c->b_alias, (long long)c->op_aat,
                         as_key(c->a_rp), as_key(c->a_ci), as_key(c->a_va),
-                        (long long)c->cut_cached,
+                        (long long)c->cut_cached, (long long)c->tiles_count,
                         (long long)c->bat_active, (long long)c->bat_count,
                         (long long)c->bat_rows})
         k.push_back(v);
@@ -755,7 +762,7 @@ int numeric_enqueue(rtt_context c, int *c_row_ptr, int *c_col_idx, double *c_val
     nc.dmma_pair_cutoff = cutoff;
     nc.counters = c->counters.as<long long>();
     // TMA staging reads the tile arrays: only when they were built
-    nc.b_staging = c->cfg.b_staging != 0 && c->A.payload && TB.payload;
+    nc.b_staging = c->cfg.b_staging != 0 && c->A.payload && TB.payload && c->tiles_count;
     nc.split_target = c->cfg.split_target;
     if (c->cfg.stage_timing)
     {

@@ -111,19 +111,29 @@ def test_batched(orc):
     ctx.close()
 
 
+@pytest.mark.parametrize("cfg", [{}, dict(b_staging=1), dict(dmma_pair_cutoff=1)],
+                         ids=lambda c: "_".join(c) or "default")
+@pytest.mark.parametrize("which", ["A", "A sorted", "B"])
 @pytest.mark.parametrize("n", [40, 60000])
-def test_tiles_of_repeated_columns(n, orc):
-    """Rows that are unsorted and repeat columns until a tile holds more than 255
-    entries, which a tile's byte offsets cannot count: one window, and several."""
+def test_tiles_of_repeated_columns(n, which, cfg, orc):
+    """Rows that repeat columns until a tile holds more than 255 entries, which a
+    tile's byte offsets cannot count: unsorted or not, one window and several."""
     rng = np.random.default_rng(20)
     a_cols = [np.concatenate([rng.integers(0, 16, 40), rng.integers(0, 300, 5)]) for _ in range(50)]
     rp = np.arange(51, dtype=np.int32) * 45
     a = G.CSR(50, 300, rp, np.concatenate(a_cols).astype(np.int32), rng.uniform(-1, 1, 50 * 45))
     b = _shuffled(G.random_csr(300, n, min(0.2, 1200 / n), seed=21), 22)
-    ctx = R.Context(0)
+    if which == "A sorted":
+        order = np.lexsort((a.col, np.repeat(np.arange(50), 45)))
+        a = G.CSR(50, 300, rp, a.col[order].copy(), a.val[order].copy())
+    elif which == "B":
+        a, b = G.random_csr(70, 50, 0.2, seed=23), a
+    ctx = R.Context(0, cfg)
     dev = (_dev(a), _dev(b))
     nnz, _ = ctx.symbolic(*dev)
-    out = _out(50, nnz)
-    ctx.numeric(*out)
-    _close(out, a, b, orc, "repeated columns")
+    out = _out(a.m, nnz)
+    for _ in range(3):  # the third replays a graph
+        out[2].fill_(float("nan"))
+        ctx.numeric(*out)
+        _close(out, a, b, orc, "repeated columns")
     ctx.close()
