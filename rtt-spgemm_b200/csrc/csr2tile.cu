@@ -34,7 +34,8 @@ namespace
 // belong to, so a hub row costs what its entries cost.  (A warp
 // per 32 rows left the 32 hub rows of an R-MAT matrix to one warp: 460 us for
 // the checks of R-MAT 2^16's 1M entries and 1 ms for its segments; now 14 and
-// 19 us.  96^3 stencil, 23.4M entries: 45 us and 110 us before, 44 and 124 us.)  The row starts among the 256 entries are marked in a shared bitmap.
+// 19 us.  96^3 stencil, 23.4M entries: 45 us and 110 us before, 42 and 126 us.)  The
+// row starts among the 256 entries are marked in a shared bitmap.
 constexpr int CS_WARPS = 8, CS_THREADS = CS_WARPS * 32;
 constexpr int CS_BLOCK = 256, CS_WORDS = CS_BLOCK / 32;
 constexpr int CS_CTAS_MAX = 4096; // CTAs of entries, at most
@@ -134,8 +135,8 @@ __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__
 // flags[0]: some row's tile column decreases (needs the generic path)
 // flags[1]: some row's column decreases (entries not sorted inside rows)
 // flags[2]: some row repeats a column
-// unmade (one of two words beside the error word): set for errors and flags[0]; what follows then makes no segments and no
-// index.  A word of its own beside the error word, which is hardly ever written:
+// unmade (one of two words beside the error word): set for errors and flags[0];
+// what follows then makes no segments and no index.  A word of its own beside the error word, which is hardly ever written:
 // flags[0], cleared for every matrix, took the small products' kernels 0.5 us each.
 __global__ void __launch_bounds__(CS_THREADS, 4)
     k_csr_scan(int m, int n, int nnz, const int *__restrict__ rowptr, const int *__restrict__ col,
@@ -642,7 +643,6 @@ __global__ void __launch_bounds__(256) k_c2t_fill(int m, int tilem, const int *_
     }
 }
 
-// ------------------------------------------------------------ row segments
 // ------------------------------------------------ fast path, heavy tile rows
 // A tile row holding a row with thousands of entries (an R-MAT hub) spans
 // thousands of tile columns; the half-warp above takes them one per step and
@@ -1261,8 +1261,9 @@ inline int grid_for(long long threads, int block) { return (int)((threads + bloc
 // entries each.  One block for small matrices, so that they spread over the
 // SMs; up to 8, where a chunk's own set-up (its first row, the segments before
 // it) is spread over more entries, while every SM keeps 8 CTAs (64^3 stencil:
-// the scan 18 us against 24 with one block); more only to stay within
-// CS_CTAS_MAX.
+// the scan 18 us against 24 with one block; the symbolic step with a block per 400
+// / 1200 / 4000 CTAs 489 / 497 / 506 us, of 96^3 1437 / 1437 / 1449); more only to
+// stay within CS_CTAS_MAX.
 struct CsChunks
 {
     int blocks, ctas;

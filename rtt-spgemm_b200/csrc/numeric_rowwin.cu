@@ -7,8 +7,8 @@
 // only a few entries of each row: on R-MAT 2^16 A*A^T that kernel set up 90
 // million (A entry, window) pairs for 4.5 products each, and the set-up, not
 // the products, was its time.  Here a warp owns one scalar row, so a window
-// holds EW entries of that row alone: about 10 million pairs on the same
-// product, and a banded row with scattered entries (about 256 entries in 80
+// holds EW entries of that row alone: about 18 million pairs on the same
+// product (6 of whole rows, 12 of pieces), and a banded row with scattered entries (about 256 entries in 80
 // tiles, among 1,200 tiles of its tile row) is one window and one walk.
 //
 // A window lives in the warp's shared memory:
@@ -38,9 +38,9 @@
 //
 // What bounds it: issue and shared-memory latency at 14 to 20 warps per SM
 // (about 5 warp instructions per product, 0.42 issued per cycle and scheduler
-// on R-MAT 2^16; DRAM under 6 %).  Against the windows of the tile-row kernel
-// (B200): R-MAT 2^16 A*A^T 20.3 -> 4.9 ms, banded 200k with half-band 32 4.6
-// -> 2.2 ms.
+// on R-MAT 2^16; DRAM under 6 %).  The whole numeric step against the windows of
+// the tile-row kernel (B200): R-MAT 2^16 A*A^T 20.3 -> 5.2 ms (this kernel 4.75),
+// banded 200k with half-band 32 4.6 -> 2.2 ms (this kernel 1.9).
 #include "rtt_internal.cuh"
 
 #include <algorithm>
@@ -63,7 +63,10 @@ constexpr long long EW_LONG = 1024;
 constexpr int RW_SPAN_MAX = 512; // 32-tile words of bm, at most
 constexpr int RW_UNROLL = 4;     // B rows whose first 32 entries are loaded together
 constexpr int RW_GROUP = 4;      // rows of one task, at most
-constexpr size_t PART_BYTES_MAX = size_t(1) << 30; // 2 million rows of B
+// The table of B's parts is made up to this size (2 million rows of B); past it, or
+// where it cannot be had, pieces search: the 4,000 longest rows of R-MAT 2^20 (6
+// edges a row) times the matrix 41 ms with it, of 2^21 168 ms without.
+constexpr size_t PART_BYTES_MAX = size_t(1) << 30;
 constexpr int CUTS = 128; // parts of like weight that B's columns are cut into
 constexpr int ROW_CURSORS = 2048; // A entries of a row whose place in B is kept
 constexpr int PLAN_WARPS = 8;
@@ -777,7 +780,9 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     RTT_CUDA(cudaMemsetAsync(S.w_queue.p, 0, sizeof(TaskQueue), s));
     int *cut_tile = S.r_cut.as<int>();
     k_cut_tiles<<<1, CUT_THREADS, 0, s>>>(B, S.tilen, cut_tile);
-    // a task per row when the groups would leave warps without work
+    // a task per row when the groups would leave warps without work: from 64 rows an
+    // SM two, from 256 four (a quarter of that: banded 20k numeric step 244 us
+    // against 234; four times: 224, and 306 against 318 on banded 50k, half-band 8)
     const int group = S.m >= 64 * RW_GROUP * sms ? RW_GROUP : S.m >= 64 * sms ? 2 : 1;
     const long long target =
         cfg.split_target > 0 ? std::max(1ll, std::min(TARGET_MAX, (long long)cfg.split_target / TD))

@@ -15,9 +15,9 @@
 // Every output is summed by one warp in the order of its row's A entries with
 // fma: bitwise numeric_flat.cu's result.
 //
-// What bounds it: L1 and shared memory (95 % of L1 throughput; 17 shared
+// What bounds it: L1 and shared memory (93 % of L1 throughput; 16 shared
 // wavefronts per B row of 27 products, 6 of them bank conflicts of the
-// accumulator's read-modify-write, and 7 of loads), DRAM 9 %.  64^3 stencil
+// accumulator's read-modify-write, and 6 of loads), DRAM 10 %.  64^3 stencil
 // 692 -> 575 us, 96^3 2.29 -> 1.95 ms against numeric_flat.cu's kernel (B200).
 #include "rtt_internal.cuh"
 

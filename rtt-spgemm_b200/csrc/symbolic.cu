@@ -199,12 +199,19 @@ constexpr size_t BIT_BYTES_MAX = size_t(1) << 30; // (and C's, as large as that 
 // k_sym_count_bits): one warp would walk them alone while the rest of the grid
 // has finished.
 constexpr long long S1_WIDE_PAIRS = 1 << 16;
+// With B's bitmaps, from this many pairs where their words number fewer than twice
+// the pairs.  Symbolic step, one B200: from 128 / 512 / 4,096 pairs R-MAT 2^14 A^2 587
+// / 600 / 668 us, 2^16 A*A^T 2.21 / 2.19 / 2.33 ms; words up to once / twice / eight
+// times the pairs: banded 2k 112 / 97 / 97 us, banded 50k with half-band 8 249 / 249
+// / 345.
 constexpr long long S1_BITS_PAIRS = 512;
 constexpr int S1_WIDE_WARPS = 16;
 
 // Rows listed as wide whose C tiles fill at least 1 / DENSE_SPAN of the tile
 // columns they span keep their masks densely in step 2 (k_sym_dense), window
-// by window of DENSE_TILES tile columns.
+// by window of DENSE_TILES tile columns.  (Spans of 4 / 8 / 16 / 32: R-MAT 2^16 A*A^T
+// symbolic 2.08 / 2.19 / 2.17 / 2.18 ms, R-MAT 2^12, 2^14 and banded rows within 1 %:
+// rows lie well to either side, or gain little.)
 constexpr int DENSE_TILES = 1024, DENSE_WORDS = DENSE_TILES / 32, DENSE_SPAN = 8;
 
 // Step-1 outcome of tile row I: C tiles, the step-2 window flag and the
@@ -264,7 +271,7 @@ __global__ void __launch_bounds__(SYM_WARPS * 32)
     int lo, hi;
     long long pairs;
     row_window(A, B, a0, a1, lo, hi, pairs);
-    // with B's bitmaps at hand: where their words are fewer than half the pairs
+    // with B's bitmaps at hand: where their words are fewer than twice the pairs
     if (pairs > S1_WIDE_PAIRS ||
         (bit_words > 0 && pairs > S1_BITS_PAIRS && 2 * pairs > (long long)(a1 - a0) * bit_words))
     {
@@ -1284,7 +1291,9 @@ int symbolic_tile_counts(Workspace &ws, const DevTiles &A, const DevTiles &B, Sy
         const int sms = ws.sms;
         // B's tile rows as bitmaps, where they are not much larger than B's
         // tile lists (R-MAT 2^16: 2 MB, 2^20: 512 MB; the 96^3 stencil's 380 MB
-        // against 1.3 million tiles are not built)
+        // against 1.3 million tiles are not built).  16 / 64 / 256 bytes a tile: R-MAT
+        // 2^16 A*A^T symbolic 8.35 / 2.19 / 2.19 ms, 2^17 with 4 edges a row 6.8 /
+        // 6.8 / 2.06, whose bitmaps are 8 times A
         const int bit_words = ceil_div(std::max(B.tilen, 1), DENSE_TILES) * DENSE_WORDS;
         const size_t bit_bytes = sizeof(uint32_t) * (size_t)bit_words * (size_t)B.tilem;
         // (a tile for 8 entries while the host does not know B's tiles yet)
