@@ -97,7 +97,7 @@ class Tuner:
     def _load(self) -> dict:
         try:
             table = json.loads(self.path.read_text())
-            if table.get("version") == VERSION:
+            if isinstance(table, dict) and table.get("version") == VERSION:
                 return table
         except (OSError, ValueError):
             pass
