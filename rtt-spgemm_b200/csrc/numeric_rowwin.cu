@@ -68,7 +68,14 @@ constexpr int RW_GROUP = 4;      // rows of one task, at most
 // edges a row) times the matrix 41 ms with it, of 2^21 168 ms without.
 constexpr size_t PART_BYTES_MAX = size_t(1) << 30;
 constexpr int CUTS = 128; // parts of like weight that B's columns are cut into
-constexpr int ROW_CURSORS = 2048; // A entries of a row whose place in B is kept
+// A entries of a row whose places in B are kept from one window to the next, by the
+// longest row of A (in segments, a power of two between these; the least where it
+// is not known).
+constexpr int CURSORS_MIN = 256, CURSORS_MAX = 4096;
+// Rows of more A entries than this drop those whose B rows end; shorter ones keep
+// every entry's place in its own position, half the bytes (16 banded instances 3.36
+// ms, 3.39 with lists for all rows).
+constexpr int LIST_MIN = 2 * CURSORS_MIN;
 constexpr int PLAN_WARPS = 8;
 // Work of one task (products, and 4 for each pair of an A entry and a
 // window): rows with more are cut.  Between these by nnz(C) / 2048, so that
@@ -373,8 +380,8 @@ __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
                      const int *__restrict__ csr_rowptr, int *__restrict__ csr_col,
                      double *__restrict__ csr_val, const RowTask *__restrict__ big,
                      const RowTask *__restrict__ normal, TaskQueue *q, int span,
-                     const int *__restrict__ part, const int *__restrict__ cut_tile, int2 *cursors,
-                     int *err)
+                     const int *__restrict__ part, const int *__restrict__ cut_tile, int4 *cursors,
+                     int ncursors, int *err)
 {
     static_assert(EW <= 65535, "entry offsets are 16 bits");
     extern __shared__ __align__(16) unsigned char rw_raw[];
@@ -383,7 +390,7 @@ __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
         rw_raw + (size_t)(threadIdx.x >> 5) * row_smem_bytes<EW, TW>(span));
     uint2 *bm = reinterpret_cast<uint2 *>(&S + 1);
     const unsigned lt = (1u << lane) - 1u;
-    int2 *cur = cursors + (size_t)(blockIdx.x * RW_WARPS + (threadIdx.x >> 5)) * ROW_CURSORS;
+    int4 *cur = cursors + (size_t)(blockIdx.x * RW_WARPS + (threadIdx.x >> 5)) * ncursors;
     const int nbig = *(volatile int *)&q->big, ntask = nbig + *(volatile int *)&q->normal;
     for (;;)
     {
@@ -420,6 +427,11 @@ __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
             }
             int lo = 0; // first column of the row's window (not its first in the task)
             bool first = true; // the row's first window in this task
+            // A entries whose B rows go on past the window: the first of them in
+            // cur (place, end, a_ik), then all from e_over on
+            int kept = 0, e_over = ea;
+            const bool lists = ee - ea > LIST_MIN;
+            int2 *places = reinterpret_cast<int2 *>(cur); // (rows without lists: place, end)
             // a whole row ends with its last entry, a piece with its last tile
             while (t < tend && dst < row_end)
             {
@@ -635,50 +647,49 @@ __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
                 };
                 // ---- products: the row's A entries, 32 to a batch.  A B row
                 // starts at its head, or at the piece's part of it; what the
-                // window leaves is kept for the next one (of the first
-                // ROW_CURSORS entries; the others' places are searched).
-                for (int q0 = ea; q0 < ee; q0 += 32)
-                {
-                    const int e = q0 + lane;
-                    const bool keep = e - ea < ROW_CURSORS;
-                    int fs = 0, fe = 0;
-                    double a = 0.0;
-                    if (e < ee)
+                // window leaves is kept for the next one, and exhausted entries
+                // leave the list (three hub rows of 200,000 entries with 3 products
+                // each, walked in all of 128 pieces' 7 windows, took 156 ms, now 43;
+                // R-MAT 2^16 A*A^T 7.44 -> 7.28 ms, 2^14 A^2 1.34 -> 1.32).  Entries past the list's room are searched again.
+                //
+                // entry e of A's row: its part of the B row from the window's first
+                // column on
+                auto entry = [&](int e, int &fs, int &fe, double &a) {
+                    fs = fe = 0;
+                    a = 0.0;
+                    if (e >= ee)
+                        return;
+                    a = __ldg(A.csr_val + e);
+                    const int k = __ldg(A.csr_col + e);
+                    if ((unsigned)k < (unsigned)B.m)
                     {
-                        a = __ldg(A.csr_val + e);
-                        if (!first && keep)
+                        // (parts lie in the row: k_row_prepare)
+                        const bool listed = TABLE && piece;
+                        const int *p = listed ? part + (size_t)k * (CUTS + 1) : B.csr_rowptr + k;
+                        fs = __ldg(p + (listed ? tk.y & 0xFFFF : 0));
+                        fe = __ldg(p + (listed ? tk.y >> 16 : 1));
+                        fs = min(max(fs, 0), B.nnz);
+                        fe = min(max(fe, fs), B.nnz);
+                        if (!TABLE && piece)
                         {
-                            const int2 c = cur[e - ea];
-                            fs = c.x;
-                            fe = c.y;
-                        }
-                        else
-                        {
-                            const int k = __ldg(A.csr_col + e);
-                            if ((unsigned)k < (unsigned)B.m)
-                            {
-                                // (parts lie in the row: k_row_prepare)
-                                const bool listed = TABLE && piece;
-                                const int *p = listed ? part + (size_t)k * (CUTS + 1) : B.csr_rowptr + k;
-                                fs = __ldg(p + (listed ? tk.y & 0xFFFF : 0));
-                                fe = __ldg(p + (listed ? tk.y >> 16 : 1));
-                                fs = min(max(fs, 0), B.nnz);
-                                fe = min(max(fe, fs), B.nnz);
-                                if (!TABLE && piece)
-                                {
-                                    fs = lower_bound(B.csr_col, fs, fe,
-                                                     first_column(__ldg(cut_tile + (tk.y & 0xFFFF))));
-                                    fe = lower_bound(B.csr_col, fs, fe,
-                                                     first_column(__ldg(cut_tile + (tk.y >> 16))));
-                                }
-                            }
-                            if (!first)
-                                fs = lower_bound(B.csr_col, fs, fe, lo);
+                            fs = lower_bound(B.csr_col, fs, fe,
+                                             first_column(__ldg(cut_tile + (tk.y & 0xFFFF))));
+                            fe = lower_bound(B.csr_col, fs, fe,
+                                             first_column(__ldg(cut_tile + (tk.y >> 16))));
                         }
                     }
-                    if (first && !more)
+                    if (!first)
+                        fs = lower_bound(B.csr_col, fs, fe, lo);
+                };
+                int used = 0, e_next = e_over;
+                if (first && !more)
+                {
+                    // one window: items of at most 32 B entries, in order
+                    for (int q0 = ea; q0 < ee; q0 += 32)
                     {
-                        // one window: items of at most 32 B entries, in order
+                        int fs, fe;
+                        double a;
+                        entry(q0 + lane, fs, fe, a);
                         const int nch = (fe - fs + 31) >> 5;
                         const int cincl = warp_incl_scan(nch);
                         const int items = __shfl_sync(FULL, cincl, 31);
@@ -702,21 +713,77 @@ __global__ void __launch_bounds__(RW_WARPS * 32, RW_CTAS)
                             __syncwarp();
                             products(min(32, items - i0), std::false_type());
                         }
-                        continue;
                     }
-                    // entries whose B row has nothing in the window leave the list
-                    const bool has = fs < fe && (!more || __ldg(B.csr_col + fs) < hi);
-                    const unsigned list = __ballot_sync(FULL, has);
-                    const int at = __popc(list & lt);
-                    __syncwarp(); // the previous batch (or the zeroes) is done
-                    if (has)
-                        S.ent[at] = make_int4(fs, fe - fs, __double2loint(a), __double2hiint(a));
-                    __syncwarp();
-                    products(__popc(list), std::true_type());
-                    __syncwarp();
-                    if (more && keep && e < ee)
-                        cur[e - ea] = make_int2(has ? S.ent[at].x : fs, fe);
                 }
+                else
+                {
+                    bool room = true;
+                    for (int q0 = -kept, qa = e_over; q0 < 0 || qa < ee;)
+                    {
+                        const bool listed_entry = q0 < 0;
+                        int fs = 0, fe = 0;
+                        double a = 0.0;
+                        if (listed_entry)
+                        {
+                            const int at = kept + q0 + lane;
+                            if (at < kept && lists)
+                            {
+                                const int4 c = cur[at];
+                                fs = c.x;
+                                fe = c.y;
+                                a = __hiloint2double(c.w, c.z);
+                            }
+                            else if (at < kept)
+                            {
+                                const int2 c = places[at];
+                                fs = c.x;
+                                fe = c.y;
+                                a = __ldg(A.csr_val + ea + at);
+                            }
+                            q0 += 32;
+                        }
+                        else
+                        {
+                            entry(qa + lane, fs, fe, a);
+                            qa += 32;
+                        }
+                        // entries whose B row has nothing in the window leave the list
+                        const bool has = fs < fe && (!more || __ldg(B.csr_col + fs) < hi);
+                        const unsigned list = __ballot_sync(FULL, has);
+                        const int at = __popc(list & lt);
+                        __syncwarp(); // the previous batch (or the zeroes) is done
+                        if (has)
+                            S.ent[at] = make_int4(fs, fe - fs, __double2loint(a), __double2hiint(a));
+                        __syncwarp();
+                        products(__popc(list), std::true_type());
+                        __syncwarp();
+                        if (more && !lists)
+                        {
+                            const int i = (listed_entry ? kept + q0 : qa - ea) - 32 + lane;
+                            if (i < ee - ea)
+                                places[i] = make_int2(has ? S.ent[at].x : fs, fe);
+                            used = ee - ea;
+                            e_next = ee;
+                        }
+                        else if (more)
+                        {
+                            const int rest = has ? S.ent[at].x : fs;
+                            const unsigned live = __ballot_sync(FULL, rest < fe);
+                            room = room && used + __popc(live) <= ncursors; // (a list never grows)
+                            if (room)
+                            {
+                                if (rest < fe)
+                                    cur[used + __popc(live & lt)] =
+                                        make_int4(rest, fe, __double2loint(a), __double2hiint(a));
+                                used += __popc(live);
+                                if (!listed_entry)
+                                    e_next = min(qa, ee);
+                            }
+                        }
+                    }
+                }
+                kept = used;
+                e_over = e_next;
                 first = false;
                 __syncwarp();
                 // ---- the window's entries into C
@@ -764,7 +831,10 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     RTT_CHECK(S.r_big.ensure(sizeof(RowTask) * (size_t)big_cap, s));
     RTT_CHECK(S.r_mask.ensure(sizeof(uint16_t) * row_masks(S.numtile, S.tilem, 0, 0), s));
     RTT_CHECK(S.r_cut.ensure(sizeof(int) * (CUTS + 1), s));
-    RTT_CHECK(S.r_cursor.ensure(sizeof(int2) * (size_t)grid * RW_WARPS * ROW_CURSORS, s));
+    int ncursors = CURSORS_MIN;
+    while (ncursors < CURSORS_MAX && ncursors < A.max_row_segs)
+        ncursors *= 2;
+    RTT_CHECK(S.r_cursor.ensure(sizeof(int4) * (size_t)grid * RW_WARPS * ncursors, s));
     RTT_CHECK(S.w_queue.ensure(sizeof(TaskQueue), s));
     // the table of B's parts where it is small enough and can be had
     const size_t part_bytes = sizeof(int) * (size_t)B.m * (CUTS + 1) + 16;
@@ -803,7 +873,7 @@ int rowwin_run(Workspace &ws, const DevTiles &A, const DevTiles &B, SymbolicOut 
     kern<<<grid, RW_WARPS * 32, smem, ws.side>>>(
         A, B, S.nnz, S.c_tile_ptr.as<int>(), S.c_tile_col.as<int>(), S.r_mask.as<uint16_t>(),
         cfg.csr_rowptr, cfg.csr_col, cfg.csr_val, S.r_big.as<RowTask>(), S.r_normal.as<RowTask>(),
-        S.w_queue.as<TaskQueue>(), span, part, cut_tile, S.r_cursor.as<int2>(), ws.err.as<int>());
+        S.w_queue.as<TaskQueue>(), span, part, cut_tile, S.r_cursor.as<int4>(), ncursors, ws.err.as<int>());
     ws.launches++;
     RTT_CUDA(cudaEventRecord(ws.join_ev, ws.side));
     return RTT_OK;

@@ -29,8 +29,8 @@ not copied again.  Each context's own workspace sits outside this
 accounting (and outside structure_bytes, which counts the requests' bounds),
 so pool_bytes should leave room for it below the device's memory: 12 to 16
 bytes per entry of A and B (row segments, tile index), about 100 per C tile,
-and where tile rows of C need several windows 32 more per C tile, 48 MB of
-window cursors, 516 bytes per row of B (at most 1 GiB) and bitmaps of tile
+and where tile rows of C need several windows 32 more per C tile, 12 to 200 MB
+of window cursors, 516 bytes per row of B (at most 1 GiB) and bitmaps of tile
 rows (at most 1 GiB each for B and C).  The last four are done without when
 they cannot be had.
 

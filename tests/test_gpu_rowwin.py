@@ -59,10 +59,19 @@ def _spans():
 
 
 def _long():
-    # 3,000 A entries per row (places kept for 2,048), C rows of many windows
+    # 3,000 A entries per row, places kept for all; C rows of many windows
     rng = np.random.default_rng(7)
     b = _rows([rng.choice(9000, 40, replace=False) for _ in range(6000)], 9000, 8)
     return _pick(20, 3000, 6000, 9), b
+
+
+def _over():
+    # 9,000 A entries per row, places kept for 4,096: the others are searched,
+    # and take the places of those whose B rows end early
+    rng = np.random.default_rng(20)
+    b = _rows([rng.choice(9000, 30, replace=False) if k % 3 else rng.choice(2000, 5, replace=False)
+               for k in range(12000)], 9000, 21)
+    return _pick(20, 9000, 12000, 22), b
 
 
 def _hub():
@@ -95,6 +104,7 @@ def _groups(m, n):
 
 
 CASES = {"entries": _entries, "tiles": _tiles, "spans": _spans, "long": _long, "hub": _hub,
+         "over": _over,
          "entries_long": _entries_long, "tiles_long": _tiles_long,
          "groups2": lambda: _groups(9473, 20000),
          # (and columns further apart than one column index spans)
