@@ -98,14 +98,15 @@ __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__
     if (lane < CS_WORDS)
         bits[lane] = 0u;
     __syncwarp();
-    auto mark = [&](int r) -> bool {
-        const long long x = r < rows ? (long long)__ldg(rowptr + r) : LLONG_MAX;
+    // (unsigned: rows may number INT_MAX)
+    auto mark = [&](unsigned r) -> bool {
+        const long long x = r < (unsigned)rows ? (long long)__ldg(rowptr + r) : LLONG_MAX;
         const bool in = x < end;
         if (in && x >= s0)
             atomicOr(&bits[(x - s0) >> 5], 1u << ((x - s0) & 31));
         return in;
     };
-    int n = __popc(__ballot_sync(FULL, mark(cursor + lane)));
+    int n = __popc(__ballot_sync(FULL, mark((unsigned)cursor + lane)));
     cursor += n;
     if (n == 32)
     {
@@ -114,7 +115,7 @@ __device__ __forceinline__ int mark_rows(uint32_t *bits, const int *__restrict__
             bool in[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                in[q] = mark(cursor + q * 32 + lane);
+                in[q] = mark((unsigned)cursor + q * 32 + lane);
             n = 0;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -424,14 +425,15 @@ __global__ void __launch_bounds__(ST_WARPS * 32, ST_CTAS)
     for (int I = blockIdx.x * ST_WARPS + warp; I < tilem; I += gridDim.x * ST_WARPS)
     {
         // lane r < 16: row r's segments
-        const int d = lane <= TD ? __ldg(rowptr + min(I * TD + lane, m)) : 0;
+        const unsigned r = (unsigned)I * TD + lane; // (rows may number INT_MAX)
+        const int d = lane <= TD ? __ldg(rowptr + min(r, (unsigned)m)) : 0;
         if (stop != 0)
             break;
         const uint2 wd = __ldg(word + (d >> 5));
         int p = (int)wd.y + __popc(wd.x & ((1u << (d & 31)) - 1u));
         int e = __shfl_down_sync(FULL, p, 1);
-        if ((lane < TD || I == tilem - 1) && lane <= TD && I * TD + lane <= m)
-            seg_ptr[I * TD + lane] = p;
+        if ((lane < TD || I == tilem - 1) && lane <= TD && r <= (unsigned)m)
+            seg_ptr[r] = p;
         if (lane >= TD)
             p = e = 0;
         const int s0 = __shfl_sync(FULL, p, 0), s1 = __shfl_sync(FULL, e, TD - 1);
