@@ -398,10 +398,11 @@ __global__ void k_seg_rows(int m, const int *__restrict__ rowptr, const uint2 *_
 
 // Tile index of every tile row from its rows' segments: the tile columns of
 // its segments as a bitmap, a warp per tile row, windows of ST_BITS tile
-// columns, or merged where its few segments span many windows.  Tile row I's list starts at its first segment, so its place needs
-// no count of the tiles before it: tile_ptr[I] = seg_ptr[16 I], tile_end[I] one
-// past its last tile.  seg_ptr[r] is the number of segments before row r's first
-// entry.  out[0] += tiles, out[1] = the most segments of a row.
+// columns, or merged where its few segments span many windows.  Tile row I's list
+// starts at its first segment, so its place needs no count of the tiles before it:
+// tile_ptr[I] = seg_ptr[16 I], tile_end[I] one past its last tile.  seg_ptr[r] is
+// the number of segments before row r's first entry.  out[0] += tiles, out[1] = the
+// most segments of a row.
 // One wave of ST_CTAS CTAs per SM (32 registers), not a CTA for every 4 tile
 // rows: the 156,000 of a matrix of 10 million short rows queued for the two words
 // of out.  That matrix 361 -> 198 us (10 and 12 CTAs per SM: 237), 96^3 stencil 51
@@ -409,8 +410,9 @@ __global__ void k_seg_rows(int m, const int *__restrict__ rowptr, const uint2 *_
 constexpr int ST_WARPS = 4, ST_WORDS = 256, ST_BITS = ST_WORDS * 32, ST_CTAS = 16;
 __global__ void __launch_bounds__(ST_WARPS * 32, ST_CTAS)
     k_seg_tiles(int m, int tilem, const int *__restrict__ rowptr, const uint2 *__restrict__ word,
-                int *__restrict__ seg_ptr, const unsigned long long *__restrict__ seg, int *__restrict__ tile_ptr,
-                int *__restrict__ tile_end, int *__restrict__ tile_col, int *out, const int *unmade)
+                int *__restrict__ seg_ptr, const unsigned long long *__restrict__ seg,
+                int *__restrict__ tile_ptr, int *__restrict__ tile_end,
+                int *__restrict__ tile_col, int *out, const int *unmade)
 {
     __shared__ uint32_t s_bits[ST_WARPS][ST_WORDS];
     __shared__ int s_count, s_max;
@@ -500,11 +502,11 @@ __global__ void __launch_bounds__(ST_WARPS * 32, ST_CTAS)
             __syncwarp();
             for (int q0 = 0; q0 < nwords; q0 += 32)
             {
-                uint32_t word = q0 + lane < nwords ? bits[q0 + lane] : 0u;
-                const int v = __popc(word), incl = warp_incl_scan(v);
+                uint32_t set = q0 + lane < nwords ? bits[q0 + lane] : 0u;
+                const int v = __popc(set), incl = warp_incl_scan(v);
                 int at = s0 + n + incl - v;
-                for (; word != 0u; word &= word - 1u)
-                    tile_col[at++] = w + (q0 + lane) * 32 + __ffs(word) - 1;
+                for (; set != 0u; set &= set - 1u)
+                    tile_col[at++] = w + (q0 + lane) * 32 + __ffs(set) - 1;
                 n += __shfl_sync(FULL, incl, 31);
             }
             __syncwarp();
